@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -78,7 +79,7 @@ struct Small {
     uint32_t over_n;
     uint32_t err;
     uint32_t fallback[8];
-    uint32_t maxrun[8];
+    uint32_t redone[8];  // decoder blocks that assumed a wrong entry, per stream
     unsigned long long max2[2];
     unsigned long long totals[8];
     unsigned long long codewords[8];
@@ -1300,6 +1301,10 @@ struct DecodeJob {
     bool fill = false;
     uint64_t fill_value = 0;
     int fixed_len = 0;  // Huffman: every codeword has this length (decoded without entry tables)
+    bool byte_symbols = false;  // Huffman: every symbol value is below 256
+    // Every codeword length is a multiple of some g > 1: decoding from a position that is no
+    // multiple of g never falls in step, so the entry-table decoder takes the stream.
+    bool tables = false;
 };
 
 // cells_out: decompress_to_cells (block_decompressor_rle.hpp:230-335): *d_out receives the
@@ -1405,16 +1410,18 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         return TabOff{pl.add(4 * t.root.size()), pl.add(4 * t.tree.size()), pl.add(8 * t.symvals.size() + 8)};
     };
     const TabOff to_sym = plan_tab(ht_sym), to_quad = plan_tab(ht_quad), to_cnt = plan_tab(ht_cnt);
-    // decode look-back state per stream (up to 4 streams)
-    auto dec_tiles = [](uint64_t bits) { return cdiv(cdiv(std::max<uint64_t>(bits, 1), kDecodeSubBits), kDecodeBlockSubs); };
-    const uint64_t dtiles = std::max({dec_tiles(s_gr.data_len * 8), dec_tiles(s_sym.data_len * 8),
-                                      h.direct ? 1 : dec_tiles(h.streams[5].data_len * 8),
-                                      rle ? dec_tiles(s_cnt->data_len * 8) : 1});
+    // decode look-back state per stream (up to 4 streams), for either decoder
+    const uint64_t dbits[4] = {s_gr.data_len * 8, s_sym.data_len * 8, h.direct ? 0 : h.streams[5].data_len * 8,
+                               rle ? s_cnt->data_len * 8 : 0};
+    uint64_t ttiles[4], dtiles[4];  // blocks of the entry-table decoder; of either
     size_t o_dflag[4], o_dagg[4], o_dinc[4];
     for (int i = 0; i < 4; ++i) {
-        o_dflag[i] = pl.add(4 * dtiles);
-        o_dagg[i] = pl.add(8 * dtiles * kDecodeMaxL);
-        o_dinc[i] = pl.add(16 * dtiles);
+        ttiles[i] = cdiv(cdiv(std::max<uint64_t>(dbits[i], 1), kDecodeSubBits), kDecodeBlockSubs);
+        const uint64_t stiles = sync_geometry(i == 0 ? kCodeGolombRice : kCodeHuffman, dbits[i]).tiles;
+        dtiles[i] = std::max(ttiles[i], stiles);
+        o_dflag[i] = pl.add(4 * ttiles[i]);
+        o_dagg[i] = pl.add(8 * ttiles[i] * kDecodeMaxL);
+        o_dinc[i] = pl.add(16 * dtiles[i]);
     }
     const uint64_t rtiles = cdiv(std::max<uint64_t>(U, 1), kScanTile);
     const size_t o_rflag = pl.add(4 * rtiles * 5), o_ragg = pl.add(16 * rtiles * 5), o_rinc = pl.add(16 * rtiles * 5);
@@ -1422,7 +1429,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
 
     TRY(memset_small(c, offsetof(Small, err), sizeof(uint32_t), 0));
     TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
-    TRY(memset_small(c, offsetof(Small, fallback), sizeof(uint32_t) * 8 * 2, 0));  // fallback + maxrun
+    TRY(memset_small(c, offsetof(Small, fallback), sizeof(uint32_t) * 8 * 2, 0));  // fallback + redone
     TRY(memset_small(c, offsetof(Small, codewords), sizeof(unsigned long long) * 8, 0));
     CUDA_TRY(cudaMemcpyAsync(c->d_small->hil_inv, hm.inv.data(), 256, cudaMemcpyHostToDevice, st));
     auto upload = [&](const HuffTables& t, const TabOff& o) -> xnyz_status {
@@ -1483,6 +1490,10 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         bool same = !pm.codes.empty();
         for (const auto& ce : pm.codes) same = same && ce.len == t.max_len;
         if (same && t.max_len == t.root_bits) j.fixed_len = t.max_len;
+        int g = 0;
+        for (const auto& ce : pm.codes) g = std::gcd(g, static_cast<int>(ce.len));
+        j.tables = g > 1;
+        j.byte_symbols = std::all_of(pm.symbols.begin(), pm.symbols.end(), [](uint64_t v) { return v < 256; });
         jobs.push_back(j);
         return XNYZ_OK;
     };
@@ -1492,7 +1503,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         j.words = words_of(s_gr, j.base_bits);
         j.total_bits = s_gr.data_len * 8;
         j.nsym = P;
-        j.width = 8;
+        j.width = 4;  // (values of 2^32 and more, none in block mode: decoded again with 8)
         j.out = at<unsigned long long>(c, o_patch);
         j.table.param = grk;
         j.slot = 0;
@@ -1535,11 +1546,29 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
                             at<unsigned long long>(c, o_xoff), at<unsigned long long>(c, o_rv), SMALL_FIELD(c, err),
                             xs);
     }
-    // A fixed-length -rle count stream sums the point count as it decodes (totals[0], zeroed on
-    // its own stream first).
+    // The -rle count stream sums the point count as it decodes (totals[0], zeroed on its own
+    // stream first) unless the entry-table decoder takes it.
     bool counts_summed = false;
     for (auto& j : jobs)
-        if (rle && j.slot == 3 && j.width == 4 && j.fixed_len && !j.fill) counts_summed = true;
+        if (rle && j.slot == 3 && j.width == 4 && !j.fill && (j.fixed_len || !j.tables)) counts_summed = true;
+    // the self-synchronising and the entry-table decoder (their state cleared first)
+    auto launch_sync = [&](const DecodeJob& j, cudaStream_t js, unsigned long long* sum_out) -> xnyz_status {
+        CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_dinc[j.slot]), 0, 16 * dtiles[j.slot], js));
+        launch_decode_sync(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.byte_symbols, j.nsym, j.width, j.out,
+                           at<uint8_t>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
+                           SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, redone[j.slot]),
+                           SMALL_FIELD(c, codewords[j.slot]), sum_out, js);
+        return XNYZ_OK;
+    };
+    auto launch_tables = [&](const DecodeJob& j, cudaStream_t js) -> xnyz_status {
+        CUDA_TRY(cudaMemsetAsync(at<uint32_t>(c, o_dflag[j.slot]), 0, 4 * ttiles[j.slot], js));
+        launch_decode_stream(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.L, j.nsym, j.width, j.out,
+                             at<uint32_t>(c, o_dflag[j.slot]), at<unsigned long long>(c, o_dagg[j.slot]),
+                             at<unsigned long long>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
+                             SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, codewords[j.slot]),
+                             js);
+        return XNYZ_OK;
+    };
     for (auto& j : jobs) {
         if (j.fill) {
             if (j.width == 1)
@@ -1551,23 +1580,21 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         cudaStream_t js = side(c, j.slot);
         Prof pr(c, j.kind == kCodeGolombRice ? "decode_golomb_rice" : (j.kind == kCodeHuffman ? "decode_huffman" : "decode_exp_golomb"),
                 1, j.total_bits / 8.0 + static_cast<double>(j.nsym) * j.width, js);
+        const bool sum = counts_summed && j.slot == 3;
+        if (sum) CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, totals), 0, sizeof(unsigned long long) * 8, js));
+        unsigned long long* sum_out = sum ? SMALL_FIELD(c, totals[0]) : nullptr;
         if (j.fixed_len) {
             if (j.nsym * static_cast<uint64_t>(j.fixed_len) > j.total_bits)
                 return fail(XNYZ_ERR_BAD_STREAM, "Huffman stream shorter than its symbols");
-            const bool sum = counts_summed && j.slot == 3;
-            if (sum) CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, totals), 0, sizeof(unsigned long long) * 8, js));
             launch_decode_fixed(j.words, j.base_bits, j.total_bits, j.table, j.fixed_len, j.nsym, j.width, j.out,
-                                SMALL_FIELD(c, err), js, sum ? SMALL_FIELD(c, totals[0]) : nullptr);
+                                SMALL_FIELD(c, err), js, sum_out);
             continue;
         }
-        // Golomb-Rice tracks k + 2 entry offsets per subsequence (derived in the kernel).
-        const uint32_t* Lrun = nullptr;
-        CUDA_TRY(cudaMemsetAsync(at<uint32_t>(c, o_dflag[j.slot]), 0, 4 * dtiles, js));
-        launch_decode_stream(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.L, Lrun, j.nsym, j.width, j.out,
-                             at<uint32_t>(c, o_dflag[j.slot]), at<unsigned long long>(c, o_dagg[j.slot]),
-                             at<unsigned long long>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
-                             SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, codewords[j.slot]),
-                             js);
+        if (j.tables) {  // (Huffman only)
+            TRY(launch_tables(j, js));
+            continue;
+        }
+        TRY(launch_sync(j, js, sum_out));
     }
     CUDA_TRY(cudaGetLastError());
     TRY(join_sides(c));
@@ -1586,16 +1613,37 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         return fetch_small(c, offsetof(Small, err), offsetof(Small, tile_counters) - offsetof(Small, err));
     };
     TRY(count_total());
-    bool refetch = false;
-    for (auto& j : jobs) {
-        if (j.fill || j.fixed_len) continue;
-        if (c->h_small->fallback[j.slot]) {
-            launch_decode_sequential(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.nsym, j.width, j.out,
-                                     SMALL_FIELD(c, codewords[j.slot]), SMALL_FIELD(c, err), st);
-            refetch = true;
+    // A stream with wide values is decoded again with 64-bit output, one that did not fall in step
+    // by the entry-table decoder, one whose bounded wait expired sequentially (each may take the
+    // next way in turn).  The counts are summed again.
+    bool patch32 = true;
+    for (int pass = 0; pass < 3; ++pass) {
+        bool again = false;
+        for (auto& j : jobs) {
+            const uint32_t why = c->h_small->fallback[j.slot];
+            if (j.fill || j.fixed_len || !why) continue;
+            if (j.kind == kCodeGolombRice) {
+                j.width = 8;
+                patch32 = false;
+            }
+            CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, fallback[j.slot]), 0, 4, st));
+            CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, redone[j.slot]), 0, 4, st));
+            CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, tile_counters[30 + j.slot]), 0, 4, st));
+            if (why == 4u) {
+                TRY(launch_sync(j, st, nullptr));
+            } else if (!(why & 1u) && !j.tables) {
+                j.tables = true;
+                TRY(launch_tables(j, st));
+            } else {
+                launch_decode_sequential(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.nsym, j.width, j.out,
+                                         SMALL_FIELD(c, codewords[j.slot]), SMALL_FIELD(c, err), st);
+            }
+            again = true;
         }
+        if (!again) break;
+        counts_summed = false;
+        TRY(count_total());
     }
-    if (refetch) TRY(count_total());
     TRY(device_errors(c));
     for (auto& j : jobs)
         if (!j.fill && !j.fixed_len && c->h_small->codewords[j.slot] < j.nsym)
@@ -1640,6 +1688,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     RecoverInputs ri{};
     ri.rep_sym = at<uint8_t>(c, o_rep);
     ri.rep_patch = at<unsigned long long>(c, o_patch);
+    ri.patch32 = patch32;
     ri.npatch = P;
     ri.quad_sym = at<uint8_t>(c, o_quad);
     ri.is_start = at<uint8_t>(c, o_isst);

@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(kThreads) count_total_kernel(const i32* __rest
 // ------------------------------------------------------------- recover units -------------
 struct RecoverArgs {
     const u8* rep_sym;
-    const u64* rep_patch;
+    const void* rep_patch;
+    int patch32;
     u64 npatch;
     const u8* quad_sym;
     const u8* is_start;
@@ -271,7 +272,8 @@ __global__ void __launch_bounds__(kThreads, 6) recover_units_kernel(RecoverArgs 
         if (!valid) return 0;
         if (has_val) return a.rep_val[base + e];
         if (sym) return sym - 1u;
-        if (z < a.npatch) return a.rep_patch[z];
+        if (z < a.npatch)
+            return a.patch32 ? (u64)static_cast<const u32*>(a.rep_patch)[z] : static_cast<const u64*>(a.rep_patch)[z];
         atomicOr(a.err, kErrBadStream);
         return 0;
     };
@@ -541,6 +543,7 @@ void launch_recover_units(const RecoverInputs& in, uint64_t units, uint64_t nout
     RecoverArgs a;
     a.rep_sym = in.rep_sym;
     a.rep_patch = in.rep_patch;
+    a.patch32 = in.patch32;
     a.npatch = in.npatch;
     a.quad_sym = in.quad_sym;
     a.is_start = in.is_start;

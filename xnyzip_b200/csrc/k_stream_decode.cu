@@ -1,6 +1,8 @@
 // Parallel decoding of one unindexed prefix-code stream: Huffman (huffman_encoder.hpp:205-243),
 // Golomb-Rice (golomb_rice_encoder.hpp:150-192) and exp-Golomb (huffman_encoder.hpp:398-442).
-// The streams carry no sync points, so decoding is exact for any prefix code:
+// The streams carry no sync points.  decode_sync_kernel decodes from guessed entries and corrects
+// them; streams that do not fall in step go to decode_stream_kernel, whose work does not depend
+// on that.  Both are exact for any prefix code.  The entry-table decoder:
 //
 //   1. every thread owns one S-bit subsequence and computes, for each entry offset e < L
 //      (L = longest codeword; Golomb-Rice: k + 2 classes), where decoding from there leaves
@@ -862,6 +864,489 @@ __global__ void __launch_bounds__(T) decode_stream_kernel(Args a) {
     }
 }
 
+// ------------------------------------------------- self-synchronising decoder ----------
+// Decoding from a wrong bit offset falls in step with the right codewords after a few of them
+// for nearly every code, so the subsequences (a.S bits, one per thread) are decoded from a
+// guess and then corrected: every thread decodes its subsequence from its first bit, takes the
+// exit its predecessor arrived at as its entry and decodes again if that differs, until nothing
+// changes.  A state in which every entry is the predecessor's exit is the one true decoding
+// from the first thread's entry, whatever the guesses were, so the result is exact for any
+// prefix code; only the number of rounds depends on the code.
+//
+// The first G threads of a block redo the last G subsequences of the block before, so that the
+// block's own entry has normally fallen in step as well.  A block publishes (entry it assumed,
+// exit, codewords); a later block walks back over a chain of blocks whose assumed entries match
+// the exits before them, up to one whose result is final (32 at a time), and so gets its true
+// entry and its output position.  A block whose assumption was wrong decodes again from the
+// true entry.  Waits are bounded.  Streams that do not fall in step (kNotConverged, or too many
+// wrong assumptions) are left to decode_stream_kernel, whose entry tables do not depend on it.
+//
+// What bounds it: the dependent chain of codewords within a subsequence (two word reads, a
+// funnel shift, a table read), hidden by the other warps.  A subsequence is an odd number of
+// words, so that lanes at the same place of theirs read distinct banks.  Measured against the
+// entry-table decoder on one B200: the Golomb-Rice stream of 64M terrain points (truncated
+// octahedron, L2 0.001; 150 MB in, 256 MB out) 2187 -> 426 us, of 1013 points 119 -> 20 us; the
+// Huffman streams of a 120K-point direct container 273 -> 47 us, of 8M points (cube, L2 0.1)
+// 568 -> 113 us.
+constexpr int kSyncThreads = 128;
+constexpr int kSyncHalo = 8;
+constexpr int kMaxRounds = 64;
+constexpr u32 kMaxRedo = 256;
+constexpr u32 kNotConverged = 2u;
+constexpr u32 kWideValue = 4u;
+constexpr int kMaxMultiBits = 10;
+
+struct SyncArgs {
+    const u32* words;
+    u32 base;
+    u64 total_bits;
+    u64 nsub;
+    int S, G;
+    Code code;
+    int mb;          // Huffman: window bits of the several-symbols table
+    int multi_out;   // its symbols are the values (all below 256)
+    u64 nsym;
+    int out_width;
+    void* out;
+    unsigned __int128* status;  // per tile (tile_status)
+    u32* tile_counter;
+    u32* err;
+    u32* need_fallback;
+    u32* redone;
+    unsigned long long* total_codewords;
+    unsigned long long* sum_out;  // 32-bit symbols: sum of max(symbol, 0), or null
+};
+
+__host__ __device__ inline size_t sync_smem(int S, int rb, int mb) {
+    return 8 * kSyncThreads + (rb ? (8ull << mb) + (4ull << rb) : 0) + 4 * (size_t)(kSyncThreads * S / 32 + kSyncHalo);
+}
+
+// A block's published state, read and written as one 128-bit word so that no fence is needed:
+// bits 0..61 codewords (of the block; through the block once final), 62..63 flag (1 assumed, 2
+// final), 64..95 assumed entry and 96..127 exit, relative to the block's and the next block's
+// first bit.
+__device__ __forceinline__ unsigned __int128 tile_status(u32 flag, u64 codewords, u64 entry, u64 exit) {
+    return ((unsigned __int128)((exit << 32) | entry) << 64) | (codewords | ((u64)flag << 62));
+}
+__device__ __forceinline__ void st_status(unsigned __int128* p, unsigned __int128 v) {
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
+}
+__device__ __forceinline__ unsigned __int128 ld_status(const unsigned __int128* p) {
+    unsigned __int128 v;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// A thread's run of 32-bit words out[first], out[first + 1], ..: four at a time as one 16-byte
+// store where they lie on a 16-byte boundary.  (A lane's stores land in sectors of their own, so
+// their number is what the store path is busy with.)
+struct WordRun {
+    u32* out;
+    u64 first;
+    u32 a, b, c, d;  // the last four words, d the latest
+    __device__ __forceinline__ void put(u64 i, u32 v) {
+        a = b;
+        b = c;
+        c = d;
+        d = v;
+        if ((i & 3u) == 3u) {
+            if (i - 3u >= first && i >= 3u) {
+                *reinterpret_cast<uint4*>(out + i - 3u) = make_uint4(a, b, c, d);
+            } else {
+                rest(i + 1, 3u);
+            }
+        }
+    }
+    // the last n (1..3) words before `end`, those from `first` on
+    __device__ __forceinline__ void rest(u64 end, u32 n) {
+        if (n > 0u && end > first) out[end - 1] = d;
+        if (n > 1u && end > first + 1) out[end - 2] = c;
+        if (n > 2u && end > first + 2) out[end - 3] = b;
+    }
+    __device__ __forceinline__ void finish(u64 end) { rest(end, (u32)(end & 3u)); }
+};
+
+// A thread's run of bytes from `first` on; whole words go through a WordRun.
+struct ByteRun {
+    u8* out;
+    u64 first, at;
+    u64 acc;  // bytes of the word that holds `at`, and up to three beyond
+    WordRun w;
+    __device__ __forceinline__ void begin(u8* o, u64 i) {
+        out = o;
+        first = at = i;
+        acc = 0;
+        w.out = reinterpret_cast<u32*>(o);
+        w.first = (i + 3) >> 2;
+        w.a = w.b = w.c = w.d = 0;
+    }
+    __device__ __forceinline__ void bytes(u64 lo, u64 hi, u32 v) const {  // [lo, hi) of one word
+        for (u64 j = lo; j < hi; ++j) out[j] = (u8)(v >> ((j & 3u) * 8u));
+    }
+    // n (1..4) bytes, the first in the low byte
+    __device__ __forceinline__ void put(u32 v, u32 n) {
+        const u32 k = (u32)at & 3u;
+        acc |= (u64)v << (8u * k);
+        at += n;
+        if (k + n >= 4u) {
+            const u64 i = (at - n) >> 2;
+            if (i >= w.first) w.put(i, (u32)acc);
+            else bytes(first, 4 * i + 4, (u32)acc);
+            acc >>= 32;
+        }
+    }
+    __device__ __forceinline__ void finish() {
+        const u64 whole = at >> 2;
+        if (whole > w.first) w.finish(whole);
+        const u64 lo = max(first, whole * 4);
+        if (lo < at) bytes(lo, at, (u32)acc);
+    }
+};
+
+// What a block's threads decode with: the staged words (byte-swapped for MSB-first codes), whose
+// bit 0 is stream bit `org`, and the code.  Positions in the staged words are 32-bit (`q`).
+template <int KIND>
+struct SyncStream {
+    const u32* sw;
+    u64 org;
+    Code code;
+    // Huffman, per window of mb bits, the codewords that lie in it: bits taken and number of all of
+    // them (bytes 0 and 1; 0: read one codeword) and of the first four (bytes 2 and 3)
+    const u32* mlen;
+    const u32* msym;  // the symbols of those four
+    int mb;
+    Src g;  // unstaged, for codewords that do not fit the 32-bit window
+
+    __device__ __forceinline__ u32 window(u32 q) const {
+        const u32* w = sw + (q >> 5);
+        return KIND == kCodeGolombRice ? __funnelshift_r(w[0], w[1], q) : __funnelshift_l(w[1], w[0], q);
+    }
+    // One codeword at q: its value and its length, which may exceed 32 bits (Golomb-Rice and
+    // exp-Golomb; Huffman: kFar for a prefix that is no code).
+    __device__ __forceinline__ u64 one(u32 q, u64& v, bool want) const {
+        const u32 win = window(q);
+        const int k = code.k;
+        if (KIND == kCodeHuffman) {
+            u32 sym;
+            const u32 len = huff_lookup(code, win, sym);
+            v = 0;
+            if (!len) return kFar;
+            if (want) v = code.symvals ? __ldg(&code.symvals[sym]) : (u64)sym;
+            return len;
+        }
+        if (KIND == kCodeGolombRice) {
+            const u32 t = (u32)__ffs((int)~win) - 1u;
+            if (t < 32u && k <= 32) {
+                if (want) {
+                    const u32 r = window(q + t + 1u);
+                    v = ((u64)t << k) | (k >= 32 ? r : r & ((1u << k) - 1u));
+                }
+                return t + 1u + (u32)k;
+            }
+            return gr_generic(g, org + q, k, v);
+        }
+        const u32 z = (u32)__clz((int)win);
+        if (2u * z + 1u + (u32)k <= 32u) {
+            const u32 n1 = (win << z) >> (31u - z);
+            const u32 low = k ? __brev((win << (2u * z + 1u)) >> (32 - k)) >> (32 - k) : 0u;
+            const u64 u = ((u64)(n1 - 1u) << k) | low;
+            v = code.zigzag ? ((u >> 1) ^ (~(u & 1ull) + 1ull)) : u;
+            return 2u * z + 1u + (u32)k;
+        }
+        return eg_generic(g, org + q, k, code.zigzag, v);
+    }
+    // From q to the first codeword start at or after qe; adds the codewords passed to c.
+    __device__ __forceinline__ u64 walk(u32 q, u32 qe, u32& c) const {
+        while (q < qe) {
+            if (KIND == kCodeHuffman && q + (u32)mb <= qe) {  // every codeword of the window starts before qe
+                const u32 e = mlen[window(q) >> (32 - mb)];
+                if (e) {
+                    q += e & 0xffu;
+                    c += (e >> 8) & 0xffu;
+                    continue;
+                }
+            }
+            ++c;
+            if (KIND == kCodeGolombRice) {
+                const u32 t = (u32)__ffs((int)~window(q)) - 1u;
+                if (t < 32u) {
+                    q += t + 1u + (u32)code.k;
+                    continue;
+                }
+            }
+            u64 v;
+            const u64 len = one(q, v, false);
+            if (len >= kFar) return org + q + len;
+            q += (u32)len;
+        }
+        return org + q;
+    }
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
+    constexpr int TT = kSyncThreads;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ u32 slot;
+    __shared__ u64 s_entry, s_first, s_wsum[TT / 32];
+    u64* sx = reinterpret_cast<u64*>(smem_raw);
+    u32* mlen = reinterpret_cast<u32*>(sx + TT);
+    u32* msym = mlen + (KIND == kCodeHuffman ? (1 << a.mb) : 0);
+    u32* root = msym + (KIND == kCodeHuffman ? (1 << a.mb) : 0);
+    u32* sw = root + (KIND == kCodeHuffman ? (1 << a.code.rb) : 0);
+
+    const u32 tile = claim_tile(a.tile_counter, &slot);
+    const int t = threadIdx.x, S = a.S, G = a.G;
+    const u32 lane = lane_id();
+    const int staged = TT * S / 32 + kSyncHalo;
+    const long long sub = (long long)tile * (TT - G) - G + t;  // my subsequence
+    const int first_t = tile == 0 ? G : 0;                     // the block's first thread with one
+    const bool valid = t >= first_t && sub < (long long)a.nsub;
+
+    SyncStream<KIND> str;
+    str.g.g = a.words;
+    str.g.base = a.base;
+    str.g.total_bits = a.total_bits;
+    str.g.nwords = (a.base + a.total_bits + 31) >> 5;
+    str.g.sm = nullptr;
+    str.g.sm_w0 = 0;
+    str.g.staged = 0;
+    str.sw = sw;
+    str.code = a.code;
+    str.mlen = mlen;
+    str.msym = msym;
+    str.mb = a.mb;
+    // (tile 0 stages from the stream's start)
+    const u64 w0 = (u64)((long long)tile * (TT - G) - (tile == 0 ? 0 : G)) * (u32)(S / 32);
+    str.org = w0 * 32 - a.base;
+#pragma unroll 8
+    for (int i = t; i < staged; i += TT) {
+        const u64 k = w0 + (u64)i;
+        const u32 x = k < str.g.nwords ? __ldg(a.words + k) : 0u;
+        sw[i] = KIND == kCodeGolombRice ? x : __byte_perm(x, 0, 0x0123);
+    }
+    if (KIND == kCodeHuffman) {
+#pragma unroll 8
+        for (int i = t; i < (1 << a.code.rb); i += TT) root[i] = __ldg(a.code.root + i);
+        str.code.root = root;
+        __syncthreads();
+        for (int w = t; w < (1 << a.mb); w += TT) {
+            u32 at = 0, n = 0, syms = 0, four = 0;
+            while (at < (u32)a.mb) {
+                const u32 e = root[(((u32)w << (32 - a.mb)) << at) >> (32 - a.code.rb)];
+                const u32 len = e >> 24;
+                if (len == 0u || len >= 128u || at + len > (u32)a.mb) break;
+                at += len;
+                if (n < 4) {
+                    syms |= (e & 0xffu) << (8 * n);
+                    four = at | ((n + 1) << 8);
+                }
+                ++n;
+            }
+            mlen[w] = at | (n << 8) | (four << 16);
+            msym[w] = syms;
+        }
+    }
+    __syncthreads();
+
+    const u64 B = valid ? (u64)sub * (u32)S : 0ull;
+    const u64 Bend = valid ? min(B + (u64)S, a.total_bits) : 0ull;
+    u64 entry = B;
+    u32 count = 0;
+    // Rounds from thread `from` on (its entry stays) until every entry is the exit before it.
+    auto settle = [&](int from, bool active) {
+        for (int round = 0;; ++round) {
+            if (active) {
+                count = 0;
+                sx[t] = entry < Bend ? str.walk((u32)(entry - str.org), (u32)(Bend - str.org), count) : entry;
+            }
+            __syncthreads();
+            const u64 e = t > from && valid ? sx[t - 1] : entry;
+            active = valid && t > from && e != entry;
+            entry = e;
+            if (!__syncthreads_or(active)) return true;
+            if (round == kMaxRounds) return false;
+        }
+    };
+    bool settled = settle(first_t, valid);
+
+    // codewords before mine within the block's own subsequences, and the block's total
+    const bool own = valid && t >= G;
+    u64 before = 0, total = 0;
+    auto sum_counts = [&]() {
+        const u32 mine = own ? count : 0u;
+        const u32 incl = warp_incl_add(mine);
+        __syncthreads();  // (s_wsum may still be read by the previous call's)
+        if (lane == 31) s_wsum[t >> 5] = incl;
+        __syncthreads();
+        u64 b = incl - mine, all = 0;
+        for (int w = 0; w < TT / 32; ++w) {
+            if (w < (t >> 5)) b += s_wsum[w];
+            all += s_wsum[w];
+        }
+        before = b;
+        total = all;
+    };
+    sum_counts();
+    const int last_t = (int)min((long long)TT - 1, (long long)a.nsub - 1 - ((long long)tile * (TT - G) - G));
+    if (t == G) s_entry = entry;
+    __syncthreads();
+    const u64 assumed = s_entry;
+
+    // first bit of this block's own subsequences and of the next block's
+    const u64 tile_at = (u64)tile * (u64)(TT - G) * (u64)S, next_at = tile_at + (u64)(TT - G) * (u64)S;
+    auto exit_of = [&]() { return sx[last_t] > next_at ? sx[last_t] - next_at : 0ull; };  // (0: the last block)
+    if (t < 32) {
+        bool failed = !settled || (exit_of() >> 32) != 0 || ((assumed - tile_at) >> 32) != 0;
+        u32 why = kNotConverged;
+        u64 E = assumed - tile_at, C = 0;
+        if (tile > 0) {
+            if (lane == 0 && !failed) st_status(&a.status[tile], tile_status(1u, total, assumed - tile_at, exit_of()));
+            // 128 blocks per step, four per lane (the nearest first)
+            long long top = (long long)tile - 1;
+            u64 pend = 0;
+            u32 spins = 0;
+            while (!failed) {
+                u32 f[4];
+                u64 n[4], ex[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const long long q = top - 4 * (long long)lane - j;
+                    const unsigned __int128 v = q >= 0 ? ld_status(&a.status[q]) : (unsigned __int128)2u << 62;
+                    n[j] = (u64)v & ((1ull << 62) - 1);
+                    f[j] = (u32)((u64)v >> 62);
+                    ex[j] = (u64)(v >> 64);
+                }
+                // my four up to my first final one, chained to the next lane's first exit
+                const u64 xnext = __shfl_down_sync(kFullMask, ex[0] >> 32, 1);
+                bool bad = false, fin = false;
+                u64 add = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (fin) continue;
+                    add += n[j];
+                    if (f[j] == 2u) {
+                        fin = true;
+                    } else if (f[j] == 0u) {
+                        bad = true;
+                    } else {
+                        const u64 x = j < 3 ? ex[j < 3 ? j + 1 : 3] >> 32 : xnext;
+                        if ((j < 3 || lane < 31u) && (ex[j] & 0xffffffffull) != x) bad = true;
+                    }
+                }
+                const u32 fm = __ballot_sync(kFullMask, fin);
+                const u32 last = fm ? (u32)__ffs(fm) - 1u : 31u;
+                const u64 x0 = __shfl_sync(kFullMask, ex[0] >> 32, 0);
+                const bool link = top == (long long)tile - 1 || pend == x0;
+                if (__any_sync(kFullMask, bad && lane <= last) || !link) {
+                    const u32 given_up = __shfl_sync(kFullMask, lane == 0 ? ld_volatile(a.need_fallback) : 0u, 0);
+                    if (++spins > kSpinLimit) {
+                        failed = true;
+                        why = 1u;
+                        if (lane == 0) atomicOr(a.err, kErrTimeout);
+                    } else if ((given_up & ~kWideValue) != 0u) {
+                        failed = true;
+                    }
+                    if (spins > 64) __nanosleep(100);
+                    if (!link) {  // the chain's last link has been decoded again: start over
+                        top = (long long)tile - 1;
+                        C = 0;
+                    }
+                    continue;
+                }
+                if (top == (long long)tile - 1) E = x0;
+                C += warp_sum(lane <= last ? add : 0ull);
+                if (fm) break;
+                pend = __shfl_sync(kFullMask, ex[3] & 0xffffffffull, 31);
+                top -= 128;
+            }
+        }
+        if (lane == 0) {
+            if (failed) {  // seen by whoever reads the status below
+                atomicOr(a.need_fallback, why);
+                __threadfence();
+            }
+            const bool same = E == assumed - tile_at;
+            if (!failed && !same && atomicAdd(a.redone, 1u) >= kMaxRedo) atomicOr(a.need_fallback, kNotConverged);
+            if (failed || same) st_status(&a.status[tile], tile_status(2u, C + total, 0ull, exit_of() & 0xffffffffull));
+            s_entry = failed ? assumed : tile_at + E;
+            s_first = C;
+        }
+    }
+    __syncthreads();
+    if (s_entry != assumed) {  // block-uniform: decode again from the true entry
+        if (t == G) entry = s_entry;
+        const bool ok = settle(G, t == G);
+        sum_counts();
+        if (t == 0) {
+            if (!ok || (exit_of() >> 32) != 0) {
+                atomicOr(a.need_fallback, kNotConverged);
+                __threadfence();
+            }
+            st_status(&a.status[tile], tile_status(2u, s_first + total, 0ull, exit_of() & 0xffffffffull));
+        }
+    }
+    if (tile == gridDim.x - 1 && t == 0) *a.total_codewords = s_first + total;
+
+    u64 sum = 0;
+    u64 idx = s_first + before;
+    if (own && entry < Bend && idx < a.nsym && !(ld_volatile(a.need_fallback) & ~kWideValue)) {
+        u32 q = (u32)(entry - str.org);
+        const u32 qe = (u32)(Bend - str.org);
+        const bool bytes = a.out_width == 1;
+        ByteRun br;
+        br.begin(static_cast<u8*>(a.out), idx);
+        WordRun wr{static_cast<u32*>(a.out), idx, 0, 0, 0, 0};
+        bool wide = false;
+        while (q < qe && idx < a.nsym) {
+            if (KIND == kCodeHuffman && a.multi_out && q + (u32)a.mb <= qe && idx + 4 <= a.nsym) {
+                const u32 w = str.window(q) >> (32 - a.mb);
+                const u32 e = mlen[w] >> 16;
+                if (e) {
+                    u32 syms = msym[w];
+                    const u32 n = e >> 8;
+                    q += e & 0xffu;
+                    if (bytes) {
+                        br.put(syms, n);
+                        idx += n;
+                    } else {
+                        for (u32 i = 0; i < n; ++i, syms >>= 8, ++idx) {
+                            wr.put(idx, syms & 0xffu);
+                            sum += syms & 0xffu;
+                        }
+                    }
+                    continue;
+                }
+            }
+            u64 v;
+            const u64 len = str.one(q, v, true);
+            if (str.org + q + len > a.total_bits) {
+                atomicOr(a.err, kErrBadStream);
+                break;
+            }
+            if (KIND == kCodeHuffman && bytes) {
+                br.put((u32)v & 0xffu, 1u);
+            } else if (a.out_width == 4) {
+                wr.put(idx, (u32)v);
+                wide |= (v >> 32) != 0;
+                sum += (u64)max((i32)(u32)v, 0);
+            } else {
+                static_cast<u64*>(a.out)[idx] = v;
+            }
+            ++idx;
+            if (len >= kFar) break;  // past every subsequence of this thread
+            q += (u32)len;
+        }
+        if (KIND == kCodeHuffman && bytes) br.finish();
+        else if (a.out_width == 4 && idx > wr.first) wr.finish(idx);
+        if (KIND == kCodeGolombRice && wide) atomicOr(a.need_fallback, kWideValue);
+    }
+    if (a.sum_out) {
+        sum = warp_sum(sum);
+        if (lane == 0 && sum) atomicAdd(a.sum_out, sum);
+    }
+}
+
 // One-thread decoder, run by the host after a bounded wait of the parallel decoder expired.
 template <int KIND>
 __global__ void decode_sequential_kernel(Args a) {
@@ -976,10 +1461,9 @@ Args make_args(int kind, const uint32_t* words, uint64_t base_bits, uint64_t tot
 }  // namespace
 
 void launch_decode_stream(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
-                          int L, const uint32_t* L_run, uint64_t nsym, int out_width, void* out, uint32_t* flag,
+                          int L, uint64_t nsym, int out_width, void* out, uint32_t* flag,
                           unsigned long long* agg, unsigned long long* inc, uint32_t* tile_counter, uint32_t* err,
                           uint32_t* need_fallback, unsigned long long* total_codewords, cudaStream_t st) {
-    (void)L_run;
     if (kind == kCodeHuffman && (t.root_bits < 1 || t.root_bits > kMaxRootBits)) {
         atomic_flag_host_error(err, st);  // the host builds tables with 1 <= root_bits <= 11
         return;
@@ -1013,6 +1497,75 @@ void launch_decode_stream(int kind, const uint32_t* words, uint64_t base_bits, u
                              smem_max);
         decode_stream_kernel<kCodeExpGolomb><<<tiles, T, smem, st>>>(a);
     }
+}
+
+SyncGeometry sync_geometry(int kind, uint64_t total_bits) {
+    SyncGeometry g{};
+    // Subsequences of 33 (Golomb-Rice), 17, 9 or 5 words: the longest that still leaves every SM
+    // a few blocks (a round costs a subsequence's whole chain, so short ones settle sooner; long
+    // ones need fewer rounds, and fewer of them are decoded twice by neighbouring blocks).
+    const uint64_t want = 112ull * 148 * 4;
+    int w = kind == kCodeGolombRice ? 33 : 17;
+    const int smallest = kind == kCodeGolombRice ? 9 : 5;
+    while (w > smallest && total_bits < want * 32 * (uint64_t)w) w = w / 2 + 1;
+    g.S = 32 * w;
+    const uint64_t nsub = (total_bits + g.S - 1) / g.S;
+    if (nsub <= (uint64_t)kSyncThreads) {
+        g.tiles = nsub ? 1 : 0;
+        return g;
+    }
+    // decoded ahead of a block: 8192 bits (Golomb-Rice codewords are longer) or 2048
+    g.G = (kind == kCodeGolombRice ? 8192 : 2048) / g.S;
+    if (g.G < 8) g.G = 8;
+    if (g.G > kSyncThreads / 2) g.G = kSyncThreads / 2;
+    g.tiles = (nsub + (kSyncThreads - g.G) - 1) / (kSyncThreads - g.G);
+    return g;
+}
+
+void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
+                        bool byte_symbols, uint64_t nsym, int out_width, void* out, void* status,
+                        uint32_t* tile_counter, uint32_t* err, uint32_t* need_fallback, uint32_t* redone, unsigned long long* total_codewords,
+                        unsigned long long* sum_out, cudaStream_t st) {
+    if (kind == kCodeHuffman && (t.root_bits < 1 || t.root_bits > kMaxRootBits)) {
+        atomic_flag_host_error(err, st);  // the host builds tables with 1 <= root_bits <= 11
+        return;
+    }
+    const SyncGeometry g = sync_geometry(kind, total_bits);
+    if (!g.tiles) return;
+    SyncArgs a{};
+    a.words = words;
+    a.base = (u32)base_bits;
+    a.total_bits = total_bits;
+    a.S = g.S;
+    a.G = g.G;
+    a.nsub = (total_bits + g.S - 1) / g.S;
+    a.code.root = t.root;
+    a.code.tree = t.tree;
+    a.code.symvals = t.symvals;
+    a.code.rb = kind == kCodeHuffman ? t.root_bits : 0;
+    a.code.k = t.param;
+    a.code.zigzag = t.zigzag;
+    a.mb = t.root_bits < kMaxMultiBits ? t.root_bits : kMaxMultiBits;
+    a.multi_out = byte_symbols && !t.symvals;
+    a.nsym = nsym;
+    a.out_width = out_width;
+    a.out = out;
+    a.status = static_cast<unsigned __int128*>(status);
+    a.tile_counter = tile_counter;
+    a.err = err;
+    a.need_fallback = need_fallback;
+    a.redone = redone;
+    a.total_codewords = total_codewords;
+    a.sum_out = out_width == 4 ? sum_out : nullptr;
+    const unsigned tiles = (unsigned)g.tiles;
+    // at most 16.5 KB of words, 16 KB of tables and 1 KB of exits: below the 48 KB that need no opt-in
+    const int smem = (int)sync_smem(g.S, a.code.rb, a.mb);
+    if (kind == kCodeHuffman)
+        decode_sync_kernel<kCodeHuffman><<<tiles, kSyncThreads, smem, st>>>(a);
+    else if (kind == kCodeGolombRice)
+        decode_sync_kernel<kCodeGolombRice><<<tiles, kSyncThreads, smem, st>>>(a);
+    else
+        decode_sync_kernel<kCodeExpGolomb><<<tiles, kSyncThreads, smem, st>>>(a);
 }
 
 void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t, int len,

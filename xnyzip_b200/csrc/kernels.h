@@ -198,11 +198,27 @@ constexpr int kDecodeBlockSubs = 128; // subsequences per thread block
 // tiles = ceil(ceil(bits / sub bits) / kDecodeBlockSubs) (kDecodeSubBits, the smaller, bounds
 // the tiles of every kind).
 // The stream starts `base_bits` (< 32) into `words`.  L = entry offsets tracked (the longest
-// codeword; Golomb-Rice derives k + 2 from its parameter, L_run is unused).
+// codeword; Golomb-Rice derives k + 2 from its parameter).
 void launch_decode_stream(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
-                          int L, const uint32_t* L_run, uint64_t nsym, int out_width, void* out, uint32_t* flag,
+                          int L, uint64_t nsym, int out_width, void* out, uint32_t* flag,
                           unsigned long long* agg, unsigned long long* inc, uint32_t* tile_counter, uint32_t* err,
                           uint32_t* need_fallback, unsigned long long* total_codewords, cudaStream_t st);
+// Self-synchronising decoder: needs no entry tables, for streams whose decoding falls in step
+// from any bit offset.  *need_fallback (starts at 0) tells why the stream has to be decoded
+// otherwise: 1 a bounded wait expired, 2 it did not fall in step, 4 a Golomb-Rice value of 2^32 or
+// more with out_width 4.  status: 16 bytes per tile, zeroed, 16-byte aligned; *redone starts at 0.
+// out: 16-byte aligned.  byte_symbols: every symbol value is below 256.  out_width 4: *sum_out
+// (when given) grows by the sum of max(symbol, 0).
+struct SyncGeometry {
+    int S;           // bits per subsequence
+    int G;           // subsequences a block decodes ahead of its own
+    uint64_t tiles;  // blocks
+};
+SyncGeometry sync_geometry(int kind, uint64_t total_bits);
+void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
+                        bool byte_symbols, uint64_t nsym, int out_width, void* out, void* status,
+                        uint32_t* tile_counter, uint32_t* err, uint32_t* need_fallback, uint32_t* redone,
+                        unsigned long long* total_codewords, unsigned long long* sum_out, cudaStream_t st);
 // One-thread decoder the host runs when a bounded wait of the parallel decoder expired.
 // A Huffman stream whose codewords all have length len (== t.root_bits <= 11): every symbol
 // from its own len bits (out_width 1: u8, 4: u32 values; with out_width 4 and sum_out, *sum_out
@@ -253,7 +269,8 @@ struct RecoverParams {
 };
 struct RecoverInputs {
     const uint8_t* rep_sym;
-    const unsigned long long* rep_patch;
+    const void* rep_patch;      // Golomb-Rice decoded patches: u32 when patch32, else u64
+    int patch32;
     uint64_t npatch;
     const uint8_t* quad_sym;
     const uint8_t* is_start;       // block mode: 1 where a non-empty block starts
