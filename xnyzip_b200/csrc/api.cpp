@@ -332,8 +332,13 @@ struct SortBufs {
 xnyz_status radix_sort(xnyz_ctx* c, SortBufs& b, uint64_t n, int passes, uint32_t* d_hist, int& result) {
     result = 0;
     if (passes == 0 || n <= 1) return XNYZ_OK;
-    const uint64_t tiles = cdiv(n, kSortTile);
-    const size_t need = tiles * 256;
+    if (n <= kSortSmall) {
+        Prof pr(c, "sort_pass", 1, (b.vals[0] ? 24.0 : 16.0) * n * passes);
+        launch_sort_small(b.keys[0], b.keys[0], b.vals[0], b.vals[0], n, passes, c->stream);
+        CUDA_TRY(cudaGetLastError());
+        return XNYZ_OK;
+    }
+    const size_t need = sort_tiles(n) * 256;
     if (c->sort_status_cap < need) {
         CUDA_TRY(cudaStreamSynchronize(c->stream));
         if (c->sort_status) cudaFree(c->sort_status);
@@ -488,7 +493,7 @@ struct CPlan {
 };
 CPlan make_cplan(uint64_t n, bool want_order, size_t reserved, bool ext) {
     CPlan c{};
-    c.tiles = cdiv(n, kSortTile);
+    c.tiles = cdiv(n, kUnitTile);
     Plan pl;
     pl.total = reserved;
     c.o_k0 = pl.add(8 * n);

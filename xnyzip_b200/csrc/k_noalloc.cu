@@ -29,7 +29,8 @@ namespace xnyz {
 namespace {
 
 constexpr unsigned long long kNoAllocMaxKeys = 1ull << 20;
-constexpr unsigned long long kTilesMax = kNoAllocMaxKeys / dev::kSortTile;
+constexpr unsigned long long kTilesMax = 256;
+static_assert(dev::sort_tiles(kNoAllocMaxKeys) <= kTilesMax && dev::sort_tiles(256 * 2048) <= kTilesMax, "status rows");
 // byte offsets inside the scratch array
 constexpr size_t kOffKeys = 0;
 constexpr size_t kOffVals = kOffKeys + 8 * kNoAllocMaxKeys;
@@ -94,10 +95,14 @@ extern "C" xnyz_status xnyz_sort_noalloc(uint64_t* dev_keys, uint32_t* dev_paylo
     }
     unsigned long long* kb[2] = {reinterpret_cast<unsigned long long*>(dev_keys), keys_alt};
     uint32_t* vb[2] = {dev_payload, dev_payload ? vals_alt : nullptr};
-    launch_sort_histogram(kb[0], n, passes, hist, st);
-    launch_sort_offsets(hist, passes, st);
     int cur = 0;
-    for (int p = 0; p < passes; ++p) {
+    if (n <= kSortSmall) {
+        launch_sort_small(kb[0], kb[0], vb[0], vb[0], n, passes, st);
+    } else {
+        launch_sort_histogram(kb[0], n, passes, hist, st);
+        launch_sort_offsets(hist, passes, st);
+    }
+    for (int p = 0; p < passes && n > kSortSmall; ++p) {
         uint32_t epoch;
         {
             std::lock_guard<std::mutex> lk(g_mu);

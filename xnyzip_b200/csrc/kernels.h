@@ -127,12 +127,19 @@ void launch_hilbert(const unsigned long long* in, uint64_t n, const uint8_t* tab
                     unsigned long long* out, cudaStream_t st);
 
 // --- sort -----------------------------------------------------------------------------
-constexpr int kSortTile = 4096;
+// Keys per block of a pass: small arrays take small tiles, so that they still cover the 148 SMs
+// (1M keys: 244 tiles of 4096, 120K: 59 of 2048).  At most 256 tiles up to 2^20 keys.
+constexpr uint32_t sort_tile(uint64_t n) { return n <= 256u * 2048 ? 2048u : n <= 256u * 4096 ? 4096u : 8192u; }
+constexpr uint64_t sort_tiles(uint64_t n) { return (n + sort_tile(n) - 1) / sort_tile(n); }
 void launch_sort_histogram(const unsigned long long* keys, uint64_t n, int passes, uint32_t* hist, cudaStream_t st);
 void launch_sort_offsets(uint32_t* hist, int passes, cudaStream_t st);  // in place: counts -> exclusive offsets
 void launch_sort_pass(const unsigned long long* kin, unsigned long long* kout, const uint32_t* vin, uint32_t* vout,
                       uint64_t n, int shift, const uint32_t* offsets, unsigned long long* status, uint32_t epoch,
                       uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
+// All passes of up to kSortSmall keys in one launch; the output may be the input.
+constexpr uint64_t kSortSmall = 8192;
+void launch_sort_small(const unsigned long long* kin, unsigned long long* kout, const uint32_t* vin, uint32_t* vout,
+                       uint64_t n, int passes, cudaStream_t st);
 
 // --- compress segments + encoders -------------------------------------------------------
 constexpr int kUnitTile = 4096;
