@@ -126,6 +126,8 @@ struct xnyz_ctx {
     size_t h_stage_cap = 0;
     uint8_t* d_container = nullptr;  // device container returned by xnyz_compress_device
     size_t d_container_cap = 0;
+    uint8_t* d_blob = nullptr;  // host bytes of a container whose header is large
+    size_t d_blob_cap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // Side streams for independent streams of one container (the entropy coders and
     // decoders run concurrently); forked from and joined back into `stream` by events.
@@ -182,6 +184,19 @@ xnyz_status ensure_host_stage(xnyz_ctx* c, size_t bytes) {
     const size_t want = align_up(bytes + bytes / 8, 1 << 20);
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_stage), want, cudaHostAllocDefault));
     c->h_stage_cap = want;
+    return XNYZ_OK;
+}
+
+// The buffer of the container that xnyz_compress_device returns (+ 64 bytes of zero padding).
+xnyz_status ensure_container(xnyz_ctx* c, size_t bytes) {
+    if (c->d_container_cap >= bytes + 64) return XNYZ_OK;
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (c->d_container) cudaFree(c->d_container);
+    c->d_container = nullptr;
+    c->d_container_cap = 0;
+    const size_t want = align_up(bytes + bytes / 4 + 64, 1 << 20);
+    CUDA_TRY(cudaMalloc(&c->d_container, want));
+    c->d_container_cap = want;
     return XNYZ_OK;
 }
 
@@ -378,6 +393,7 @@ struct Container {
         size_t len;
         size_t blob_off;   // host piece: offset in `blob`
         const void* dsrc;  // device piece: source (nullptr for host pieces)
+        bool placed;       // device piece already in its place of the device container
     };
     std::vector<uint8_t> blob;  // all host bytes, in container order
     std::vector<Piece> pieces;
@@ -387,7 +403,7 @@ struct Container {
         if (!pieces.empty() && !pieces.back().dsrc) {
             pieces.back().len += n;
         } else {
-            pieces.push_back(Piece{size, n, blob.size(), nullptr});
+            pieces.push_back(Piece{size, n, blob.size(), nullptr, false});
         }
         const uint8_t* b = static_cast<const uint8_t*>(p);
         blob.insert(blob.end(), b, b + n);
@@ -398,12 +414,12 @@ struct Container {
         host_bytes(&v, sizeof(V));
     }
     // [u64 data_len][u64 meta_len][meta][data]  (block_compressor.hpp:152-155)
-    void stream(const std::vector<uint8_t>& meta, const void* ddata, size_t data_bytes) {
+    void stream(const std::vector<uint8_t>& meta, const void* ddata, size_t data_bytes, bool placed = false) {
         pod<uint64_t>(data_bytes);
         pod<uint64_t>(meta.size());
         host_bytes(meta.data(), meta.size());
         if (data_bytes) {
-            pieces.push_back(Piece{size, data_bytes, 0, ddata});
+            pieces.push_back(Piece{size, data_bytes, 0, ddata, placed});
             size += data_bytes;
         }
     }
@@ -417,7 +433,7 @@ struct Container {
         for (const auto& pr : parts) {
             if (!pr.second) continue;
             if (pr.first) {
-                pieces.push_back(Piece{size, pr.second, 0, pr.first});
+                pieces.push_back(Piece{size, pr.second, 0, pr.first, false});
                 size += pr.second;
             } else {
                 const std::vector<uint8_t> z(pr.second, 0);
@@ -437,22 +453,51 @@ struct Container {
         }
         return cudaSuccess;
     }
-    // Assemble into device memory; host pieces are staged through `stage` (pinned, >= blob).
-    cudaError_t to_device(uint8_t* dst, uint8_t* stage, cudaStream_t st) const {
-        std::memcpy(stage, blob.data(), blob.size());
-        for (const Piece& pc : pieces) {
-            const cudaError_t e =
-                pc.dsrc ? cudaMemcpyAsync(dst + pc.off, pc.dsrc, pc.len, cudaMemcpyDeviceToDevice, st)
-                        : cudaMemcpyAsync(dst + pc.off, stage + pc.blob_off, pc.len, cudaMemcpyHostToDevice, st);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    }
 };
 
 std::vector<uint8_t> le5(uint32_t n, uint8_t b) {
     return {static_cast<uint8_t>(n), static_cast<uint8_t>(n >> 8), static_cast<uint8_t>(n >> 16),
             static_cast<uint8_t>(n >> 24), b};
+}
+
+// Assembles the container in c->d_container in one launch: the host bytes travel as a kernel
+// argument (through pinned memory when they are many), the pieces not yet in place are copied, and
+// 64 zero bytes follow.
+xnyz_status container_to_device(xnyz_ctx* c, const Container& k) {
+    const uint8_t* blob = nullptr;
+    if (k.blob.size() > kGatherInline) {
+        TRY(ensure_host_stage(c, k.blob.size()));
+        if (c->d_blob_cap < k.blob.size()) {
+            CUDA_TRY(cudaStreamSynchronize(c->stream));
+            if (c->d_blob) cudaFree(c->d_blob);
+            c->d_blob = nullptr;
+            c->d_blob_cap = 0;
+            const size_t want = align_up(2 * k.blob.size(), 1 << 16);
+            CUDA_TRY(cudaMalloc(&c->d_blob, want));
+            c->d_blob_cap = want;
+        }
+        std::memcpy(c->h_stage, k.blob.data(), k.blob.size());
+        CUDA_TRY(cudaMemcpyAsync(c->d_blob, c->h_stage, k.blob.size(), cudaMemcpyHostToDevice, c->stream));
+        blob = c->d_blob;
+    }
+    GatherArgs g{};
+    if (!blob) std::memcpy(g.inline_bytes, k.blob.data(), k.blob.size());
+    auto add = [&](const Container::Piece& pc) {
+        g.piece[g.count++] = GatherPiece{pc.dsrc ? static_cast<const uint8_t*>(pc.dsrc) : blob ? blob + pc.blob_off : nullptr,
+                                         pc.off, pc.len, static_cast<uint32_t>(pc.dsrc || blob ? 0 : pc.blob_off), 0};
+    };
+    for (const Container::Piece& pc : k.pieces) {
+        if (pc.placed) continue;
+        if (g.count == kGatherPieces - 1) {
+            launch_gather(g, c->d_container, c->stream);
+            g.count = 0;
+        }
+        add(pc);
+    }
+    g.piece[g.count++] = GatherPiece{nullptr, k.size, 64, 0, 1};
+    launch_gather(g, c->d_container, c->stream);
+    CUDA_TRY(cudaGetLastError());
+    return XNYZ_OK;
 }
 
 struct CompressOut {
@@ -486,7 +531,7 @@ xnyz_status lb_clear(xnyz_ctx* c, const LB& l, int channels) {
 struct CPlan {
     uint64_t tiles;
     size_t o_k0, o_k1, o_v0, o_v1, o_rep, o_quad, o_patch, o_blkid, o_blkunit, o_unitpos, o_counts, o_over_v,
-        o_over_u, o_dblk, o_dcnt;
+        o_over_u;
     LB lb_units, lb_enc;
     size_t o_repval = 0, o_xw = 0, o_xk = 0, o_xoff = 0, o_xcost = 0, o_xfeat = 0, o_xconf = 0, o_xflag = 0;
     size_t total;
@@ -509,8 +554,6 @@ CPlan make_cplan(uint64_t n, bool want_order, size_t reserved, bool ext) {
     c.o_counts = pl.add(4 * n);
     c.o_over_v = pl.add(4 * n);
     c.o_over_u = pl.add(4 * n);
-    c.o_dblk = pl.add(8 * n);
-    c.o_dcnt = pl.add(8 * n);
     c.lb_units = plan_lb(pl, c.tiles, 3);
     c.lb_enc = plan_lb(pl, c.tiles, 4);
     if (ext) {
@@ -606,7 +649,7 @@ struct CellInput {
 };
 
 xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xnyz_params& prm, bool want_order,
-                          size_t arena_reserved, CompressOut& R, const CellInput* cin = nullptr) {
+                          size_t arena_reserved, CompressOut& R, const CellInput* cin = nullptr, bool to_device = false) {
     if (prm.quantizer != XNYZ_QUANT_CUBE && prm.quantizer != XNYZ_QUANT_TO && prm.quantizer != XNYZ_QUANT_ADAPTIVE)
         return fail(XNYZ_ERR_INVALID_ARG, "quantizer must be 0 (cube), 1 (truncated octahedron) or 2 (adaptive)");
     if (cin && prm.quantizer == XNYZ_QUANT_ADAPTIVE)
@@ -739,8 +782,7 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     const uint64_t tiles = cp.tiles;
     const size_t o_k0 = cp.o_k0, o_k1 = cp.o_k1, o_v0 = cp.o_v0, o_v1 = cp.o_v1, o_rep = cp.o_rep, o_quad = cp.o_quad,
                  o_patch = cp.o_patch, o_blkid = cp.o_blkid, o_blkunit = cp.o_blkunit, o_unitpos = cp.o_unitpos,
-                 o_counts = cp.o_counts, o_over_v = cp.o_over_v, o_over_u = cp.o_over_u, o_dblk = cp.o_dblk,
-                 o_dcnt = cp.o_dcnt;
+                 o_counts = cp.o_counts, o_over_v = cp.o_over_v, o_over_u = cp.o_over_u;
     const LB lb_units = cp.lb_units, lb_enc = cp.lb_enc;
     Plan pl;
     pl.total = cp.total;
@@ -824,9 +866,8 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     }
     if (!direct) {
         TRY(memset_small(c, offsetof(Small, max2), sizeof(unsigned long long) * 2, 0));
-        Prof pr(c, "block_deltas", 1, 28.0 * NB);
-        launch_block_deltas(uo.blk_id, uo.blk_unit, NB, U, at<unsigned long long>(c, o_dblk),
-                            at<unsigned long long>(c, o_dcnt), c->d_small->max2, st);
+        Prof pr(c, "block_max", 1, 12.0 * NB);
+        launch_block_max(uo.blk_id, uo.blk_unit, NB, U, c->d_small->max2, st);
     }
     // ---- 6b. extended container: block parameters of the repos / SFC-delta stream ----
     const uint64_t ext_nb = ext ? cdiv(U, kParamBlock) : 0;
@@ -944,8 +985,15 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     auto words_for = [](uint64_t bits) { return cdiv(bits, 32) + 4; };
     Plan pe;
     pe.total = pl.total;
-    const size_t o_w_blk = pe.add(4 * words_for(NB * static_cast<uint64_t>(w_blk)));
-    const size_t o_w_cnt = pe.add(4 * words_for(NB * static_cast<uint64_t>(w_cnt)));
+    // The block streams (widths of 8 and more) are packed straight into the device container, at
+    // the places that the header and the stream lengths fix; else into the workspace.
+    const uint64_t len_blk = direct ? 0 : cdiv(NB * static_cast<uint64_t>(w_blk), 8),
+                   len_cnt = direct ? 0 : cdiv(NB * static_cast<uint64_t>(w_cnt), 8);
+    const size_t at_blk = (ext ? 8 : 0) + 16 + (adaptive ? 12 : 0) + 14 + 21, at_cnt = at_blk + len_blk + 21;
+    const bool in_blk = to_device && !direct && w_blk >= kPackDirectWidth,
+               in_cnt = to_device && !direct && w_cnt >= kPackDirectWidth;
+    const size_t o_w_blk = pe.add(in_blk ? 0 : 4 * words_for(8 * len_blk));
+    const size_t o_w_cnt = pe.add(in_cnt ? 0 : 4 * words_for(8 * len_cnt));
     const size_t o_w_gr = pe.add(4 * words_for(bits_gr));
     const size_t o_w_rep = pe.add(4 * words_for(bits_rep));
     const size_t o_w_quad = pe.add(4 * words_for(bits_quad));
@@ -953,12 +1001,20 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     const size_t o_dense = pe.add(kCountDense * 5);
     const size_t o_sparse = pe.add(sparse_val.size() * 9 + 16);
     const size_t o_w_xp = pe.add(4 * words_for(ext_bits));
-    const size_t enc_begin = o_w_blk, enc_end = pe.total;
+    // zeroed for the encoders: all but the directly packed block streams
+    const size_t enc_begin = w_blk >= kPackDirectWidth && w_cnt >= kPackDirectWidth ? o_w_gr : o_w_blk,
+                 enc_end = pe.total;
     if (pe.total > c->arena.cap) {
         // Growing would move the arena; the inputs above live in it.  Plan for the worst
         // case next time and redo this call.
         return fail(XNYZ_ERR_OOM, "__grow__:" + std::to_string(pe.total));
     }
+    if (to_device)  // everything but the Golomb-Rice stream has its exact size
+        TRY(ensure_container(c, at_cnt + len_cnt + 4096 + code_rep.meta.size() + code_quad.meta.size() +
+                                    code_cnt.meta.size() + cdiv(bits_gr, 8) + cdiv(bits_rep, 8) + cdiv(bits_quad, 8) +
+                                    cdiv(bits_cnt, 8) + (ext ? 10 * ext_nb + cdiv(ext_bits, 8) : 0)));
+    uint8_t* const p_blk = in_blk ? c->d_container + at_blk : at<uint8_t>(c, o_w_blk);
+    uint8_t* const p_cnt = in_cnt ? c->d_container + at_cnt : at<uint8_t>(c, o_w_cnt);
     CUDA_TRY(cudaMemsetAsync(c->arena.base + enc_begin, 0, enc_end - enc_begin, st));
     TRY(memset_small(c, offsetof(Small, totals), sizeof(unsigned long long) * 8, 0));
     TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
@@ -968,9 +1024,9 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
         return LookBackState{lbs.flag + ch * lb_enc.tiles, lbs.agg + ch * lb_enc.tiles, lbs.inc + ch * lb_enc.tiles};
     };
     if (!direct) {
-        Prof pr(c, "bitpack", 2, 16.0 * NB + (w_blk + w_cnt) * NB / 8.0);
-        launch_bitpack(at<unsigned long long>(c, o_dblk), NB, w_blk, at<uint32_t>(c, o_w_blk), st);
-        launch_bitpack(at<unsigned long long>(c, o_dcnt), NB, w_cnt, at<uint32_t>(c, o_w_cnt), st);
+        Prof pr(c, "bitpack", 1, 12.0 * NB + (w_blk + w_cnt) * NB / 8.0);
+        launch_block_pack(uo.blk_id, uo.blk_unit, NB, U, {p_blk, at<uint32_t>(c, o_w_blk), w_blk},
+                          {p_cnt, at<uint32_t>(c, o_w_cnt), w_cnt}, st);
     }
     // The four entropy coders are independent: one side stream each.
     uint32_t* dbits = at<uint32_t>(c, o_dense);
@@ -1083,10 +1139,10 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     if (direct) {
         rep_streams();
     } else {
-        K.stream(le5(static_cast<uint32_t>(NB), static_cast<uint8_t>(w_blk)), at<uint32_t>(c, o_w_blk),
-                 cdiv(NB * static_cast<uint64_t>(w_blk), 8));
-        K.stream(le5(static_cast<uint32_t>(NB), static_cast<uint8_t>(w_cnt)), at<uint32_t>(c, o_w_cnt),
-                 cdiv(NB * static_cast<uint64_t>(w_cnt), 8));
+        K.stream(le5(static_cast<uint32_t>(NB), static_cast<uint8_t>(w_blk)), p_blk, len_blk, in_blk);
+        K.stream(le5(static_cast<uint32_t>(NB), static_cast<uint8_t>(w_cnt)), p_cnt, len_cnt, in_cnt);
+        if ((in_blk && K.pieces[1].off != at_blk) || (in_cnt && K.pieces[3].off != at_cnt))
+            return fail(XNYZ_ERR_CUDA, "block streams misplaced");
         rep_streams();
         K.stream({}, nullptr, 0);  // quad patches: quad deltas are < 8, never patched
         K.stream(code_quad.meta, at<uint32_t>(c, o_w_quad), cdiv(bits_quad, 8));
@@ -1126,8 +1182,8 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
 
 // Runs compress_core, growing the arena and retrying once when the encoders need more.
 xnyz_status compress_run(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xnyz_params& p, bool want_order,
-                         size_t reserved, CompressOut& R, const CellInput* cin = nullptr) {
-    xnyz_status s = compress_core(c, d_xyz, n, p, want_order, reserved, R, cin);
+                         size_t reserved, CompressOut& R, const CellInput* cin = nullptr, bool to_device = false) {
+    xnyz_status s = compress_core(c, d_xyz, n, p, want_order, reserved, R, cin, to_device);
     if (s == XNYZ_ERR_OOM && g_last_error.rfind("__grow__:", 0) == 0) {
         const size_t need = std::stoull(g_last_error.substr(9));
         // Input points may live in the arena's reserved prefix: keep them.
@@ -1147,7 +1203,7 @@ xnyz_status compress_run(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xnyz
             TRY(ensure_arena(c, need));
         }
         R = CompressOut{};
-        s = compress_core(c, d_xyz, n, p, want_order, reserved, R, cin);
+        s = compress_core(c, d_xyz, n, p, want_order, reserved, R, cin, to_device);
     }
     return s;
 }
@@ -1806,6 +1862,7 @@ xnyz_status xnyz_destroy(xnyz_ctx* c) {
     if (c->h_small) cudaFreeHost(c->h_small);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->d_container) cudaFree(c->d_container);
+    if (c->d_blob) cudaFree(c->d_blob);
     if (c->d_model) cudaFree(c->d_model);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -1834,6 +1891,9 @@ xnyz_status xnyz_trim(xnyz_ctx* c) {
     if (c->d_container) cudaFree(c->d_container);
     c->d_container = nullptr;
     c->d_container_cap = 0;
+    if (c->d_blob) cudaFree(c->d_blob);
+    c->d_blob = nullptr;
+    c->d_blob_cap = 0;
     return XNYZ_OK;
 }
 
@@ -1990,20 +2050,11 @@ xnyz_status xnyz_compress_device(xnyz_ctx* c, const float* xyz, uint64_t n, cons
     CUDA_TRY(cudaEventRecord(c->ev0, st));
     CompressOut R;
     TRY(ensure_arena(c, make_cplan(n, false, 0, c->block_mode != XNYZ_BLOCKS_OFF).total + encoder_reserve(n)));
-    TRY(compress_run(c, xyz, n, *params, false, 0, R));
+    TRY(compress_run(c, xyz, n, *params, false, 0, R, nullptr, true));
     HostPhase hpa(c, "c7_assemble_device");
     const size_t clen = R.cont.size;
-    if (c->d_container_cap < clen + 64) {
-        CUDA_TRY(cudaStreamSynchronize(st));
-        if (c->d_container) cudaFree(c->d_container);
-        c->d_container = nullptr;
-        const size_t want = align_up(clen + clen / 4 + 64, 1 << 20);
-        CUDA_TRY(cudaMalloc(&c->d_container, want));
-        c->d_container_cap = want;
-    }
-    TRY(ensure_host_stage(c, R.cont.blob.size()));
-    CUDA_TRY(R.cont.to_device(c->d_container, c->h_stage, st));
-    CUDA_TRY(cudaMemsetAsync(c->d_container + clen, 0, 64, st));
+    if (c->d_container_cap < clen + 64) return fail(XNYZ_ERR_CUDA, "container larger than its bound");
+    TRY(container_to_device(c, R.cont));
     CUDA_TRY(cudaEventRecord(c->ev1, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     *dev_container = c->d_container;

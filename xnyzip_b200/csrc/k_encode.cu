@@ -5,7 +5,7 @@
 //                 and patches, symbol histograms with first-occurrence units, all placed by
 //                 a three-channel chained scan (units, patches, blocks).
 //   count_stats   -rle count per unit and its histogram.
-//   block_deltas  + bitpack: BitPacker<uint64_t> of the block-id and block-count deltas.
+//   block_max, block_pack  BitPacker<uint64_t> of the block-id and block-count deltas.
 //   gr_encode     GolombRiceCoder<uint64_t>::pack of the patches.
 //   huff_encode_* HuffmanEncoder<T>::encode / exp-Golomb encode with host-built codes.
 //
@@ -285,97 +285,136 @@ __global__ void __launch_bounds__(kThreads) count_stats_kernel(const u32* __rest
         }
 }
 
-__global__ void __launch_bounds__(kThreads) block_deltas_kernel(const u64* __restrict__ blk_id,
-                                                                const u32* __restrict__ blk_unit, u64 nb, u64 units,
-                                                                u64* __restrict__ d_blk, u64* __restrict__ d_cnt,
-                                                                u64* max2) {
-    __shared__ u64 s0[kThreads / 32], s1[kThreads / 32];
+// Block b's id delta and count delta (u64, wrapping like the reference's in-place differences).
+__device__ __forceinline__ void block_deltas(const u64* __restrict__ blk_id, const u32* __restrict__ blk_unit, u64 nb,
+                                             u32 units, u64 b, u64& db, u64& dc) {
+    const u64 id = __ldg(blk_id + b), pid = b ? __ldg(blk_id + b - 1) : 0ull;
+    const u32 un = __ldg(blk_unit + b), next = b + 1 < nb ? __ldg(blk_unit + b + 1) : units;
+    db = id - pid;
+    dc = next - un;
+    if (b) dc -= (u64)(un - __ldg(blk_unit + b - 1));
+}
+
+// Largest id delta and count delta (the bit widths of the two block streams).  Reads 12 B per block;
+// a thread takes four consecutive blocks.
+__global__ void __launch_bounds__(kThreads) block_max_kernel(const u64* __restrict__ blk_id,
+                                                             const u32* __restrict__ blk_unit, u64 nb, u32 units,
+                                                             u64* max2) {
+    __shared__ u64 sm[2][kThreads / 32];
     u64 m0 = 0, m1 = 0;
-    const u64 stride = (u64)gridDim.x * kThreads;
-    for (u64 b = (u64)blockIdx.x * kThreads + threadIdx.x; b < nb; b += stride) {
-        const u64 cb = ((b + 1 < nb) ? (u64)blk_unit[b + 1] : units) - blk_unit[b];
-        u64 db, dc;
-        if (b == 0) {
-            db = blk_id[0];
-            dc = cb;
+    const u64 stride = (u64)gridDim.x * kThreads * 4;
+    for (u64 b = ((u64)blockIdx.x * kThreads + threadIdx.x) * 4; b < nb; b += stride) {
+        if (b + 4 < nb) {  // (arrays start on 256-byte boundaries)
+            const ulonglong2 i0 = __ldg(reinterpret_cast<const ulonglong2*>(blk_id + b)),
+                             i1 = __ldg(reinterpret_cast<const ulonglong2*>(blk_id + b + 2));
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(blk_unit + b));
+            const u32 u4 = __ldg(blk_unit + b + 4);
+            const u64 pid = b ? __ldg(blk_id + b - 1) : 0ull;
+            const u32 pu = b ? __ldg(blk_unit + b - 1) : 0u;
+            m0 = max(max(m0, i0.x - pid), max(i0.y - i0.x, max(i1.x - i0.y, i1.y - i1.x)));
+            const u64 c = u.x - pu, c0 = u.y - u.x, c1 = u.z - u.y, c2 = u.w - u.z, c3 = u4 - u.w;
+            m1 = max(max(m1, b ? c0 - c : c0), max(c1 - c0, max(c2 - c1, c3 - c2)));
         } else {
-            const u64 cp = (u64)blk_unit[b] - blk_unit[b - 1];
-            db = blk_id[b] - blk_id[b - 1];
-            dc = cb - cp;  // wraps like the reference's in-place u64 differences
+            for (u64 x = b; x < nb; ++x) {
+                u64 db, dc;
+                block_deltas(blk_id, blk_unit, nb, units, x, db, dc);
+                m0 = max(m0, db);
+                m1 = max(m1, dc);
+            }
         }
-        d_blk[b] = db;
-        d_cnt[b] = dc;
-        m0 = max(m0, db);
-        m1 = max(m1, dc);
     }
+#pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         m0 = max(m0, __shfl_xor_sync(kFullMask, m0, d));
         m1 = max(m1, __shfl_xor_sync(kFullMask, m1, d));
     }
     if (lane_id() == 0) {
-        s0[threadIdx.x >> 5] = m0;
-        s1[threadIdx.x >> 5] = m1;
+        sm[0][threadIdx.x >> 5] = m0;
+        sm[1][threadIdx.x >> 5] = m1;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kThreads / 32; ++w) {
-            m0 = max(m0, s0[w]);
-            m1 = max(m1, s1[w]);
-        }
-        m0 = max(m0, s0[0]);
-        m1 = max(m1, s1[0]);
-        atomicMax(&max2[0], m0);
-        atomicMax(&max2[1], m1);
+    if (threadIdx.x < 2) {
+        u64 m = 0;
+        for (int w = 0; w < kThreads / 32; ++w) m = max(m, sm[threadIdx.x][w]);
+        if (m) atomicMax(&max2[threadIdx.x], m);
     }
 }
 
-// BitPacker: value b at bit b*width, LSB-first.  A warp packs 32 consecutive values (b0 a
-// multiple of 32), which fill exactly `width` whole words of their own.  For widths 8..64,
-// lane j builds words j and j + 32 (those below `width`) from the at most ceil(32 / width) + 1
-// values each overlaps (shuffles) and stores them; narrower widths go through the warp's
-// segmented-OR writer.  (Packing 32 values per thread into whole words, measured slower: 2.8
-// -> 4.9 ms per 64M-point step, the per-thread 256-byte reads and width-word writes coalesce
-// worse.)
-__global__ void __launch_bounds__(kThreads) bitpack_kernel(const u64* __restrict__ vals, u64 n, int width,
-                                                           u32* words) {
-    const u64 stride = (u64)gridDim.x * kThreads;
-    const u32 lane = lane_id();
-    if (width >= 8 && width <= 64) {
-        const u32 wu = (u32)width;
-        const int K = (int)((32u + wu - 1u) / wu) + 1;
-        const int halves = wu > 32u ? 2 : 1;
-        u32 v0[2];
-        int p0[2];
-        for (int h = 0; h < 2; ++h) {
-            const u32 m = lane + 32u * (u32)h;
-            v0[h] = m < wu ? (32u * m) / wu : 0u;                // first value overlapping word m
-            p0[h] = (int)(v0[h] * wu) - (int)(32u * m);         // its first bit relative to the word (<= 0)
-        }
-        const u64 vmask = wu >= 64u ? ~0ull : ((1ull << wu) - 1ull);
-        const u64 total = n * (u64)wu;
-        for (u64 b0 = (u64)blockIdx.x * kThreads + (threadIdx.x & ~31u); b0 < n; b0 += stride) {
-            const u64 b = b0 + lane;
-            const u64 x = b < n ? (vals[b] & vmask) : 0ull;
-            for (int h = 0; h < halves; ++h) {
-                const u32 m = lane + 32u * (u32)h;
-                u32 word = 0;
-                for (int k = 0; k < K; ++k) {
-                    const u32 v = v0[h] + (u32)k;
-                    const u64 xv = __shfl_sync(kFullMask, x, (int)(v & 31u));
-                    const int pos = p0[h] + k * (int)wu;
-                    if (m < wu && v < 32u && pos < 32) word |= pos >= 0 ? (u32)(xv << pos) : (u32)(xv >> (-pos));
-                }
-                const u64 wi = (b0 >> 5) * (u64)wu + m;
-                if (m < wu && wi * 32u < total) words[wi] = word;
-            }
+// One block stream on its way out: BitPacker (value b at bit b * width, LSB-first) into bytes
+// [dst, dst + len), dst at any byte (widths 8..64), or OR-ed into the zeroed words at `words`.
+struct PackStream {
+    u8* dst;
+    u64 len;
+    u32* words;
+    int width;
+    u32 magic;  // ceil(2^32 / width): x / width for x width < 2^32
+};
+
+constexpr int kPackTile = 2048;  // blocks per thread block; their bits fill 64 `width` whole words
+constexpr int kPackHead = 4;     // values before the tile (at most 24 bits of them reach into its first word)
+constexpr int kPackTail = 5;     // zeros after the last value, for the last word
+
+// The tile's bits of one stream from its values v[0 .. kPackHead + kPackTile) in shared memory (the
+// first kPackHead precede the tile, kPackTail follow it).  Thread-per-word: aligned word i of dst holds
+// stream bits [32 i - 8 m, 32 i - 8 m + 32) past the tile's first, m the bytes dst lies past a
+// 4-byte boundary, from the one or two (widths below 32: up to five) values that overlap them.
+__device__ __forceinline__ void pack_tile(const PackStream& s, const u64* v, u64 tile, u64 nb) {
+    const u32 wu = (u32)s.width;
+    if (wu < (u32)kPackDirectWidth) {
+        for (u32 i = threadIdx.x & ~31u; i < (u32)kPackTile; i += kThreads) {
+            const u64 b = tile * kPackTile + i + lane_id();
+            warp_write_lsb(s.words, b * wu, v[kPackHead + i + lane_id()], b < nb ? wu : 0u);
         }
         return;
     }
-    for (u64 b0 = (u64)blockIdx.x * kThreads + (threadIdx.x & ~31u); b0 < n; b0 += stride) {
-        const u64 b = b0 + lane;
-        const bool ok = b < n;
-        warp_write_lsb(words, b * (u64)width, ok ? vals[b] : 0ull, ok ? (u32)width : 0u);
+    const u32 m = (u32)(reinterpret_cast<uintptr_t>(s.dst) & 3u);
+    const u64 w0 = tile * 64 * wu;
+    u32* const out = reinterpret_cast<u32*>(s.dst - m) + w0;
+    const u32 left = (u32)min(nb - tile * kPackTile, (u64)kPackTile);
+    const u32 nwords = (left * wu + 8 * m + 31) / 32;  // the last tile's end with the stream
+    const u32 mine = left == (u32)kPackTile && (tile + 1) * kPackTile < nb ? 64 * wu : nwords;
+    const i64 first = 4 * (i64)w0 - (i64)m;  // stream byte of word 0
+    for (u32 i = threadIdx.x; i < mine; i += kThreads) {
+        const u32 q = 32 * i + kPackHead * wu - 8 * m;
+        u32 x = __umulhi(q, s.magic);
+        const u32 r = q - x * wu;
+        u32 word = (u32)(v[x] >> r), got = wu - r;
+        while (got < 32u) {
+            word |= (u32)v[++x] << got;
+            got += wu;
+        }
+        const i64 at = first + 4 * (i64)i;
+        if (at >= 0 && at + 4 <= (i64)s.len) {
+            out[i] = word;
+        } else {
+            for (int b = 0; b < 4; ++b)
+                if (at + b >= 0 && at + b < (i64)s.len) reinterpret_cast<u8*>(out + i)[b] = (u8)(word >> (8 * b));
+        }
     }
+}
+
+// Both block streams from the block ids and first units: 12 B read and the packed bits written per
+// block, straight to where the container has them; what bounds it is the instructions per word.  For
+// the 64M blocks of 64M terrain points at L2 0.001 (42 and 64 bits): deltas through memory, a
+// bit-pack pass each with shuffles and a copy into the container took 394 + 860 + 600 us, shuffles
+// alone from the ids 1044, words from shared memory (this kernel) 442 and
+// block_max 132.
+__global__ void __launch_bounds__(kThreads) block_pack_kernel(const u64* __restrict__ blk_id,
+                                                              const u32* __restrict__ blk_unit, u64 nb, u32 units,
+                                                              PackStream s0, PackStream s1) {
+    __shared__ u64 v0[kPackHead + kPackTile + kPackTail], v1[kPackHead + kPackTile + kPackTail];
+    const u64 tile = blockIdx.x;
+    const u64 mask0 = s0.width >= 64 ? ~0ull : ((1ull << s0.width) - 1), mask1 = s1.width >= 64 ? ~0ull : ((1ull << s1.width) - 1);
+    for (int i = threadIdx.x; i < kPackHead + kPackTile + kPackTail; i += kThreads) {
+        const i64 b = (i64)(tile * kPackTile) + i - kPackHead;
+        u64 db = 0, dc = 0;
+        if (b >= 0 && b < (i64)nb) block_deltas(blk_id, blk_unit, nb, units, (u64)b, db, dc);
+        v0[i] = db & mask0;
+        v1[i] = dc & mask1;
+    }
+    __syncthreads();
+    pack_tile(s0, v0, tile, nb);
+    pack_tile(s1, v1, tile, nb);
 }
 
 // Shared skeleton of the chained-scan encoders: stage a tile of inputs, give every element
@@ -623,6 +662,48 @@ __global__ void __launch_bounds__(kThreads) count_encode_kernel(const i32* __res
     run.end();
 }
 
+// One block per 16 KB of the destination (by its address) and piece.  The body goes out 16 bytes per
+// store, the source read as aligned words and shifted to the destination's alignment; the bytes
+// before and after it one by one.
+constexpr u64 kGatherChunk = 16384;
+__global__ void __launch_bounds__(kThreads) gather_kernel(const __grid_constant__ GatherArgs a, u8* __restrict__ dst) {
+    u64 c = blockIdx.x;
+    for (int i = 0; i < a.count; ++i) {
+        const GatherPiece& p = a.piece[i];
+        const u64 d0 = reinterpret_cast<u64>(dst) + p.off, d1 = d0 + p.len;
+        const u64 chunks = p.len ? (d1 - 1) / kGatherChunk - d0 / kGatherChunk + 1 : 0ull;
+        if (c >= chunks) {
+            c -= chunks;
+            continue;
+        }
+        const u64 base = (d0 / kGatherChunk + c) * kGatherChunk;
+        const u64 lo = max(base, d0), hi = min(base + kGatherChunk, d1);
+        if (!p.src) {
+            for (u64 x = lo + threadIdx.x; x < hi; x += kThreads)
+                *reinterpret_cast<u8*>(x) = p.zero ? (u8)0 : a.inline_bytes[p.inline_off + (u32)(x - d0)];
+            return;
+        }
+        const u64 s0 = reinterpret_cast<u64>(p.src) - d0;  // source address = destination address + s0
+        const u64 b0 = min((lo + 15) & ~15ull, hi), b1 = max(hi & ~15ull, b0);
+        for (u64 x = b0 + 16 * threadIdx.x; x < b1; x += 16 * kThreads) {
+            const u64 s = x + s0;
+            const u32* w = reinterpret_cast<const u32*>(s & ~3ull);
+            const u32 sh = (u32)(s & 3u) * 8u;
+            const u32 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = sh ? __ldg(w + 4) : 0u;
+            *reinterpret_cast<uint4*>(x) = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh),
+                                                      __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+        }
+        const u32 head = (u32)(b0 - lo), tail = (u32)(hi - b1);
+        if (threadIdx.x < head) {
+            *reinterpret_cast<u8*>(lo + threadIdx.x) = *reinterpret_cast<const u8*>(lo + threadIdx.x + s0);
+        } else if (threadIdx.x >= 32u && threadIdx.x - 32u < tail) {
+            const u64 x = b1 + threadIdx.x - 32u;
+            *reinterpret_cast<u8*>(x) = *reinterpret_cast<const u8*>(x + s0);
+        }
+        return;
+    }
+}
+
 inline int persistent_grid(u64 n) {
     u64 want = (n + kThreads - 1) / kThreads;
     if (want < 1) want = 1;
@@ -647,14 +728,32 @@ void launch_count_stats(const uint32_t* unit_pos, uint64_t units, uint64_t n, in
                         cudaStream_t st) {
     count_stats_kernel<<<persistent_grid(units), kThreads, 0, st>>>(unit_pos, units, n, counts, cs);
 }
-void launch_block_deltas(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
-                         unsigned long long* d_blk, unsigned long long* d_cnt, unsigned long long* max2,
-                         cudaStream_t st) {
-    block_deltas_kernel<<<persistent_grid(nblocks), kThreads, 0, st>>>(blk_id, blk_unit, nblocks, units, d_blk, d_cnt,
-                                                                       max2);
+void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
+                      unsigned long long* max2, cudaStream_t st) {
+    block_max_kernel<<<persistent_grid(nblocks), kThreads, 0, st>>>(blk_id, blk_unit, nblocks, (u32)units, max2);
 }
-void launch_bitpack(const unsigned long long* vals, uint64_t n, int width, uint32_t* words, cudaStream_t st) {
-    bitpack_kernel<<<persistent_grid(n), kThreads, 0, st>>>(vals, n, width, words);
+void launch_block_pack(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
+                       const BlockPackDst& blk, const BlockPackDst& cnt, cudaStream_t st) {
+    if (!nblocks) return;
+    auto stream = [&](const BlockPackDst& d) {
+        PackStream s{};
+        s.dst = d.dst;
+        s.len = (nblocks * (u64)d.width + 7) / 8;
+        s.words = d.words;
+        s.width = d.width;
+        s.magic = (u32)(((1ull << 32) + d.width - 1) / d.width);  // (width 1: not used)
+        return s;
+    };
+    const unsigned blocks = (unsigned)((nblocks + kPackTile - 1) / kPackTile);
+    block_pack_kernel<<<blocks, kThreads, 0, st>>>(blk_id, blk_unit, nblocks, (u32)units, stream(blk), stream(cnt));
+}
+void launch_gather(const GatherArgs& a, uint8_t* dst, cudaStream_t st) {
+    u64 blocks = 0;
+    for (int i = 0; i < a.count; ++i) {
+        const u64 d0 = reinterpret_cast<u64>(dst) + a.piece[i].off, d1 = d0 + a.piece[i].len;
+        if (a.piece[i].len) blocks += (d1 - 1) / kGatherChunk - d0 / kGatherChunk + 1;
+    }
+    if (blocks) gather_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a, dst);
 }
 void launch_gr_encode(const unsigned long long* vals, uint64_t n, int k, uint32_t* words, uint64_t cap_bits,
                       LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits, uint32_t* err,

@@ -150,11 +150,37 @@ void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, Di
 // unit_pos null: counts[] is the input (cell tables), else counts[] receives the run lengths.
 void launch_count_stats(const uint32_t* unit_pos, uint64_t units, uint64_t n, int32_t* counts, CountStats cs,
                         cudaStream_t st);
-// Block deltas (blk ids and block unit counts) and their maxima.
-void launch_block_deltas(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
-                         unsigned long long* d_blk, unsigned long long* d_cnt, unsigned long long* max2,
-                         cudaStream_t st);
-void launch_bitpack(const unsigned long long* vals, uint64_t n, int width, uint32_t* words, cudaStream_t st);
+// Largest block-id delta and block-count delta, into max2[0] and max2[1].
+void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
+                      unsigned long long* max2, cudaStream_t st);
+// Bit-packs the block-id and block-count deltas (widths 1..64).  Widths from 8 on: written to the
+// ceil(nblocks width / 8) bytes at dst (any alignment), nothing else touched; narrower: OR-ed into
+// the zeroed words at `words`.
+struct BlockPackDst {
+    uint8_t* dst;
+    uint32_t* words;
+    int width;
+};
+constexpr int kPackDirectWidth = 8;
+void launch_block_pack(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
+                       const BlockPackDst& blk, const BlockPackDst& cnt, cudaStream_t st);
+
+// Copies pieces of any alignment to dst + off in one launch; a piece without a source takes its
+// bytes from the argument itself (zero != 0: zeros).
+constexpr int kGatherPieces = 24;
+constexpr size_t kGatherInline = 4096;
+struct GatherPiece {
+    const uint8_t* src;
+    uint64_t off, len;
+    uint32_t inline_off;
+    uint32_t zero;
+};
+struct GatherArgs {
+    GatherPiece piece[kGatherPieces];
+    int count;
+    uint8_t inline_bytes[kGatherInline];
+};
+void launch_gather(const GatherArgs& args, uint8_t* dst, cudaStream_t st);
 
 constexpr int kEncTile = 4096;
 // Encoders write at most cap_bits bits (the output buffer's size) and flag an overflow beyond.
