@@ -66,18 +66,18 @@ inline size_t align_up(size_t v, size_t a = kAlign) { return (v + a - 1) / a * a
 inline uint64_t cdiv(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 inline int bitlen(uint64_t v) { return v ? 64 - __builtin_clzll(v) : 0; }
 
-// Fixed-size device state of a context (counters, histograms, code tables, tables).
+// Fixed-size device state of a context (counters, histograms, code tables, tables).  [counters,
+// first_rep) starts a call at zero, first_rep and first_quad at ~0, bins and what follows up to the
+// codes at zero; the host reads a prefix of [counters, bins) and of the bins back.
 struct Small {
     PointStats stats;
     unsigned long long counters[8];
     unsigned long long hist_rep[256];
-    uint32_t first_rep[256];
     unsigned long long hist_quad[256];
-    uint32_t first_quad[256];
-    unsigned long long cnt_hist[kCountDense];
-    uint32_t cnt_first[kCountDense];
     uint32_t over_n;
+    uint32_t max_dense;
     uint32_t err;
+    uint32_t pad;
     uint32_t fallback[8];
     uint32_t redone[8];  // decoder blocks that assumed a wrong entry, per stream
     unsigned long long max2[2];
@@ -87,13 +87,19 @@ struct Small {
     unsigned long long ext_bits;      // extended container: block payload bits
     unsigned long long ext_fallback;  // extended container: blocks searched exhaustively
     double ext_sum;                   // extended container: sum of the stream (global mode)
-    uint32_t tile_counters[64];
+    uint32_t first_rep[256];
+    uint32_t first_quad[256];
+    CountStats::Bin bins[kCountDense];
+    uint32_t tile_counters[64];  // [0, 8) sort passes, 10 units, [20, 24) encoders / 20 block streams, 30.. decoders, 40 recover
     uint32_t sort_hist[8 * 256];
     ByteCodes codes[2];
+    uint32_t dense_bits[kCountDense];
+    uint8_t dense_len[kCountDense];
     uint8_t hil_fwd[256];
     uint8_t hil_inv[256];
     float offset_in[4];
 };
+constexpr size_t kBinsFetched = 256;  // count bins that come back with the histograms
 
 // A growable device arena, carved per call.
 struct Arena {
@@ -265,6 +271,17 @@ xnyz_status memset_small(xnyz_ctx* c, size_t off, size_t bytes, int v) {
     return XNYZ_OK;
 }
 
+// Ranges to set in one launch.
+struct Fills {
+    FillArgs a{};
+    void add(void* p, size_t bytes, uint32_t value) {
+        if (bytes) a.range[a.count++] = FillRange{p, bytes / 4, value};
+    }
+    void small(xnyz_ctx* c, size_t from, size_t to, uint32_t value) {
+        add(reinterpret_cast<char*>(c->d_small) + from, to - from, value);
+    }
+};
+
 xnyz_status fetch_small(xnyz_ctx* c, size_t off, size_t bytes) {
     CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char*>(c->h_small) + off, reinterpret_cast<char*>(c->d_small) + off,
                              bytes, cudaMemcpyDeviceToHost, c->stream));
@@ -368,8 +385,7 @@ xnyz_status radix_sort(xnyz_ctx* c, SortBufs& b, uint64_t n, int passes, uint32_
         CUDA_TRY(cudaMemsetAsync(c->sort_status, 0, c->sort_status_cap * sizeof(unsigned long long), c->stream));
         c->sort_epoch = 0;
     }
-    launch_sort_offsets(d_hist, passes, c->stream);
-    TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 8, 0));
+    launch_sort_offsets(d_hist, passes, c->stream);  // (tile_counters[0, 8) are zero)
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const uint32_t epoch = ++c->sort_epoch;
@@ -394,16 +410,21 @@ struct Container {
         size_t blob_off;   // host piece: offset in `blob`
         const void* dsrc;  // device piece: source (nullptr for host pieces)
         bool placed;       // device piece already in its place of the device container
+        // device container only: 1 the late stream's length (8 bytes), 2 its data; pieces after it have
+        // `after`: their offsets grow by its length
+        int late;
+        bool after;
     };
     std::vector<uint8_t> blob;  // all host bytes, in container order
     std::vector<Piece> pieces;
     size_t size = 0;
+    bool after = false;
     void host_bytes(const void* p, size_t n) {
         if (!n) return;
-        if (!pieces.empty() && !pieces.back().dsrc) {
+        if (!pieces.empty() && !pieces.back().dsrc && !pieces.back().late && pieces.back().after == after) {
             pieces.back().len += n;
         } else {
-            pieces.push_back(Piece{size, n, blob.size(), nullptr, false});
+            pieces.push_back(Piece{size, n, blob.size(), nullptr, false, 0, after});
         }
         const uint8_t* b = static_cast<const uint8_t*>(p);
         blob.insert(blob.end(), b, b + n);
@@ -419,9 +440,18 @@ struct Container {
         pod<uint64_t>(meta.size());
         host_bytes(meta.data(), meta.size());
         if (data_bytes) {
-            pieces.push_back(Piece{size, data_bytes, 0, ddata, placed});
+            pieces.push_back(Piece{size, data_bytes, 0, ddata, placed, 0, after});
             size += data_bytes;
         }
+    }
+    // A stream whose length only the device knows yet (at most one per container).
+    void late_stream(const std::vector<uint8_t>& meta, const void* ddata) {
+        pieces.push_back(Piece{size, 8, 0, nullptr, false, 1, false});
+        size += 8;
+        pod<uint64_t>(meta.size());
+        host_bytes(meta.data(), meta.size());
+        pieces.push_back(Piece{size, 0, 0, ddata, false, 2, false});
+        after = true;
     }
     // A stream whose data is several parts: device memory, or zero bytes where ptr is null.
     void stream_parts(const std::vector<uint8_t>& meta, std::initializer_list<std::pair<const void*, size_t>> parts) {
@@ -433,7 +463,7 @@ struct Container {
         for (const auto& pr : parts) {
             if (!pr.second) continue;
             if (pr.first) {
-                pieces.push_back(Piece{size, pr.second, 0, pr.first, false});
+                pieces.push_back(Piece{size, pr.second, 0, pr.first, false, 0, after});
                 size += pr.second;
             } else {
                 const std::vector<uint8_t> z(pr.second, 0);
@@ -463,7 +493,7 @@ std::vector<uint8_t> le5(uint32_t n, uint8_t b) {
 // Assembles the container in c->d_container in one launch: the host bytes travel as a kernel
 // argument (through pinned memory when they are many), the pieces not yet in place are copied, and
 // 64 zero bytes follow.
-xnyz_status container_to_device(xnyz_ctx* c, const Container& k) {
+xnyz_status container_to_device(xnyz_ctx* c, const Container& k, const unsigned long long* late_bits, uint64_t late_most) {
     const uint8_t* blob = nullptr;
     if (k.blob.size() > kGatherInline) {
         TRY(ensure_host_stage(c, k.blob.size()));
@@ -481,20 +511,37 @@ xnyz_status container_to_device(xnyz_ctx* c, const Container& k) {
         blob = c->d_blob;
     }
     GatherArgs g{};
+    g.late_bits = late_bits;
+    g.late_most = late_most;
     if (!blob) std::memcpy(g.inline_bytes, k.blob.data(), k.blob.size());
-    auto add = [&](const Container::Piece& pc) {
-        g.piece[g.count++] = GatherPiece{pc.dsrc ? static_cast<const uint8_t*>(pc.dsrc) : blob ? blob + pc.blob_off : nullptr,
-                                         pc.off, pc.len, static_cast<uint32_t>(pc.dsrc || blob ? 0 : pc.blob_off), 0};
-    };
     for (const Container::Piece& pc : k.pieces) {
         if (pc.placed) continue;
         if (g.count == kGatherPieces - 1) {
             launch_gather(g, c->d_container, c->stream);
             g.count = 0;
         }
-        add(pc);
+        GatherPiece p{};
+        p.off = pc.off;
+        p.len = pc.late == 2 ? late_most : pc.len;
+        p.after = pc.after;
+        if (pc.late == 1) {
+            p.kind = kGatherLateLen;
+        } else if (pc.dsrc) {
+            p.kind = pc.late ? kGatherLate : kGatherCopy;
+            p.src = static_cast<const uint8_t*>(pc.dsrc);
+        } else {
+            p.kind = blob ? kGatherCopy : kGatherInlineBytes;
+            if (blob) p.src = blob + pc.blob_off;
+            else p.inline_off = static_cast<uint32_t>(pc.blob_off);
+        }
+        g.piece[g.count++] = p;
     }
-    g.piece[g.count++] = GatherPiece{nullptr, k.size, 64, 0, 1};
+    GatherPiece z{};
+    z.kind = kGatherZero;
+    z.off = k.size;
+    z.len = 64;
+    z.after = k.after;
+    g.piece[g.count++] = z;
     launch_gather(g, c->d_container, c->stream);
     CUDA_TRY(cudaGetLastError());
     return XNYZ_OK;
@@ -521,6 +568,9 @@ LB plan_lb(Plan& pl, uint64_t tiles, int channels, int agg_words_per_tile = 1, i
 }
 LookBackState lb_state(xnyz_ctx* c, const LB& l) {
     return LookBackState{at<uint32_t>(c, l.flag), at<unsigned long long>(c, l.agg), at<unsigned long long>(c, l.inc)};
+}
+void lb_clear(xnyz_ctx* c, Fills& f, const LB& l, int channels) {
+    f.add(at<uint32_t>(c, l.flag), sizeof(uint32_t) * l.tiles * channels, 0);
 }
 xnyz_status lb_clear(xnyz_ctx* c, const LB& l, int channels) {
     CUDA_TRY(cudaMemsetAsync(at<uint32_t>(c, l.flag), 0, sizeof(uint32_t) * l.tiles * channels, c->stream));
@@ -666,22 +716,24 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
 
     // ---- 1. bounding box + quantization sweep ----
     HostPhase hp1(c, "c1_stats");
-    int32_t* cells_tmp = nullptr;  // the quantization sweep's cells, when the arena holds them
+    const bool ext = c->block_mode != XNYZ_BLOCKS_OFF;
+    const CPlan cp = make_cplan(n, want_order, arena_reserved, ext);
+    TRY(ensure_arena(c, cp.total));
+    int32_t* cells_tmp = nullptr;  // the quantization sweep's cells
     {
-        PointStats init{};
-        for (int a = 0; a < 3; ++a) {
-            init.minkey[a] = ~0ull;
-            init.max_cell[a] = 0;
-            init.min_cell[a] = INT32_MAX;
-        }
-        c->h_small->stats = init;
-        c->h_small->err = 0;
-        CUDA_TRY(cudaMemcpyAsync(&c->d_small->stats, &c->h_small->stats, sizeof(PointStats), cudaMemcpyHostToDevice, st));
-        TRY(memset_small(c, offsetof(Small, err), sizeof(uint32_t), 0));
+        Fills f;
+        const size_t st0 = offsetof(Small, stats);
+        f.small(c, st0 + offsetof(PointStats, minkey), st0 + offsetof(PointStats, max_cell), ~0u);
+        f.small(c, st0 + offsetof(PointStats, max_cell), st0 + offsetof(PointStats, min_cell), cin ? 0x80000000u : 0u);
+        f.small(c, st0 + offsetof(PointStats, min_cell), st0 + offsetof(PointStats, nonfinite), 0x7fffffffu);
+        f.small(c, st0 + offsetof(PointStats, nonfinite), offsetof(Small, first_rep), 0);
+        f.small(c, offsetof(Small, first_rep), offsetof(Small, bins), ~0u);
+        f.small(c, offsetof(Small, bins), offsetof(Small, codes), 0);
+        lb_clear(c, f, cp.lb_units, 3);
+        lb_clear(c, f, cp.lb_enc, 4);
+        launch_fill(f.a, st);
     }
     if (cin) {
-        for (int a = 0; a < 3; ++a) c->h_small->stats.max_cell[a] = INT32_MIN;
-        CUDA_TRY(cudaMemcpyAsync(&c->d_small->stats, &c->h_small->stats, sizeof(PointStats), cudaMemcpyHostToDevice, st));
         launch_cells_stats(cin->cells, n, SMALL_FIELD(c, stats), st);
     } else {
         {
@@ -691,8 +743,7 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
         if (adaptive) launch_adaptive_steps(d_xyz, prm.l2_bound, SMALL_FIELD(c, stats), st);
         {
             // the cells go to the space the units fill later, for the block-mode key kernel
-            const CPlan cp0 = make_cplan(n, want_order, arena_reserved, c->block_mode != XNYZ_BLOCKS_OFF);
-            if (c->arena.cap >= cp0.total) cells_tmp = at<int32_t>(c, cp0.o_patch);  // [o_patch, o_blkunit): 16 n bytes
+            cells_tmp = at<int32_t>(c, cp.o_patch);  // [o_patch, o_blkunit): 16 n bytes
             Prof pr(c, "quantize_range", 1, 12.0 * n);
             launch_quantize_range(d_xyz, n, q, SMALL_FIELD(c, stats), 1, st, cells_tmp);
         }
@@ -776,25 +827,16 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     }
     const int passes = static_cast<int>(cdiv(key_bits, 8));
 
-    // ---- 3. arena plan ----
-    const bool ext = c->block_mode != XNYZ_BLOCKS_OFF;
-    const CPlan cp = make_cplan(n, want_order, arena_reserved, ext);
-    const uint64_t tiles = cp.tiles;
     const size_t o_k0 = cp.o_k0, o_k1 = cp.o_k1, o_v0 = cp.o_v0, o_v1 = cp.o_v1, o_rep = cp.o_rep, o_quad = cp.o_quad,
                  o_patch = cp.o_patch, o_blkid = cp.o_blkid, o_blkunit = cp.o_blkunit, o_unitpos = cp.o_unitpos,
                  o_counts = cp.o_counts, o_over_v = cp.o_over_v, o_over_u = cp.o_over_u;
     const LB lb_units = cp.lb_units, lb_enc = cp.lb_enc;
     Plan pl;
     pl.total = cp.total;
-    (void)tiles;
-    TRY(ensure_arena(c, pl.total));
 
     // ---- 4. keys + digit histograms ----
     SortBufs sb{{at<unsigned long long>(c, o_k0), at<unsigned long long>(c, o_k1)},
                 {want_order ? at<uint32_t>(c, o_v0) : nullptr, want_order ? at<uint32_t>(c, o_v1) : nullptr}};
-    TRY(memset_small(c, offsetof(Small, sort_hist), sizeof(uint32_t) * 8 * 256, 0));
-    CUDA_TRY(cudaMemcpyAsync(c->d_small->hil_fwd, hm.fwd.data(), 256, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(c->d_small->hil_inv, hm.inv.data(), 256, cudaMemcpyHostToDevice, st));
     {
         Prof pr(c, "keys", 1, 20.0 * n + (want_order ? 4.0 * n : 0.0));
         if (cin)
@@ -803,12 +845,9 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
         else if (direct)
             launch_keys_direct(d_xyz, n, q, SMALL_FIELD(c, stats), dkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0],
                                passes, c->d_small->sort_hist, st);
-        else if (cells_tmp)
+        else
             launch_keys_cells(cells_tmp, n, bkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0], passes,
                               c->d_small->sort_hist, st);
-        else
-            launch_keys_block(d_xyz, n, q, SMALL_FIELD(c, stats), bkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0],
-                              passes, c->d_small->sort_hist, st);
     }
     int res = 0;
     TRY(radix_sort(c, sb, n, passes, c->d_small->sort_hist, res));
@@ -816,18 +855,11 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     if (want_order) R.d_order = sb.vals[res];
 
     // ---- 5. units ----
-    TRY(memset_small(c, offsetof(Small, counters), sizeof(unsigned long long) * 8, 0));
-    TRY(memset_small(c, offsetof(Small, hist_rep), sizeof(unsigned long long) * 256, 0));
-    TRY(memset_small(c, offsetof(Small, first_rep), sizeof(uint32_t) * 256, 0xff));
-    TRY(memset_small(c, offsetof(Small, hist_quad), sizeof(unsigned long long) * 256, 0));
-    TRY(memset_small(c, offsetof(Small, first_quad), sizeof(uint32_t) * 256, 0xff));
-    TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
-    TRY(lb_clear(c, lb_units, 3));
     UnitOutputs uo{};
     uo.rep_val = ext ? at<unsigned long long>(c, cp.o_repval) : nullptr;
     uo.rep_sym = at<uint8_t>(c, o_rep);
     uo.quad_sym = at<uint8_t>(c, o_quad);
-    uo.patches = at<unsigned long long>(c, o_patch);
+    uo.patches = at<void>(c, o_patch);
     uo.blk_id = at<unsigned long long>(c, o_blkid);
     uo.blk_unit = at<uint32_t>(c, o_blkunit);
     uo.unit_pos = at<uint32_t>(c, o_unitpos);
@@ -846,40 +878,80 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
                                SMALL_FIELD(c, tile_counters[10]), SMALL_FIELD(c, err), st);
     }
     CUDA_TRY(cudaGetLastError());
-    TRY(fetch_small(c, offsetof(Small, counters), sizeof(unsigned long long) * 8));
-    const uint64_t U = c->h_small->counters[0], P = c->h_small->counters[1], NB = c->h_small->counters[2];
-    const uint64_t psum = c->h_small->counters[3];
-    TRY(check_device_errors(c));
-    hp2.end();
-    HostPhase hp3(c, "c3_stats");
-
-    // ---- 6. count and block statistics ----
+    // ---- 6. count and block statistics (sizes read on the device: the host learns them below) ----
     if (rle) {
-        TRY(memset_small(c, offsetof(Small, cnt_hist), sizeof(unsigned long long) * kCountDense, 0));
-        TRY(memset_small(c, offsetof(Small, cnt_first), sizeof(uint32_t) * kCountDense, 0xff));
-        TRY(memset_small(c, offsetof(Small, over_n), sizeof(uint32_t), 0));
-        CountStats cs{c->d_small->cnt_hist, c->d_small->cnt_first, at<uint32_t>(c, o_over_v), at<uint32_t>(c, o_over_u),
+        CountStats cs{c->d_small->bins, SMALL_FIELD(c, max_dense), at<uint32_t>(c, o_over_v), at<uint32_t>(c, o_over_u),
                       SMALL_FIELD(c, over_n)};
-        Prof pr(c, "count_stats", 1, 8.0 * U);
-        if (cin) launch_gather_i32(cin->counts, R.d_order, U, at<int32_t>(c, o_counts), st);  // container order
-        launch_count_stats(cin ? nullptr : uo.unit_pos, U, n, at<int32_t>(c, o_counts), cs, st);
+        Prof pr(c, "count_stats", 1, 8.0 * n);
+        if (cin) launch_gather_i32(cin->counts, R.d_order, n, at<int32_t>(c, o_counts), st);  // container order
+        launch_count_stats(cin ? nullptr : uo.unit_pos, n, SMALL_FIELD(c, counters[0]), n, at<int32_t>(c, o_counts), cs, st);
     }
     if (!direct) {
-        TRY(memset_small(c, offsetof(Small, max2), sizeof(unsigned long long) * 2, 0));
-        Prof pr(c, "block_max", 1, 12.0 * NB);
-        launch_block_max(uo.blk_id, uo.blk_unit, NB, U, c->d_small->max2, st);
+        Prof pr(c, "block_max", 1, 12.0 * n);
+        launch_block_max(uo.blk_id, uo.blk_unit, n, c->d_small->counters, c->d_small->max2, st);
     }
     // ---- 6b. extended container: block parameters of the repos / SFC-delta stream ----
-    const uint64_t ext_nb = ext ? cdiv(U, kParamBlock) : 0;
-    if (ext) TRY(select_block_params(c, cp, U, ext_nb));
+    if (ext) {
+        TRY(fetch_small(c, offsetof(Small, counters), sizeof(unsigned long long)));
+        TRY(select_block_params(c, cp, c->h_small->counters[0], cdiv(c->h_small->counters[0], kParamBlock)));
+    }
     CUDA_TRY(cudaGetLastError());
-    TRY(fetch_small(c, offsetof(Small, hist_rep),
-                    offsetof(Small, tile_counters) - offsetof(Small, hist_rep)));  // hists, counts, maxima
+    TRY(fetch_small(c, offsetof(Small, counters),
+                    offsetof(Small, bins) + sizeof(CountStats::Bin) * kBinsFetched - offsetof(Small, counters)));
+    TRY(device_errors(c));
     const Small& H = *c->h_small;
-    hp3.end();
+    const uint64_t U = H.counters[0], P = H.counters[1], NB = H.counters[2];
+    const uint64_t psum = H.counters[3];
+    const uint64_t ext_nb = ext ? cdiv(U, kParamBlock) : 0;
+    const uint32_t max_dense = rle ? H.max_dense : 0;
+    if (max_dense >= kBinsFetched)
+        TRY(fetch_small(c, offsetof(Small, bins) + sizeof(CountStats::Bin) * kBinsFetched,
+                        sizeof(CountStats::Bin) * (max_dense + 1 - kBinsFetched)));
+    hp2.end();
     HostPhase hp4(c, "c4_codebooks");
 
-    // ---- 7. codebooks (host replay of the reference's container order) ----
+    // ---- 7a. the Golomb-Rice patches, while the host builds the codebooks ----
+    const uint8_t grk = golomb_rice_k(psum, P, false);
+    // Output sizes: Huffman and bit-pack streams are known exactly; the Golomb-Rice stream is
+    // bounded by P*(k+1) + sum(v >> k) <= P*(k+1) + (sum >> k) + P.
+    const unsigned __int128 gr_bound =
+        ext ? 0 : static_cast<unsigned __int128>(P) * (grk + 2) + (psum >> grk);
+    if (gr_bound > (static_cast<unsigned __int128>(1) << 40))
+        return fail(XNYZ_ERR_UNSUPPORTED, "Golomb-Rice stream larger than 2^40 bits");
+    const uint64_t bits_gr = static_cast<uint64_t>(gr_bound);
+    auto words_for = [](uint64_t bits) { return cdiv(bits, 32) + 4; };
+    Plan pe;
+    pe.total = pl.total;
+    const size_t o_w_gr = pe.add(4 * words_for(bits_gr));
+    const LookBackState lbs = lb_state(c, lb_enc);
+    auto job = [&](int ch, int kind, const void* in, uint64_t count, int k, size_t o_words, uint64_t bits) {
+        EncodeJob j{};
+        j.kind = kind;
+        j.k = k;
+        j.in = in;
+        j.n = count;
+        j.words = at<uint32_t>(c, o_words);
+        j.cap_bits = 32 * words_for(bits);
+        j.lb = LookBackState{lbs.flag + ch * lb_enc.tiles, lbs.agg + ch * lb_enc.tiles, lbs.inc + ch * lb_enc.tiles};
+        j.tile_counter = SMALL_FIELD(c, tile_counters[20 + ch]);
+        j.total_bits = SMALL_FIELD(c, totals[ch]);
+        return j;
+    };
+    EncodeArgs enc{};
+    enc.err = SMALL_FIELD(c, err);
+    const bool has_gr = P && !ext;
+    if (has_gr) enc.job[enc.count++] = job(0, direct ? kEncodeGolombRice64 : kEncodeGolombRice32, uo.patches, P, grk, o_w_gr, bits_gr);
+    // (few patches: with the other coders in one launch)
+    const bool gr_early = has_gr && P >= 65536 && pe.total <= c->arena.cap;
+    if (gr_early) {
+        Fills f;
+        f.add(at<uint32_t>(c, o_w_gr), 4 * words_for(bits_gr), 0);
+        launch_fill(f.a, st);
+        Prof pr(c, "encode_golomb_rice", 1, (direct ? 8.0 : 4.0) * P + bits_gr / 8.0);
+        launch_encode(enc, st);
+        enc.count = 0;
+    }
+    // ---- 7b. codebooks (host replay of the reference's container order) ----
     std::vector<SymbolStat> st_rep, st_quad, st_cnt;
     for (int s = 0; s < 256; ++s) {
         if (H.hist_rep[s]) st_rep.push_back(SymbolStat{static_cast<uint64_t>(s), H.hist_rep[s], H.first_rep[s]});
@@ -908,11 +980,13 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     StreamCode code_cnt;
     std::vector<uint32_t> sparse_val, sparse_bits;
     std::vector<uint8_t> sparse_len;
-    std::vector<uint32_t> dense_bits(kCountDense, 0);
-    std::vector<uint8_t> dense_len(kCountDense, 0);
+    uint32_t* const dense_bits = c->h_small->dense_bits;
+    uint8_t* const dense_len = c->h_small->dense_len;
+    std::memset(dense_bits, 0, 4 * (static_cast<size_t>(max_dense) + 1));
+    std::memset(dense_len, 0, static_cast<size_t>(max_dense) + 1);
     if (rle) {
-        for (int v = 0; v < kCountDense; ++v)
-            if (H.cnt_hist[v]) st_cnt.push_back(SymbolStat{static_cast<uint64_t>(v), H.cnt_hist[v], H.cnt_first[v]});
+        for (uint32_t v = 0; v <= max_dense; ++v)
+            if (H.bins[v].n) st_cnt.push_back(SymbolStat{v, H.bins[v].n, ~H.bins[v].inv_first});
         const uint32_t over = H.over_n;
         if (over) {
             std::vector<uint32_t> ov(over), ou(over);
@@ -961,8 +1035,6 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     };
     c->h_small->codes[0] = to_bytecodes(code_rep);
     c->h_small->codes[1] = to_bytecodes(code_quad);
-    CUDA_TRY(cudaMemcpyAsync(c->d_small->codes, c->h_small->codes, sizeof(ByteCodes) * 2, cudaMemcpyHostToDevice, st));
-    const uint8_t grk = golomb_rice_k(psum, P, false);
     int w_blk = 1, w_cnt = 1;
     if (!direct) {
         w_blk = H.max2[0] == 0 ? 1 : bitlen(H.max2[0]);
@@ -972,19 +1044,9 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     hp4.end();
     HostPhase hp5(c, "c5_encode");
     // ---- 8. encoders ----
-    // Output sizes: Huffman and bit-pack streams are known exactly; the Golomb-Rice stream is
-    // bounded by P*(k+1) + sum(v >> k) <= P*(k+1) + (sum >> k) + P.
     const uint64_t bits_rep = code_rep.encoded_bits, bits_quad = direct ? 0 : code_quad.encoded_bits;
     const uint64_t bits_cnt = rle ? code_cnt.encoded_bits : 0;
-    const unsigned __int128 gr_bound =
-        ext ? 0 : static_cast<unsigned __int128>(P) * (grk + 2) + (psum >> grk);
-    if (gr_bound > (static_cast<unsigned __int128>(1) << 40))
-        return fail(XNYZ_ERR_UNSUPPORTED, "Golomb-Rice stream larger than 2^40 bits");
-    const uint64_t bits_gr = static_cast<uint64_t>(gr_bound);
     const uint64_t ext_bits = ext ? H.ext_bits : 0;
-    auto words_for = [](uint64_t bits) { return cdiv(bits, 32) + 4; };
-    Plan pe;
-    pe.total = pl.total;
     // The block streams (widths of 8 and more) are packed straight into the device container, at
     // the places that the header and the stream lengths fix; else into the workspace.
     const uint64_t len_blk = direct ? 0 : cdiv(NB * static_cast<uint64_t>(w_blk), 8),
@@ -994,16 +1056,12 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
                in_cnt = to_device && !direct && w_cnt >= kPackDirectWidth;
     const size_t o_w_blk = pe.add(in_blk ? 0 : 4 * words_for(8 * len_blk));
     const size_t o_w_cnt = pe.add(in_cnt ? 0 : 4 * words_for(8 * len_cnt));
-    const size_t o_w_gr = pe.add(4 * words_for(bits_gr));
     const size_t o_w_rep = pe.add(4 * words_for(bits_rep));
     const size_t o_w_quad = pe.add(4 * words_for(bits_quad));
     const size_t o_w_cn = pe.add(4 * words_for(bits_cnt));
-    const size_t o_dense = pe.add(kCountDense * 5);
-    const size_t o_sparse = pe.add(sparse_val.size() * 9 + 16);
     const size_t o_w_xp = pe.add(4 * words_for(ext_bits));
-    // zeroed for the encoders: all but the directly packed block streams
-    const size_t enc_begin = w_blk >= kPackDirectWidth && w_cnt >= kPackDirectWidth ? o_w_gr : o_w_blk,
-                 enc_end = pe.total;
+    const size_t zero_end = pe.total;
+    const size_t o_sparse = pe.add(sparse_val.size() * 9 + 16);
     if (pe.total > c->arena.cap) {
         // Growing would move the arena; the inputs above live in it.  Plan for the worst
         // case next time and redo this call.
@@ -1015,90 +1073,88 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
                                     cdiv(bits_cnt, 8) + (ext ? 10 * ext_nb + cdiv(ext_bits, 8) : 0)));
     uint8_t* const p_blk = in_blk ? c->d_container + at_blk : at<uint8_t>(c, o_w_blk);
     uint8_t* const p_cnt = in_cnt ? c->d_container + at_cnt : at<uint8_t>(c, o_w_cnt);
-    CUDA_TRY(cudaMemsetAsync(c->arena.base + enc_begin, 0, enc_end - enc_begin, st));
-    TRY(memset_small(c, offsetof(Small, totals), sizeof(unsigned long long) * 8, 0));
-    TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
-    TRY(lb_clear(c, lb_enc, 4));
-    const LookBackState lbs = lb_state(c, lb_enc);
-    auto chan = [&](int ch) {
-        return LookBackState{lbs.flag + ch * lb_enc.tiles, lbs.agg + ch * lb_enc.tiles, lbs.inc + ch * lb_enc.tiles};
-    };
+    {
+        Fills f;  // what the encoders OR into (block streams: only those of narrow widths)
+        if (has_gr && !gr_early) f.add(at<uint32_t>(c, o_w_gr), 4 * words_for(bits_gr), 0);
+        if (!direct && w_blk < kPackDirectWidth) f.add(at<uint32_t>(c, o_w_blk), 4 * words_for(8 * len_blk), 0);
+        if (!direct && w_cnt < kPackDirectWidth) f.add(at<uint32_t>(c, o_w_cnt), 4 * words_for(8 * len_cnt), 0);
+        f.add(at<uint32_t>(c, o_w_rep), zero_end - o_w_rep, 0);
+        launch_fill(f.a, st);
+    }
+    // code tables: the byte codes and (-rle) the dense count table in one copy
+    CUDA_TRY(cudaMemcpyAsync(c->d_small->codes, c->h_small->codes,
+                             sizeof(ByteCodes) * 2 + (rle ? 4 * (static_cast<size_t>(max_dense) + 1) : 0),
+                             cudaMemcpyHostToDevice, st));
     if (!direct) {
         Prof pr(c, "bitpack", 1, 12.0 * NB + (w_blk + w_cnt) * NB / 8.0);
         launch_block_pack(uo.blk_id, uo.blk_unit, NB, U, {p_blk, at<uint32_t>(c, o_w_blk), w_blk},
                           {p_cnt, at<uint32_t>(c, o_w_cnt), w_cnt}, st);
     }
-    // The four entropy coders are independent: one side stream each.
-    uint32_t* dbits = at<uint32_t>(c, o_dense);
-    uint8_t* dlen = reinterpret_cast<uint8_t*>(dbits + kCountDense);
-    uint32_t* sval = at<uint32_t>(c, o_sparse);
-    uint32_t* sbits = sval + sparse_val.size();
-    uint8_t* slen = reinterpret_cast<uint8_t*>(sbits + sparse_val.size());
-    if (rle) {
-        CUDA_TRY(cudaMemcpyAsync(dbits, dense_bits.data(), 4 * kCountDense, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(dlen, dense_len.data(), kCountDense, cudaMemcpyHostToDevice, st));
-        if (!sparse_val.empty()) {
-            CUDA_TRY(cudaMemcpyAsync(sval, sparse_val.data(), 4 * sparse_val.size(), cudaMemcpyHostToDevice, st));
-            CUDA_TRY(cudaMemcpyAsync(sbits, sparse_bits.data(), 4 * sparse_val.size(), cudaMemcpyHostToDevice, st));
-            CUDA_TRY(cudaMemcpyAsync(slen, sparse_len.data(), sparse_val.size(), cudaMemcpyHostToDevice, st));
-        }
-    }
-    TRY(fork_sides(c));
     if (ext && U) {
-        Prof pr(c, "encode_blocks", 1, 8.0 * U + ext_bits / 8.0, side(c, 0));
+        Prof pr(c, "encode_blocks", 1, 8.0 * U + ext_bits / 8.0);
         launch_block_encode(at<unsigned long long>(c, cp.o_repval), U, at<uint8_t>(c, cp.o_xw), at<uint8_t>(c, cp.o_xk),
-                            at<unsigned long long>(c, cp.o_xoff), at<uint32_t>(c, o_w_xp), side(c, 0));
-    }
-    if (P && !ext) {
-        Prof pr(c, "encode_golomb_rice", 1, 8.0 * P + bits_gr / 8.0, side(c, 0));
-        launch_gr_encode(uo.patches, P, grk, at<uint32_t>(c, o_w_gr), 32 * words_for(bits_gr), chan(0),
-                         SMALL_FIELD(c, tile_counters[0]), SMALL_FIELD(c, totals[0]), SMALL_FIELD(c, err), side(c, 0));
+                            at<unsigned long long>(c, cp.o_xoff), at<uint32_t>(c, o_w_xp), st);
     }
     // A code whose codewords all have one length (quads at fine bounds: eight 3-bit codes;
     // most -rle count streams: two 1-bit codes) places symbol i at bits [i L, (i + 1) L).
     const int fl_rep = fixed_code_len(c->h_small->codes[0].len, 256);
     const int fl_quad = fixed_code_len(c->h_small->codes[1].len, 256);
-    const int fl_cnt = (rle && !code_cnt.exp_golomb && sparse_val.empty()) ? fixed_code_len(dense_len.data(), kCountDense) : 0;
-    if (!ext && !code_rep.exp_golomb) {
-        Prof pr(c, "encode_huffman", 1, 1.0 * U + bits_rep / 8.0, side(c, 1));
-        if (fl_rep)
-            launch_fixed_encode_u8(uo.rep_sym, U, c->d_small->codes[0].bits, fl_rep, at<uint32_t>(c, o_w_rep),
-                                   SMALL_FIELD(c, totals[1]), side(c, 1));
-        else
-            launch_huff_encode_u8(uo.rep_sym, U, &c->d_small->codes[0], at<uint32_t>(c, o_w_rep), 32 * words_for(bits_rep),
-                                  chan(1), SMALL_FIELD(c, tile_counters[1]), SMALL_FIELD(c, totals[1]), SMALL_FIELD(c, err),
-                                  side(c, 1));
+    const int fl_cnt = (rle && !code_cnt.exp_golomb && sparse_val.empty()) ? fixed_code_len(dense_len, max_dense + 1) : 0;
+    double enc_bytes = (has_gr && !gr_early) ? (direct ? 8.0 : 4.0) * P + bits_gr / 8.0 : 0.0;
+    auto byte_job = [&](int ch, const uint8_t* in, int fixed, const ByteCodes* codes, size_t o_words, uint64_t bits) {
+        EncodeJob j = job(ch, fixed ? kEncodeFixedU8 : kEncodeHuffman, in, U, fixed, o_words, bits);
+        j.codes = codes;
+        j.bits = codes->bits;
+        enc.job[enc.count++] = j;
+        enc_bytes += 1.0 * U + bits / 8.0;
+    };
+    if (!ext && !code_rep.exp_golomb) byte_job(1, uo.rep_sym, fl_rep, &c->d_small->codes[0], o_w_rep, bits_rep);
+    if (!direct) byte_job(2, uo.quad_sym, fl_quad, &c->d_small->codes[1], o_w_quad, bits_quad);
+    if (rle) {
+        EncodeJob j = job(3, fl_cnt ? kEncodeFixedI32 : kEncodeCounts, at<int32_t>(c, o_counts), U,
+                          fl_cnt ? fl_cnt : code_cnt.exp_golomb ? code_cnt.eg_k : -1, o_w_cn, bits_cnt);
+        j.bits = c->d_small->dense_bits;
+        if (!fl_cnt && !code_cnt.exp_golomb) {
+            CUDA_TRY(cudaMemcpyAsync(c->d_small->dense_len, dense_len, static_cast<size_t>(max_dense) + 1, cudaMemcpyHostToDevice, st));
+            j.len = c->d_small->dense_len;
+            if (!sparse_val.empty()) {
+                uint32_t* sval = at<uint32_t>(c, o_sparse);
+                uint32_t* sbits = sval + sparse_val.size();
+                uint8_t* slen = reinterpret_cast<uint8_t*>(sbits + sparse_val.size());
+                CUDA_TRY(cudaMemcpyAsync(sval, sparse_val.data(), 4 * sparse_val.size(), cudaMemcpyHostToDevice, st));
+                CUDA_TRY(cudaMemcpyAsync(sbits, sparse_bits.data(), 4 * sparse_val.size(), cudaMemcpyHostToDevice, st));
+                CUDA_TRY(cudaMemcpyAsync(slen, sparse_len.data(), sparse_val.size(), cudaMemcpyHostToDevice, st));
+                j.sparse_val = sval;
+                j.sparse_bits = sbits;
+                j.sparse_len = slen;
+                j.sparse_n = static_cast<uint32_t>(sparse_val.size());
+            }
+        }
+        enc.job[enc.count++] = j;
+        enc_bytes += 4.0 * U + bits_cnt / 8.0;
     }
-    if (!direct) {
-        Prof pr(c, "encode_huffman", 1, 1.0 * U + bits_quad / 8.0, side(c, 2));
-        if (fl_quad)
-            launch_fixed_encode_u8(uo.quad_sym, U, c->d_small->codes[1].bits, fl_quad, at<uint32_t>(c, o_w_quad),
-                                   SMALL_FIELD(c, totals[2]), side(c, 2));
-        else
-            launch_huff_encode_u8(uo.quad_sym, U, &c->d_small->codes[1], at<uint32_t>(c, o_w_quad),
-                                  32 * words_for(bits_quad), chan(2), SMALL_FIELD(c, tile_counters[2]),
-                                  SMALL_FIELD(c, totals[2]), SMALL_FIELD(c, err), side(c, 2));
-    }
-    if (rle && fl_cnt) {
-        Prof pr(c, "encode_counts", 1, 4.0 * U + bits_cnt / 8.0, side(c, 3));
-        launch_fixed_encode_i32(at<int32_t>(c, o_counts), U, dbits, fl_cnt, at<uint32_t>(c, o_w_cn),
-                                SMALL_FIELD(c, totals[3]), side(c, 3));
-    } else if (rle) {
-        Prof pr(c, "encode_counts", 1, 4.0 * U + bits_cnt / 8.0, side(c, 3));
-        launch_count_encode(at<int32_t>(c, o_counts), U, code_cnt.exp_golomb ? code_cnt.eg_k : -1, dbits, dlen, sval,
-                            sbits, slen, static_cast<uint32_t>(sparse_val.size()), at<uint32_t>(c, o_w_cn),
-                            32 * words_for(bits_cnt), chan(3), SMALL_FIELD(c, tile_counters[3]),
-                            SMALL_FIELD(c, totals[3]), SMALL_FIELD(c, err), side(c, 3));
+    {
+        Prof pr(c, "encode", enc.count ? 1 : 0, enc_bytes);
+        launch_encode(enc, st);
     }
     CUDA_TRY(cudaGetLastError());
-    TRY(join_sides(c));
-    TRY(fetch_small(c, offsetof(Small, err), offsetof(Small, codewords) - offsetof(Small, err)));  // err .. totals
-    TRY(device_errors(c));
-    const uint64_t gr_bits = c->h_small->totals[0];
-    if (!ext && !code_rep.exp_golomb && c->h_small->totals[1] != bits_rep)
-        return fail(XNYZ_ERR_CUDA, "Huffman encoder size mismatch (repos)");
-    if (!direct && c->h_small->totals[2] != bits_quad) return fail(XNYZ_ERR_CUDA, "Huffman encoder size mismatch (quads)");
-    if (rle && c->h_small->totals[3] != bits_cnt) return fail(XNYZ_ERR_CUDA, "count encoder size mismatch");
+    // the encoders' sizes and errors, once the host has waited for them
+    auto check_encoders = [&]() -> xnyz_status {
+        TRY(device_errors(c));
+        if (!ext && !code_rep.exp_golomb && c->h_small->totals[1] != bits_rep)
+            return fail(XNYZ_ERR_CUDA, "Huffman encoder size mismatch (repos)");
+        if (!direct && c->h_small->totals[2] != bits_quad)
+            return fail(XNYZ_ERR_CUDA, "Huffman encoder size mismatch (quads)");
+        if (rle && c->h_small->totals[3] != bits_cnt) return fail(XNYZ_ERR_CUDA, "count encoder size mismatch");
+        return XNYZ_OK;
+    };
+    const size_t tot0 = offsetof(Small, over_n), tot_bytes = offsetof(Small, codewords) - tot0;  // err .. totals
+    uint64_t gr_bytes = 0;
+    if (!to_device) {
+        TRY(fetch_small(c, tot0, tot_bytes));
+        TRY(check_encoders());
+        if (has_gr) gr_bytes = cdiv(c->h_small->totals[0], 8);
+    }
 
     hp5.end();
     HostPhase hp6(c, "c6_container");
@@ -1132,7 +1188,8 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
                                   {at<uint32_t>(c, o_w_xp), cdiv(ext_bits, 8)}});
             K.stream({}, nullptr, 0);
         } else {
-            K.stream(gr_meta, at<uint32_t>(c, o_w_gr), P ? cdiv(gr_bits, 8) : 0);
+            if (to_device && has_gr) K.late_stream(gr_meta, at<uint32_t>(c, o_w_gr));
+            else K.stream(gr_meta, at<uint32_t>(c, o_w_gr), gr_bytes);
             K.stream(code_rep.meta, at<uint32_t>(c, o_w_rep), cdiv(bits_rep, 8));
         }
     };
@@ -1151,6 +1208,14 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     K.pod<float>(S.offset[0]);
     K.pod<float>(S.offset[1]);
     K.pod<float>(S.offset[2]);
+
+    if (to_device) {  // the container is laid out on the device, where the Golomb-Rice length is known
+        TRY(container_to_device(c, K, SMALL_FIELD(c, totals[0]), cdiv(bits_gr, 8)));
+        CUDA_TRY(cudaEventRecord(c->ev1, st));
+        TRY(fetch_small(c, tot0, tot_bytes));
+        TRY(check_encoders());
+        if (has_gr) K.size += cdiv(c->h_small->totals[0], 8);
+    }
 
     xnyz_compress_info& I = R.info;
     I.num_points = n;
@@ -1492,7 +1557,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
     TRY(memset_small(c, offsetof(Small, fallback), sizeof(uint32_t) * 8 * 2, 0));  // fallback + redone
     TRY(memset_small(c, offsetof(Small, codewords), sizeof(unsigned long long) * 8, 0));
-    CUDA_TRY(cudaMemcpyAsync(c->d_small->hil_inv, hm.inv.data(), 256, cudaMemcpyHostToDevice, st));
     auto upload = [&](const HuffTables& t, const TabOff& o) -> xnyz_status {
         if (!t.root.empty())
             CUDA_TRY(cudaMemcpyAsync(at<uint32_t>(c, o.root), t.root.data(), 4 * t.root.size(), cudaMemcpyHostToDevice, st));
@@ -1671,7 +1735,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             launch_count_total(at<int32_t>(c, o_counts), U, SMALL_FIELD(c, totals[0]), st);
         }
         CUDA_TRY(cudaGetLastError());
-        return fetch_small(c, offsetof(Small, err), offsetof(Small, tile_counters) - offsetof(Small, err));
+        return fetch_small(c, offsetof(Small, err), offsetof(Small, first_rep) - offsetof(Small, err));
     };
     TRY(count_total());
     // A stream with wide values is decoded again with 64-bit output, one that did not fall in step
@@ -1838,6 +1902,8 @@ xnyz_status xnyz_create(xnyz_ctx** out, int device, void* stream) {
     }
     CUDA_TRY(cudaMalloc(&c->d_small, sizeof(Small)));
     CUDA_TRY(cudaMemset(c->d_small, 0, sizeof(Small)));
+    CUDA_TRY(cudaMemcpy(c->d_small->hil_fwd, hilbert_machines().fwd.data(), 256, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(c->d_small->hil_inv, hilbert_machines().inv.data(), 256, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_small), sizeof(Small), cudaHostAllocDefault));
     std::memset(c->h_small, 0, sizeof(Small));
     CUDA_TRY(cudaEventCreate(&c->ev0));
@@ -1847,7 +1913,6 @@ xnyz_status xnyz_create(xnyz_ctx** out, int device, void* stream) {
         CUDA_TRY(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
         CUDA_TRY(cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming));
     }
-    (void)hilbert_machines();
     *out = c.release();
     return XNYZ_OK;
 }
@@ -2054,9 +2119,6 @@ xnyz_status xnyz_compress_device(xnyz_ctx* c, const float* xyz, uint64_t n, cons
     HostPhase hpa(c, "c7_assemble_device");
     const size_t clen = R.cont.size;
     if (c->d_container_cap < clen + 64) return fail(XNYZ_ERR_CUDA, "container larger than its bound");
-    TRY(container_to_device(c, R.cont));
-    CUDA_TRY(cudaEventRecord(c->ev1, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
     *dev_container = c->d_container;
     *container_len = clen;
     if (info) {
@@ -2548,7 +2610,6 @@ xnyz_status xnyz_stage_hilbert(xnyz_ctx* c, const uint64_t* dev_in, uint64_t n, 
     CUDA_TRY(cudaSetDevice(c->device));
     const auto& hm = hilbert_machines();
     uint8_t* tab = inverse ? c->d_small->hil_inv : c->d_small->hil_fwd;
-    CUDA_TRY(cudaMemcpyAsync(tab, inverse ? hm.inv.data() : hm.fwd.data(), 256, cudaMemcpyHostToDevice, c->stream));
     launch_hilbert(reinterpret_cast<const unsigned long long*>(dev_in), n, tab, static_cast<int>(iteration), 0u,
                    reinterpret_cast<unsigned long long*>(dev_out), c->stream);
     CUDA_TRY(cudaGetLastError());
@@ -2568,7 +2629,7 @@ xnyz_status xnyz_stage_sort(xnyz_ctx* c, uint64_t* dev_keys, uint32_t* dev_paylo
     TRY(ensure_arena(c, pl.total));
     SortBufs sb{{reinterpret_cast<unsigned long long*>(dev_keys), at<unsigned long long>(c, ok)},
                 {dev_payload, dev_payload ? at<uint32_t>(c, ov) : nullptr}};
-    TRY(memset_small(c, offsetof(Small, sort_hist), sizeof(uint32_t) * 8 * 256, 0));
+    TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * (64 + 8 * 256), 0));  // and sort_hist
     TRY(memset_small(c, offsetof(Small, err), sizeof(uint32_t), 0));
     launch_sort_histogram(sb.keys[0], n, passes, c->d_small->sort_hist, c->stream);
     int res = 0;

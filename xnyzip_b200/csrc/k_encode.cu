@@ -6,8 +6,9 @@
 //                 a three-channel chained scan (units, patches, blocks).
 //   count_stats   -rle count per unit and its histogram.
 //   block_max, block_pack  BitPacker<uint64_t> of the block-id and block-count deltas.
-//   gr_encode     GolombRiceCoder<uint64_t>::pack of the patches.
-//   huff_encode_* HuffmanEncoder<T>::encode / exp-Golomb encode with host-built codes.
+//   encode        the entropy coders: GolombRiceCoder<uint64_t>::pack of the patches,
+//                 HuffmanEncoder<T>::encode / exp-Golomb encode with host-built codes.
+//   gather        the container's pieces, at any alignment; fill: the call's zeroed state.
 //
 // Reference (paths relative to its source/): quantizer/block_quantizer.hpp:117-149 (LCP
 // streams), composer/block_compressor.hpp:110-114,146-147 (deltas), encoder/
@@ -38,18 +39,9 @@ __device__ __forceinline__ u64 direct_key_sfc(u64 k, const DirectKeyParams& kp) 
 }
 
 // Warp-aggregated histogram update with first-occurrence tracking; the lowest lane of a
-// group of equal symbols holds the smallest unit index (units grow with the lane).
-__device__ __forceinline__ void hist_add(u32* hist, u32* first, bool valid, u32 sym, u32 unit) {
-    const u32 peers = __match_any_sync(kFullMask, valid ? sym : (0x10000u | lane_id()));
-    if (valid && lane_id() == (u32)(__ffs(peers) - 1)) {
-        atomicAdd(&hist[sym], (u32)__popc(peers));
-        atomicMin(&first[sym], unit);
-    }
-}
-
-// The same update with the groups of equal symbols found through a per-warp bit mask in
-// shared memory (one atomicOr per lane) instead of match.any, which serialises on the
-// address-divergence pipe.  `masks` is zero on entry and on return.
+// group of equal symbols holds the smallest unit index (units grow with the lane).  The groups are
+// found through a per-warp bit mask in shared memory (one atomicOr per lane) instead of match.any,
+// which serialises on the address-divergence pipe.  `masks` is zero on entry and on return.
 __device__ __forceinline__ void hist_add_masked(u32* masks, u32* hist, u32* first, bool valid, u32 sym, u32 unit) {
     const u32 lane = lane_id();
     if (valid) atomicOr(&masks[sym], 1u << lane);
@@ -198,7 +190,9 @@ __global__ void __launch_bounds__(kThreads) units_kernel(const u64* __restrict__
             if (out.rep_val) out.rep_val[u] = vi;
             if (!DIRECT) out.quad_sym[u] = (u8)qsym;
             if (patch) {
-                out.patches[pp + __popc(pm & lt)] = vi;
+                const u64 at = pp + __popc(pm & lt);
+                if (DIRECT) static_cast<u64*>(out.patches)[at] = vi;
+                else static_cast<u32*>(out.patches)[at] = (u32)vi;  // 18-bit codes
                 mysum += vi;
             }
             if (!DIRECT && nblk) {
@@ -245,44 +239,77 @@ __global__ void __launch_bounds__(kThreads) units_kernel(const u64* __restrict__
     }
 }
 
-// -rle: count of each unit = distance to the next unit's first point.
-__global__ void __launch_bounds__(kThreads) count_stats_kernel(const u32* __restrict__ unit_pos, u64 units, u64 n,
+// -rle: count of each unit = distance to the next unit's first point, and the counts' histogram with
+// first occurrences (kept as ~unit, so that everything starts at zero).  Most counts are 1: those are
+// tallied by ballots in registers, the others go through the block's histogram.  Block b of a warp's
+// sequence is read two rounds at a time (293 -> 138 us for 64M units).  units and n are device values
+// when units_dev is given.
+__global__ void __launch_bounds__(kThreads) count_stats_kernel(const u32* __restrict__ unit_pos, u64 units,
+                                                               const unsigned long long* units_dev, u64 n,
                                                                i32* __restrict__ counts, CountStats cs) {
     __shared__ u32 sh[kCountDense], sf[kCountDense];
+    __shared__ u32 smax;
+    if (units_dev) units = *units_dev;
     for (int i = threadIdx.x; i < kCountDense; i += kThreads) {
         sh[i] = 0;
-        sf[i] = 0xffffffffu;
+        sf[i] = 0u;
     }
+    if (threadIdx.x == 0) smax = 0;
     __syncthreads();
-    const u64 stride = (u64)gridDim.x * kThreads;
-    const u64 start = (u64)blockIdx.x * kThreads + (threadIdx.x & ~31u);
-    for (u64 b0 = start; b0 < units; b0 += stride) {
-        const u64 u = b0 + lane_id();
-        const bool ok = u < units;
-        u32 c = 0;
-        if (ok) {
-            if (unit_pos) {
-                const u64 nxt = (u + 1 < units) ? (u64)unit_pos[u + 1] : n;
-                c = (u32)(nxt - unit_pos[u]);
-                counts[u] = (i32)c;
-            } else {  // counts given (cell tables)
-                c = (u32)counts[u];
+    const u32 lane = lane_id();
+    const u64 stride = (u64)gridDim.x * kThreads * 4;
+    u32 ones = 0, one_first = 0, top = 0;
+    for (u64 b0 = ((u64)blockIdx.x * kThreads + (threadIdx.x & ~31u)) * 4; b0 < units; b0 += stride) {
+        u32 at[4], nx[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const u64 u = b0 + 32 * r + lane;
+            if (!unit_pos) {
+                nx[r] = u < units ? (u32)counts[u] : 0u;
+                at[r] = 0;
+            } else {
+                at[r] = u < units ? __ldg(unit_pos + u) : 0u;
+                nx[r] = u + 1 < units ? __ldg(unit_pos + u + 1) : (u32)n;
             }
         }
-        const bool dense = ok && c < (u32)kCountDense;
-        hist_add(sh, sf, dense, c, (u32)u);
-        if (ok && !dense) {
-            const u32 slot = atomicAdd(cs.over_n, 1u);
-            cs.over_val[slot] = c;
-            cs.over_unit[slot] = (u32)u;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const u64 u = b0 + 32 * r + lane;
+            const bool ok = u < units;
+            const u32 c = nx[r] - at[r];
+            if (ok && unit_pos) counts[u] = (i32)c;
+            const u32 m1 = __ballot_sync(kFullMask, ok && c == 1u);
+            if (m1) {
+                ones += (u32)__popc(m1);
+                if (!one_first) one_first = ~((u32)(b0 + 32 * r) + (u32)__ffs(m1) - 1u);
+            }
+            if (ok && c != 1u) {
+                if (c < (u32)kCountDense) {
+                    atomicAdd(&sh[c], 1u);
+                    if (sf[c] < ~(u32)u) atomicMax(&sf[c], ~(u32)u);
+                    top = max(top, c);
+                } else {
+                    const u32 slot = atomicAdd(cs.over_n, 1u);
+                    cs.over_val[slot] = c;
+                    cs.over_unit[slot] = (u32)u;
+                }
+            }
         }
     }
+    if (lane == 0 && ones) {
+        atomicAdd(&sh[1], ones);
+        atomicMax(&sf[1], one_first);
+        top = max(top, 1u);
+    }
+    if (top) atomicMax(&smax, top);
     __syncthreads();
-    for (int i = threadIdx.x; i < kCountDense; i += kThreads)
+    const u32 last = smax;
+    for (u32 i = threadIdx.x; i <= last; i += kThreads)
         if (sh[i]) {
-            atomicAdd(&cs.hist[i], (u64)sh[i]);
-            atomicMin(&cs.first[i], sf[i]);
+            atomicAdd(&cs.bins[i].n, (u64)sh[i]);
+            atomicMax(&cs.bins[i].inv_first, sf[i]);
         }
+    if (threadIdx.x == 0 && last) atomicMax(cs.max_dense, last);
 }
 
 // Block b's id delta and count delta (u64, wrapping like the reference's in-place differences).
@@ -298,8 +325,10 @@ __device__ __forceinline__ void block_deltas(const u64* __restrict__ blk_id, con
 // Largest id delta and count delta (the bit widths of the two block streams).  Reads 12 B per block;
 // a thread takes four consecutive blocks.
 __global__ void __launch_bounds__(kThreads) block_max_kernel(const u64* __restrict__ blk_id,
-                                                             const u32* __restrict__ blk_unit, u64 nb, u32 units,
-                                                             u64* max2) {
+                                                             const u32* __restrict__ blk_unit,
+                                                             const unsigned long long* __restrict__ counters, u64* max2) {
+    const u64 nb = counters[2];
+    const u32 units = (u32)counters[0];
     __shared__ u64 sm[2][kThreads / 32];
     u64 m0 = 0, m1 = 0;
     const u64 stride = (u64)gridDim.x * kThreads * 4;
@@ -417,82 +446,124 @@ __global__ void __launch_bounds__(kThreads) block_pack_kernel(const u64* __restr
     pack_tile(s1, v1, tile, nb);
 }
 
-// Shared skeleton of the chained-scan encoders: stage a tile of inputs, give every element
-// its bit length, scan, look back, write.
-template <typename T>
-__device__ __forceinline__ u32 stage_tile(const T* __restrict__ in, u64 n, T* s, u32* slot, u32* tile_counter,
-                                          u32& tile, u64& base) {
-    tile = claim_tile(tile_counter, slot);
-    base = (u64)tile * kTile;
-    const u32 cnt = (u32)min((u64)kTile, n - base);
-    for (int i = 0; i < kItems; ++i) {
-        const u32 e = (u32)i * kThreads + threadIdx.x;
-        if (e < cnt) s[e] = in[base + e];
-    }
-    __syncthreads();
-    return cnt;
-}
+// ---------------------------------------------------------------- entropy coders ---------
+// A container's entropy coders (Golomb-Rice patches, repos / SFC symbols, quad symbols, counts) are
+// independent and run in one launch: each takes a range of the blocks.  (Four launches on side
+// streams forked and joined by events cost 13 more calls.)  Within a coder, tiles of 4096 values
+// are chained by their code lengths; fixed-length codes need no chain.
+constexpr u32 kStageWords = 5632;  // a tile's output: 44 bits per value
+union EncodeShared {
+    struct {
+        u64 scratch[16];
+        u64 sbase;
+        u32 slot;
+        u64 table[256];  // byte symbols: length << 32 | code
+        u32 out[kStageWords];
+    } c;
+    u32 fixed[256];
+};
 
-__device__ __forceinline__ u64 tile_bit_base(LookBackState lb, u32 tile, u64 tot, u64* sbase,
-                                             unsigned long long* total_bits, u32* err) {
+__device__ __forceinline__ u64 tile_bit_base(const EncodeJob& j, u32 tile, u64 tot, u64* sbase, u32* err) {
     if (threadIdx.x < 32) {
-        LookBack64 l{lb.flag, lb.agg, lb.inc};
+        LookBack64 l{j.lb.flag, j.lb.agg, j.lb.inc};
         const u64 before = warp_lookback_add(l, tile, tot, err);
         if (threadIdx.x == 0) {
             *sbase = before;
-            if (tile == gridDim.x - 1) *total_bits = before + tot;
+            if (tile == j.blocks - 1) *j.total_bits = before + tot;
         }
     }
     __syncthreads();
     return *sbase;
 }
 
-// Thread t codes the tile's values [16 t, 16 t + 16) as one run of consecutive codewords:
-// its values are read straight from global memory (two per 16-byte load) and kept in
-// registers for the length sum and the writes; the run's bits leave a word at a time
-// (LsbRun), so a thread makes about one memory operation per 32 bits of output.
-__global__ void __launch_bounds__(kThreads) gr_encode_kernel(const u64* __restrict__ vals, u64 n, int k, u32* words,
-                                                             u64 cap_bits, LookBackState lb, u32* tile_counter,
-                                                             unsigned long long* total_bits, u32* err) {
-    __shared__ u64 scratch[16];
-    __shared__ u32 slot;
-    __shared__ u64 sbase;
-    const u32 tile = claim_tile(tile_counter, &slot);
-    const u64 base = (u64)tile * kTile;
-    const u32 cnt = (u32)min((u64)kTile, n - base);
-    const u32 e0 = threadIdx.x * kItems;
-    u64 v[kItems];
-    const bool vec = e0 + kItems <= cnt && ((reinterpret_cast<uintptr_t>(vals + base + e0) & 15u) == 0);
-    if (vec) {
+// Where a tile's codewords (tot bits from stream bit `base`) are assembled: in shared memory, zeroed
+// here, when they fit, and then stored as whole words (the first and the last, shared with the
+// neighbouring tiles, are OR-ed); else straight in the output.  A thread's words lie some ten words
+// from the next thread's, so stores from the threads' runs touch a sector each: from shared memory
+// 64M Golomb-Rice codes of 18.5 bits take 464 us, straight 492.
+struct TileWriter {
+    u32* words;
+    u64 first;  // output word that `words` starts with
+    bool staged;
+    __device__ __forceinline__ TileWriter(const EncodeJob& j, EncodeShared& sh, u64 base, u64 tot) {
+        first = base >> 5;
+        const u64 n = ((base & 31u) + tot + 31) >> 5;
+        staged = n <= kStageWords;
+        words = staged ? sh.c.out : j.words + first;
+        if (staged)
+            for (u32 i = threadIdx.x; i < (u32)n; i += kThreads) sh.c.out[i] = 0u;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void finish(const EncodeJob& j, const EncodeShared& sh, u64 base, u64 tot) const {
+        if (!staged) return;
+        __syncthreads();
+        const u32 n = (u32)(((base & 31u) + tot + 31) >> 5);
+        for (u32 i = threadIdx.x; i < n; i += kThreads) {
+            const u32 v = sh.c.out[i];
+            if (i == 0 || i + 1 == n) {
+                if (v) atomicOr(&j.words[first + i], v);
+            } else {
+                j.words[first + i] = v;
+            }
+        }
+    }
+};
+
+// Sixteen consecutive values of a thread, whole 16-byte loads where they are all there.
+template <typename T>
+__device__ __forceinline__ void load16(const T* __restrict__ in, u32 have, T (&v)[16]) {
+    if (have >= 16u) {
+        constexpr int kVec = 16 / sizeof(T);
 #pragma unroll
-        for (int i = 0; i < kItems; i += 2) {
-            const ulonglong2 p = __ldg(reinterpret_cast<const ulonglong2*>(vals + base + e0 + i));
-            v[i] = p.x;
-            v[i + 1] = p.y;
+        for (int i = 0; i < 16; i += kVec) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(in + i));
+            const u32 w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int e = 0; e < kVec; ++e) {
+                if (sizeof(T) == 8) v[i + e] = (T)((u64)w[2 * e] | ((u64)w[2 * e + 1] << 32));
+                else if (sizeof(T) == 4) v[i + e] = (T)w[e];
+                else v[i + e] = (T)(w[e / 4] >> (8 * (e % 4)));
+            }
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < kItems; ++i) v[i] = e0 + i < cnt ? __ldg(vals + base + e0 + i) : 0ull;
+        for (int i = 0; i < 16; ++i) v[i] = i < (int)have ? in[i] : (T)0;
     }
+}
+
+// Thread t codes the tile's values [16 t, 16 t + 16) as one run of consecutive codewords, kept in
+// registers for the length sum and the writes; the run's bits leave a word at a time (LsbRun).
+template <typename T>
+__device__ __forceinline__ void gr_encode_tile(const EncodeJob& j, EncodeShared& sh, u32* err) {
+    const int k = j.k;
+    const u32 tile = claim_tile(j.tile_counter, &sh.c.slot);
+    const u64 base = (u64)tile * kTile;
+    const u32 cnt = (u32)min((u64)kTile, j.n - base);
+    const u32 e0 = threadIdx.x * kItems;
+    const u32 have = e0 < cnt ? min(cnt - e0, 16u) : 0u;
+    T v[16];
+    load16(static_cast<const T*>(j.in) + base + e0, have, v);
     u64 sum = 0;
 #pragma unroll
     for (int i = 0; i < kItems; ++i)
-        if (e0 + i < cnt) sum += (v[i] >> k) + 1u + (u64)k;
+        if (i < (int)have) sum += ((u64)v[i] >> k) + 1u + (u64)k;
     u64 tot;
-    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, scratch, tot);
-    const u64 pos = tile_bit_base(lb, tile, tot, &sbase, total_bits, err) + ex;
-    if (pos + sum > cap_bits) {  // output bound (never reached with valid sizes)
-        if (sum) atomicOr(err, kErrOverflow);
+    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, sh.c.scratch, tot);
+    const u64 at = tile_bit_base(j, tile, tot, &sh.c.sbase, err);
+    if (at + tot > j.cap_bits) {  // output bound (never reached with valid sizes)
+        if (tot) atomicOr(err, kErrOverflow);
         return;
     }
+    const TileWriter out(j, sh, at, tot);
+    const u64 pos = (at & 31u) + ex;
     const u64 mask = k ? ((1ull << k) - 1) : 0ull;
     LsbRun run;
-    run.begin(words, pos);
+    run.begin(out.words, pos);
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
-        if (e0 + i >= cnt) continue;
-        const u64 q = v[i] >> k;
-        const u64 r = v[i] & mask;
+        if (i >= (int)have) continue;
+        const u64 q = (u64)v[i] >> k;
+        const u64 r = (u64)v[i] & mask;
         if (q + 1u + (u64)k <= 32u) {  // unary part, terminating zero and remainder in one piece
             run.put32((u32)((q ? ((1ull << q) - 1) : 0ull) | (r << (q + 1))), (u32)(q + 1u + (u64)k));
         } else {
@@ -502,104 +573,100 @@ __global__ void __launch_bounds__(kThreads) gr_encode_kernel(const u64* __restri
         }
     }
     run.end();
+    out.finish(j, sh, at, tot);
 }
 
-__global__ void __launch_bounds__(kThreads) huff_encode_u8_kernel(const u8* __restrict__ sym, u64 n,
-                                                                  const ByteCodes* __restrict__ codes, u32* words,
-                                                                  u64 cap_bits, LookBackState lb, u32* tile_counter,
-                                                                  unsigned long long* total_bits, u32* err) {
-    __shared__ u8 ss[kTile];
-    __shared__ u32 cbits[256];
-    __shared__ u8 clen[256];
-    __shared__ u64 scratch[16];
-    __shared__ u32 slot;
-    __shared__ u64 sbase;
-    cbits[threadIdx.x] = codes->bits[threadIdx.x];
-    clen[threadIdx.x] = codes->len[threadIdx.x];
-    u32 tile;
-    u64 base;
-    const u32 cnt = stage_tile(sym, n, ss, &slot, tile_counter, tile, base);
+__device__ __forceinline__ void huff_encode_tile(const EncodeJob& j, EncodeShared& sh, u32* err) {
+    const ByteCodes* codes = static_cast<const ByteCodes*>(j.codes);
+    sh.c.table[threadIdx.x] = ((u64)codes->len[threadIdx.x] << 32) | codes->bits[threadIdx.x];
+    const u32 tile = claim_tile(j.tile_counter, &sh.c.slot);
+    const u64 base = (u64)tile * kTile;
+    const u32 cnt = (u32)min((u64)kTile, j.n - base);
     const u32 e0 = threadIdx.x * kItems;
+    const u32 have = e0 < cnt ? min(cnt - e0, 16u) : 0u;
+    u8 v[16];
+    load16(static_cast<const u8*>(j.in) + base + e0, have, v);
     u64 sum = 0;
 #pragma unroll
     for (int i = 0; i < kItems; ++i)
-        if (e0 + i < cnt) sum += clen[ss[e0 + i]];
+        if (i < (int)have) sum += sh.c.table[v[i]] >> 32;
     u64 tot;
-    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, scratch, tot);
-    u64 pos = tile_bit_base(lb, tile, tot, &sbase, total_bits, err) + ex;
-    if (pos + sum > cap_bits) {  // output bound (never reached with valid sizes)
-        if (sum) atomicOr(err, kErrOverflow);
+    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, sh.c.scratch, tot);
+    const u64 at = tile_bit_base(j, tile, tot, &sh.c.sbase, err);
+    if (at + tot > j.cap_bits) {  // output bound (never reached with valid sizes)
+        if (tot) atomicOr(err, kErrOverflow);
         return;
     }
+    const TileWriter out(j, sh, at, tot);
+    const u64 pos = (at & 31u) + ex;
     MsbRun run;
-    run.begin(words, pos);
-#pragma unroll 4
+    run.begin(out.words, pos);
+#pragma unroll
     for (int i = 0; i < kItems; ++i) {
-        if (e0 + i >= cnt) break;
-        const u32 s = ss[e0 + i];
-        const u32 len = clen[s];
+        if (i >= (int)have) continue;
+        const u64 e = sh.c.table[v[i]];
+        const u32 len = (u32)(e >> 32);
         // Codes longer than 32 bits are the 32-bit value zero-extended (huffman_encoder.hpp:251).
         if (len > 32u) {
             run.zeros(len - 32u);
-            run.put32(cbits[s], 32u);
+            run.put32((u32)e, 32u);
         } else {
-            run.put32(cbits[s], len);
+            run.put32((u32)e, len);
         }
     }
     run.end();
+    out.finish(j, sh, at, tot);
 }
 
 // A prefix code whose codewords all have one length L (1..24 bits): symbol i occupies stream
 // bits [i L, (i + 1) L), so no scan is needed.  Thread g codes symbols [32 g, 32 g + 32), whose
 // 32 L bits fill exactly words [g L, g L + L), MSB-first and stored byte-swapped as MsbRun
-// stores them; whole words, no atomics.  Symbols index code_bits (counts: the dense table).
+// stores them; whole words, no atomics.  Symbols index j.bits (counts: the dense table).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) fixed_encode_kernel(const T* __restrict__ sym, u64 n,
-                                                                const u32* __restrict__ code_bits, int len,
-                                                                u32* __restrict__ words,
-                                                                unsigned long long* total_bits) {
-    const u64 g = (u64)blockIdx.x * kThreads + threadIdx.x;
-    const u64 total = n * (u64)len;
-    if (g == 0) *total_bits = total;
+__device__ __forceinline__ void fixed_encode_block(const EncodeJob& j, EncodeShared& sh, u32 block) {
+    const int len = j.k;
+    sh.fixed[threadIdx.x] = __ldg(&j.bits[threadIdx.x]);
+    __syncthreads();
+    const u64 g = (u64)block * kThreads + threadIdx.x;
+    const u64 total = j.n * (u64)len;
+    if (g == 0) *j.total_bits = total;
     const u64 s0 = g * 32u;
-    if (s0 >= n) return;
+    if (s0 >= j.n) return;
     const u32 mask = (1u << len) - 1u;
     u64 acc = 0, w = g * (u64)len;
     u32 nb = 0;
-#pragma unroll 4
-    for (int i = 0; i < 32; ++i) {
-        const u64 idx = s0 + (u64)i;
-        const u32 c = idx < n ? (__ldg(&code_bits[(u32)sym[idx]]) & mask) : 0u;
-        acc = (acc << len) | c;
-        nb += (u32)len;
-        if (nb >= 32u) {
-            nb -= 32u;
-            if (w * 32u < total) words[w] = __byte_perm((u32)(acc >> nb), 0, 0x0123);
-            ++w;
-            acc &= nb ? ((1ull << nb) - 1ull) : 0ull;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const u64 s = s0 + 16u * h;
+        const u32 have = s < j.n ? (u32)min(j.n - s, (u64)16) : 0u;
+        T v[16];
+        load16(static_cast<const T*>(j.in) + s, have, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const u32 x = (u32)v[i];
+            const u32 c = i < (int)have ? ((sizeof(T) == 1 || x < 256u ? sh.fixed[x & 255u] : __ldg(&j.bits[x])) & mask) : 0u;
+            acc = (acc << len) | c;
+            nb += (u32)len;
+            if (nb >= 32u) {
+                nb -= 32u;
+                if (w * 32u < total) j.words[w] = __byte_perm((u32)(acc >> nb), 0, 0x0123);
+                ++w;
+            }
         }
     }
 }
 
 __device__ __forceinline__ u32 rev_low(u64 v, int k) { return k ? (__brev((u32)v) >> (32 - k)) : 0u; }
 
-__global__ void __launch_bounds__(kThreads) count_encode_kernel(const i32* __restrict__ counts, u64 n, int eg_k,
-                                                                const u32* __restrict__ dense_bits,
-                                                                const u8* __restrict__ dense_len,
-                                                                const u32* __restrict__ sparse_val,
-                                                                const u32* __restrict__ sparse_bits,
-                                                                const u8* __restrict__ sparse_len, u32 sparse_n,
-                                                                u32* words, u64 cap_bits, LookBackState lb,
-                                                                u32* tile_counter,
-                                                                unsigned long long* total_bits, u32* err) {
-    __shared__ i32 sc[kTile];
-    __shared__ u64 scratch[16];
-    __shared__ u32 slot;
-    __shared__ u64 sbase;
-    u32 tile;
-    u64 base;
-    const u32 cnt = stage_tile(counts, n, sc, &slot, tile_counter, tile, base);
+__device__ __forceinline__ void count_encode_tile(const EncodeJob& j, EncodeShared& sh, u32* err) {
+    const u32 tile = claim_tile(j.tile_counter, &sh.c.slot);
+    const u64 base = (u64)tile * kTile;
+    const u32 cnt = (u32)min((u64)kTile, j.n - base);
     const u32 e0 = threadIdx.x * kItems;
+    const u32 have = e0 < cnt ? min(cnt - e0, 16u) : 0u;
+    i32 v[16];
+    load16(static_cast<const i32*>(j.in) + base + e0, have, v);
+    const int eg_k = j.k;
     // code of one count: (length, value bits, bit offset of the value inside the code)
     auto code = [&](i32 c, u32& len, u64& val, u32& nb) {
         if (eg_k >= 0) {
@@ -614,17 +681,17 @@ __global__ void __launch_bounds__(kThreads) count_encode_kernel(const i32* __res
             const u32 uc = (u32)c;
             u32 bits = 0, l = 0;
             if (uc < (u32)kCountDense) {
-                bits = dense_bits[uc];
-                l = dense_len[uc];
+                bits = __ldg(&j.bits[uc]);
+                l = __ldg(&j.len[uc]);
             } else {
-                u32 lo = 0, hi = sparse_n;
+                u32 lo = 0, hi = j.sparse_n;
                 while (lo < hi) {
                     const u32 mid = (lo + hi) >> 1;
-                    if (sparse_val[mid] < uc) lo = mid + 1; else hi = mid;
+                    if (j.sparse_val[mid] < uc) lo = mid + 1; else hi = mid;
                 }
-                if (lo < sparse_n && sparse_val[lo] == uc) {
-                    bits = sparse_bits[lo];
-                    l = sparse_len[lo];
+                if (lo < j.sparse_n && j.sparse_val[lo] == uc) {
+                    bits = j.sparse_bits[lo];
+                    l = j.sparse_len[lo];
                 } else {
                     atomicOr(err, kErrOverflow);
                 }
@@ -635,31 +702,68 @@ __global__ void __launch_bounds__(kThreads) count_encode_kernel(const i32* __res
         }
     };
     u64 sum = 0;
+#pragma unroll 4
     for (int i = 0; i < kItems; ++i)
-        if (e0 + i < cnt) {
+        if (i < (int)have) {
             u32 len, nb;
             u64 val;
-            code(sc[e0 + i], len, val, nb);
+            code(v[i], len, val, nb);
             sum += len;
         }
     u64 tot;
-    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, scratch, tot);
-    u64 pos = tile_bit_base(lb, tile, tot, &sbase, total_bits, err) + ex;
-    if (pos + sum > cap_bits) {  // output bound (never reached with valid sizes)
-        if (sum) atomicOr(err, kErrOverflow);
+    const u64 ex = block_exclusive<kThreads>(sum, 0ull, AddOp{}, sh.c.scratch, tot);
+    const u64 at = tile_bit_base(j, tile, tot, &sh.c.sbase, err);
+    if (at + tot > j.cap_bits) {  // output bound (never reached with valid sizes)
+        if (tot) atomicOr(err, kErrOverflow);
         return;
     }
+    const TileWriter out(j, sh, at, tot);
+    const u64 pos = (at & 31u) + ex;
     MsbRun run;
-    run.begin(words, pos);
+    run.begin(out.words, pos);
+#pragma unroll 4
     for (int i = 0; i < kItems; ++i) {
-        if (e0 + i >= cnt) break;
+        if (i >= (int)have) continue;
         u32 len, nb;
         u64 val;
-        code(sc[e0 + i], len, val, nb);
+        code(v[i], len, val, nb);
         run.zeros(len - nb);  // exp-Golomb's leading zeros, or a long Huffman code's extension
         run.put(val, nb);
     }
     run.end();
+    out.finish(j, sh, at, tot);
+}
+
+__global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant__ EncodeArgs a) {
+    __shared__ EncodeShared sh;
+    u32 b = blockIdx.x;
+    int i = 0;
+    while (b >= a.job[i].blocks) b -= a.job[i++].blocks;
+    const EncodeJob& j = a.job[i];
+    switch (j.kind) {
+        case kEncodeGolombRice32: gr_encode_tile<u32>(j, sh, a.err); break;
+        case kEncodeGolombRice64: gr_encode_tile<u64>(j, sh, a.err); break;
+        case kEncodeHuffman: huff_encode_tile(j, sh, a.err); break;
+        case kEncodeFixedU8: fixed_encode_block<u8>(j, sh, b); break;
+        case kEncodeFixedI32: fixed_encode_block<i32>(j, sh, b); break;
+        default: count_encode_tile(j, sh, a.err); break;
+    }
+}
+
+// Sets ranges of 4-byte words (a call's counters, histograms, look-back flags and OR-ed output words)
+// in one launch instead of a memset each.
+__global__ void __launch_bounds__(kThreads) fill_kernel(const __grid_constant__ FillArgs a) {
+    const u64 t = (u64)blockIdx.x * kThreads + threadIdx.x, stride = (u64)gridDim.x * kThreads;
+    for (int i = 0; i < a.count; ++i) {
+        const FillRange r = a.range[i];
+        u32* p = static_cast<u32*>(r.p);
+        const u64 head = min((u64)r.words, (u64)((16u - (u32)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) / 4u);
+        const u64 vecs = (r.words - head) / 4;
+        uint4* v = reinterpret_cast<uint4*>(p + head);
+        for (u64 x = t; x < vecs; x += stride) v[x] = make_uint4(r.value, r.value, r.value, r.value);
+        if (t < head) p[t] = r.value;
+        if (t < r.words - head - 4 * vecs) p[head + 4 * vecs + t] = r.value;
+    }
 }
 
 // One block per 16 KB of the destination (by its address) and piece.  The body goes out 16 bytes per
@@ -668,10 +772,12 @@ __global__ void __launch_bounds__(kThreads) count_encode_kernel(const i32* __res
 constexpr u64 kGatherChunk = 16384;
 __global__ void __launch_bounds__(kThreads) gather_kernel(const __grid_constant__ GatherArgs a, u8* __restrict__ dst) {
     u64 c = blockIdx.x;
+    const u64 late = a.late_bits ? min((u64)(*a.late_bits + 7) / 8, (u64)a.late_most) : 0ull;
     for (int i = 0; i < a.count; ++i) {
         const GatherPiece& p = a.piece[i];
-        const u64 d0 = reinterpret_cast<u64>(dst) + p.off, d1 = d0 + p.len;
-        const u64 chunks = p.len ? (d1 - 1) / kGatherChunk - d0 / kGatherChunk + 1 : 0ull;
+        const u64 len = p.kind == kGatherLate ? late : p.len;
+        const u64 d0 = reinterpret_cast<u64>(dst) + p.off + (p.after ? late : 0ull), d1 = d0 + len;
+        const u64 chunks = len ? (d1 - 1) / kGatherChunk - d0 / kGatherChunk + 1 : 0ull;
         if (c >= chunks) {
             c -= chunks;
             continue;
@@ -680,7 +786,9 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(const __grid_constant_
         const u64 lo = max(base, d0), hi = min(base + kGatherChunk, d1);
         if (!p.src) {
             for (u64 x = lo + threadIdx.x; x < hi; x += kThreads)
-                *reinterpret_cast<u8*>(x) = p.zero ? (u8)0 : a.inline_bytes[p.inline_off + (u32)(x - d0)];
+                *reinterpret_cast<u8*>(x) = p.kind == kGatherZero      ? (u8)0
+                                            : p.kind == kGatherLateLen ? (u8)(late >> (8 * (x - d0)))
+                                                                       : a.inline_bytes[p.inline_off + (u32)(x - d0)];
             return;
         }
         const u64 s0 = reinterpret_cast<u64>(p.src) - d0;  // source address = destination address + s0
@@ -724,13 +832,13 @@ void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, Di
     if (!tiles) return;
     units_kernel<true><<<tiles, kThreads, 0, st>>>(keys, n, rle, BlockKeyParams{}, kp, out, lb, tile_counter, err);
 }
-void launch_count_stats(const uint32_t* unit_pos, uint64_t units, uint64_t n, int32_t* counts, CountStats cs,
-                        cudaStream_t st) {
-    count_stats_kernel<<<persistent_grid(units), kThreads, 0, st>>>(unit_pos, units, n, counts, cs);
+void launch_count_stats(const uint32_t* unit_pos, uint64_t units, const unsigned long long* units_dev, uint64_t n,
+                        int32_t* counts, CountStats cs, cudaStream_t st) {
+    count_stats_kernel<<<persistent_grid((units + 3) / 4), kThreads, 0, st>>>(unit_pos, units, units_dev, n, counts, cs);
 }
-void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
-                      unsigned long long* max2, cudaStream_t st) {
-    block_max_kernel<<<persistent_grid(nblocks), kThreads, 0, st>>>(blk_id, blk_unit, nblocks, (u32)units, max2);
+void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t most_blocks,
+                      const unsigned long long* counters, unsigned long long* max2, cudaStream_t st) {
+    block_max_kernel<<<persistent_grid((most_blocks + 3) / 4), kThreads, 0, st>>>(blk_id, blk_unit, counters, max2);
 }
 void launch_block_pack(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
                        const BlockPackDst& blk, const BlockPackDst& cnt, cudaStream_t st) {
@@ -747,51 +855,27 @@ void launch_block_pack(const unsigned long long* blk_id, const uint32_t* blk_uni
     const unsigned blocks = (unsigned)((nblocks + kPackTile - 1) / kPackTile);
     block_pack_kernel<<<blocks, kThreads, 0, st>>>(blk_id, blk_unit, nblocks, (u32)units, stream(blk), stream(cnt));
 }
+void launch_fill(const FillArgs& a, cudaStream_t st) {
+    u64 most = 0;
+    for (int i = 0; i < a.count; ++i) most = a.range[i].words > most ? a.range[i].words : most;
+    if (most) fill_kernel<<<persistent_grid((most + 3) / 4), kThreads, 0, st>>>(a);
+}
 void launch_gather(const GatherArgs& a, uint8_t* dst, cudaStream_t st) {
     u64 blocks = 0;
     for (int i = 0; i < a.count; ++i) {
-        const u64 d0 = reinterpret_cast<u64>(dst) + a.piece[i].off, d1 = d0 + a.piece[i].len;
-        if (a.piece[i].len) blocks += (d1 - 1) / kGatherChunk - d0 / kGatherChunk + 1;
+        // at most this many, wherever the late stream's length puts the piece
+        if (a.piece[i].len) blocks += (a.piece[i].len + kGatherChunk - 2) / kGatherChunk + 1;
     }
     if (blocks) gather_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a, dst);
 }
-void launch_gr_encode(const unsigned long long* vals, uint64_t n, int k, uint32_t* words, uint64_t cap_bits,
-                      LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits, uint32_t* err,
-                      cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
-    if (!tiles) return;
-    gr_encode_kernel<<<tiles, kThreads, 0, st>>>(vals, n, k, words, cap_bits, lb, tile_counter, total_bits, err);
-}
-void launch_fixed_encode_u8(const uint8_t* sym, uint64_t n, const uint32_t* code_bits, int len, uint32_t* words,
-                            unsigned long long* total_bits, cudaStream_t st) {
-    const u64 threads = (n + 31) / 32;
-    const unsigned blocks = (unsigned)((threads + kThreads - 1) / kThreads);
-    fixed_encode_kernel<u8><<<blocks ? blocks : 1, kThreads, 0, st>>>(sym, n, code_bits, len, words, total_bits);
-}
-void launch_fixed_encode_i32(const int32_t* sym, uint64_t n, const uint32_t* code_bits, int len, uint32_t* words,
-                             unsigned long long* total_bits, cudaStream_t st) {
-    const u64 threads = (n + 31) / 32;
-    const unsigned blocks = (unsigned)((threads + kThreads - 1) / kThreads);
-    fixed_encode_kernel<i32><<<blocks ? blocks : 1, kThreads, 0, st>>>(sym, n, code_bits, len, words, total_bits);
-}
-void launch_huff_encode_u8(const uint8_t* sym, uint64_t n, const ByteCodes* codes, uint32_t* words,
-                           uint64_t cap_bits, LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits,
-                           uint32_t* err, cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
-    if (!tiles) return;
-    huff_encode_u8_kernel<<<tiles, kThreads, 0, st>>>(sym, n, codes, words, cap_bits, lb, tile_counter, total_bits,
-                                                      err);
-}
-void launch_count_encode(const int32_t* counts, uint64_t n, int eg_k, const uint32_t* dense_bits,
-                         const uint8_t* dense_len, const uint32_t* sparse_val, const uint32_t* sparse_bits,
-                         const uint8_t* sparse_len, uint32_t sparse_n, uint32_t* words, uint64_t cap_bits,
-                         LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits, uint32_t* err,
-                         cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
-    if (!tiles) return;
-    count_encode_kernel<<<tiles, kThreads, 0, st>>>(counts, n, eg_k, dense_bits, dense_len, sparse_val, sparse_bits,
-                                                    sparse_len, sparse_n, words, cap_bits, lb, tile_counter,
-                                                    total_bits, err);
+void launch_encode(EncodeArgs a, cudaStream_t st) {
+    u64 blocks = 0;
+    for (int i = 0; i < a.count; ++i) {
+        const u64 per = a.job[i].kind == kEncodeFixedU8 || a.job[i].kind == kEncodeFixedI32 ? 32ull * kThreads : (u64)kTile;
+        a.job[i].blocks = (u32)((a.job[i].n + per - 1) / per);
+        blocks += a.job[i].blocks;
+    }
+    if (blocks) encode_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(a);
 }
 
 }  // namespace dev

@@ -268,35 +268,9 @@ __device__ __forceinline__ u64 block_key(i32 x, i32 y, i32 z, const BlockKeyPara
     return kp.defect_flag | (xy << 21) | low;  // z == -1: id = xy + defect_base
 }
 
-__global__ void __launch_bounds__(kThreads) keys_block_kernel(const float* __restrict__ xyz, u64 n, QuantParams q,
-                                                              const PointStats* stats, BlockKeyParams kp,
-                                                              const u8* __restrict__ htab_g,
-                                                              unsigned long long* __restrict__ keys,
-                                                              u32* __restrict__ payload, int passes, u32* hist) {
-    __shared__ float off[3];
-    __shared__ u8 htab[256];
-    __shared__ u32 sh[8 * 256];
-    if (threadIdx.x == 0) load_offset(xyz, stats, off);
-    stage_hilbert_table(htab_g, htab);
-    for (int i = threadIdx.x; i < passes * 256; i += kThreads) sh[i] = 0;
-    __syncthreads();
-    DigitHist dh{sh, passes};
-    for_each_point<4>(xyz, n, [&](u64 i, float fx, float fy, float fz) {
-        const float px = __fsub_rn(fx, off[0]), py = __fsub_rn(fy, off[1]), pz = __fsub_rn(fz, off[2]);
-        i32 x, y, z;
-        quantize(q, px, py, pz, x, y, z);
-        const u64 k = block_key(x, y, z, kp, htab);
-        keys[i] = k;
-        if (payload) payload[i] = (u32)i;
-        if (passes) dh.add(k);
-    });
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * 256; i += kThreads)
-        if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
-
-// Cell tables (encode_cells_with_counts, composer/block_compressor_rle.hpp:341-470): block
-// keys straight from int32 lattice cells, and the per-axis minima / maxima of the cells.
+// Block keys from int32 lattice cells: those that the quantization sweep kept, or a cell table's
+// (encode_cells_with_counts, composer/block_compressor_rle.hpp:341-470), for which
+// cells_stats_kernel takes the per-axis minima / maxima.
 __global__ void __launch_bounds__(kThreads) keys_cells_kernel(const i32* __restrict__ cells, u64 n, BlockKeyParams kp,
                                                               const u8* __restrict__ htab_g,
                                                               unsigned long long* __restrict__ keys,
@@ -483,12 +457,6 @@ void launch_adaptive_steps(const float* xyz, float l2, PointStats* stats, cudaSt
 void launch_quantize_range(const float* xyz, uint64_t n, QuantParams q, PointStats* stats, int with_error_stats,
                            cudaStream_t st, int32_t* cells) {
     quantize_range_kernel<<<grid_for(n), kThreads, 0, st>>>(xyz, n, q, stats, with_error_stats, cells);
-}
-void launch_keys_block(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, BlockKeyParams kp,
-                       const uint8_t* hilbert_tab, unsigned long long* keys, uint32_t* payload, int passes,
-                       uint32_t* hist, cudaStream_t st) {
-    keys_block_kernel<<<grid_for(n), kThreads, 0, st>>>(xyz, n, q, stats, kp, hilbert_tab, keys, payload, passes,
-                                                        hist);
 }
 void launch_keys_direct(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, DirectKeyParams kp,
                         const uint8_t* hilbert_tab, unsigned long long* keys, uint32_t* payload, int passes,

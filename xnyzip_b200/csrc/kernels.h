@@ -58,7 +58,7 @@ struct DirectKeyParams {
 struct UnitOutputs {
     uint8_t* rep_sym;               // PFor symbol of repos / sfc delta per unit
     uint8_t* quad_sym;              // PFor symbol of the quad delta per unit (block mode)
-    unsigned long long* patches;    // PFor patches in order
+    void* patches;                  // PFor patches in order: u32 in block mode (18-bit codes), u64 in direct mode
     unsigned long long* blk_id;     // block mode: id of each block
     uint32_t* blk_unit;             // block mode: first unit of each block
     uint32_t* unit_pos;             // -rle: sorted position of each unit's first point
@@ -79,8 +79,13 @@ struct LookBackState {
 // Count-stream statistics (-rle).
 constexpr int kCountDense = 4096;
 struct CountStats {
-    unsigned long long* hist;   // [kCountDense]
-    uint32_t* first;            // [kCountDense]
+    struct Bin {                // of counts below kCountDense
+        unsigned long long n;
+        uint32_t inv_first;     // ~(first unit with this count), 0 when none
+        uint32_t unused;
+    };
+    Bin* bins;                  // [kCountDense]
+    uint32_t* max_dense;        // largest such count
     uint32_t* over_val;         // counts >= kCountDense: value
     uint32_t* over_unit;        //   ... and unit index
     uint32_t* over_n;           // number of such counts
@@ -103,9 +108,6 @@ void launch_adaptive_steps(const float* xyz, float l2, PointStats* stats, cudaSt
 // cells (optional, 3 n int32): each finite point's lattice cell, for launch_keys_cells.
 void launch_quantize_range(const float* xyz, uint64_t n, QuantParams q, PointStats* stats, int with_error_stats,
                            cudaStream_t st, int32_t* cells = nullptr);
-void launch_keys_block(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, BlockKeyParams kp,
-                       const uint8_t* hilbert_tab, unsigned long long* keys, uint32_t* payload, int passes,
-                       uint32_t* hist, cudaStream_t st);
 void launch_keys_direct(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, DirectKeyParams kp,
                         const uint8_t* hilbert_tab, unsigned long long* keys, uint32_t* payload, int passes,
                         uint32_t* hist, cudaStream_t st);
@@ -148,11 +150,12 @@ void launch_units_block(const unsigned long long* keys, uint64_t n, int rle, Blo
 void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, DirectKeyParams kp, UnitOutputs out,
                          LookBackState lb, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
 // unit_pos null: counts[] is the input (cell tables), else counts[] receives the run lengths.
-void launch_count_stats(const uint32_t* unit_pos, uint64_t units, uint64_t n, int32_t* counts, CountStats cs,
-                        cudaStream_t st);
-// Largest block-id delta and block-count delta, into max2[0] and max2[1].
-void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
-                      unsigned long long* max2, cudaStream_t st);
+void launch_count_stats(const uint32_t* unit_pos, uint64_t units, const unsigned long long* units_dev, uint64_t n,
+                        int32_t* counts, CountStats cs, cudaStream_t st);
+// Largest block-id delta and block-count delta, into max2[0] and max2[1].  counters[0] and [2] (device)
+// hold the units and blocks; most_blocks bounds the latter.
+void launch_block_max(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t most_blocks,
+                      const unsigned long long* counters, unsigned long long* max2, cudaStream_t st);
 // Bit-packs the block-id and block-count deltas (widths 1..64).  Widths from 8 on: written to the
 // ceil(nblocks width / 8) bytes at dst (any alignment), nothing else touched; narrower: OR-ed into
 // the zeroed words at `words`.
@@ -165,44 +168,71 @@ constexpr int kPackDirectWidth = 8;
 void launch_block_pack(const unsigned long long* blk_id, const uint32_t* blk_unit, uint64_t nblocks, uint64_t units,
                        const BlockPackDst& blk, const BlockPackDst& cnt, cudaStream_t st);
 
-// Copies pieces of any alignment to dst + off in one launch; a piece without a source takes its
-// bytes from the argument itself (zero != 0: zeros).
+// Lays pieces of any alignment out at dst + off in one launch: device memory, bytes of the argument
+// itself, zeros, and one stream whose length only the device knows (ceil(*late_bits / 8), at most
+// late_most): its length as 8 bytes and its data.  Pieces with `after` lie that much further on.
 constexpr int kGatherPieces = 24;
 constexpr size_t kGatherInline = 4096;
+enum { kGatherCopy, kGatherInlineBytes, kGatherZero, kGatherLateLen, kGatherLate };
 struct GatherPiece {
     const uint8_t* src;
     uint64_t off, len;
     uint32_t inline_off;
-    uint32_t zero;
+    uint8_t kind, after;
 };
 struct GatherArgs {
     GatherPiece piece[kGatherPieces];
     int count;
+    const unsigned long long* late_bits;
+    uint64_t late_most;
     uint8_t inline_bytes[kGatherInline];
 };
 void launch_gather(const GatherArgs& args, uint8_t* dst, cudaStream_t st);
 
 constexpr int kEncTile = 4096;
-// Encoders write at most cap_bits bits (the output buffer's size) and flag an overflow beyond.
-void launch_gr_encode(const unsigned long long* vals, uint64_t n, int k, uint32_t* words, uint64_t cap_bits,
-                      LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits, uint32_t* err,
-                      cudaStream_t st);
-// A code whose codewords all have one length len (1..24): symbol i at stream bits [i len, (i + 1) len)
-// (code_bits indexed by the symbol; for counts the dense table); *total_bits = n * len.
-void launch_fixed_encode_u8(const uint8_t* sym, uint64_t n, const uint32_t* code_bits, int len, uint32_t* words,
-                            unsigned long long* total_bits, cudaStream_t st);
-void launch_fixed_encode_i32(const int32_t* sym, uint64_t n, const uint32_t* code_bits, int len, uint32_t* words,
-                             unsigned long long* total_bits, cudaStream_t st);
-void launch_huff_encode_u8(const uint8_t* sym, uint64_t n, const ByteCodes* codes, uint32_t* words,
-                           uint64_t cap_bits, LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits,
-                           uint32_t* err, cudaStream_t st);
-// counts: Huffman (eg_k < 0) with a dense table [kCountDense] and sorted sparse values, or
-// exp-Golomb with parameter eg_k >= 0.
-void launch_count_encode(const int32_t* counts, uint64_t n, int eg_k, const uint32_t* dense_bits,
-                         const uint8_t* dense_len, const uint32_t* sparse_val, const uint32_t* sparse_bits,
-                         const uint8_t* sparse_len, uint32_t sparse_n, uint32_t* words, uint64_t cap_bits,
-                         LookBackState lb, uint32_t* tile_counter, unsigned long long* total_bits, uint32_t* err,
-                         cudaStream_t st);
+// One entropy coder of launch_encode.  It writes at most cap_bits bits (the output buffer's size; words
+// zeroed) and flags an overflow beyond; *total_bits receives the bits written.
+enum { kEncodeGolombRice32, kEncodeGolombRice64, kEncodeHuffman, kEncodeFixedU8, kEncodeFixedI32, kEncodeCounts };
+struct EncodeJob {
+    int kind;
+    // Golomb-Rice parameter; fixed-length codes: the length (1..24); counts: exp-Golomb parameter, or
+    // -1 for Huffman
+    int k;
+    const void* in;  // n values: u32 / u64 (Golomb-Rice), u8 symbols, i32 counts; 16-byte aligned
+    uint64_t n;
+    const ByteCodes* codes;  // kEncodeHuffman
+    // fixed-length codes and counts: code bits by symbol (at least 256 entries; counts: a dense table
+    // [kCountDense], with lengths, and sorted sparse values)
+    const uint32_t* bits;
+    const uint8_t* len;
+    const uint32_t *sparse_val, *sparse_bits;
+    const uint8_t* sparse_len;
+    uint32_t sparse_n;
+    uint32_t blocks;  // set by launch_encode
+    uint32_t* words;
+    uint64_t cap_bits;
+    LookBackState lb;
+    uint32_t* tile_counter;
+    unsigned long long* total_bits;
+};
+struct EncodeArgs {
+    EncodeJob job[4];
+    int count;
+    uint32_t* err;
+};
+void launch_encode(EncodeArgs args, cudaStream_t st);
+
+// Sets ranges of words in one launch.
+struct FillRange {
+    void* p;  // 4-byte aligned
+    uint64_t words;
+    uint32_t value;
+};
+struct FillArgs {
+    FillRange range[24];
+    int count;
+};
+void launch_fill(const FillArgs& args, cudaStream_t st);
 
 // --- decompress -------------------------------------------------------------------------
 constexpr int kScanTile = 4096;  // elements per tile of the decompress-side chained scans
