@@ -553,28 +553,20 @@ struct CompressOut {
     uint32_t* d_order = nullptr;  // -normal: input index per container position
 };
 
-// One chained-scan channel set in the arena.
+// Chained-scan states of `channels` scans in the arena.
 struct LB {
-    size_t flag, agg, inc;
+    size_t off;
     uint64_t tiles;
+    int channels;
 };
-LB plan_lb(Plan& pl, uint64_t tiles, int channels, int agg_words_per_tile = 1, int inc_words_per_tile = 1) {
-    LB l;
-    l.tiles = tiles;
-    l.flag = pl.add(sizeof(uint32_t) * tiles * channels);
-    l.agg = pl.add(sizeof(unsigned long long) * tiles * channels * agg_words_per_tile);
-    l.inc = pl.add(sizeof(unsigned long long) * tiles * channels * inc_words_per_tile);
-    return l;
+LB plan_lb(Plan& pl, uint64_t tiles, int channels) {
+    return LB{pl.add(kScanStatusBytes * tiles * channels), tiles, channels};
 }
-LookBackState lb_state(xnyz_ctx* c, const LB& l) {
-    return LookBackState{at<uint32_t>(c, l.flag), at<unsigned long long>(c, l.agg), at<unsigned long long>(c, l.inc)};
+ScanStatus lb_state(xnyz_ctx* c, const LB& l, int channel = 0) {
+    return at<char>(c, l.off + kScanStatusBytes * l.tiles * channel);
 }
-void lb_clear(xnyz_ctx* c, Fills& f, const LB& l, int channels) {
-    f.add(at<uint32_t>(c, l.flag), sizeof(uint32_t) * l.tiles * channels, 0);
-}
-xnyz_status lb_clear(xnyz_ctx* c, const LB& l, int channels) {
-    CUDA_TRY(cudaMemsetAsync(at<uint32_t>(c, l.flag), 0, sizeof(uint32_t) * l.tiles * channels, c->stream));
-    return XNYZ_OK;
+void lb_clear(xnyz_ctx* c, Fills& f, const LB& l) {
+    f.add(lb_state(c, l), kScanStatusBytes * l.tiles * l.channels, 0);
 }
 
 // Arena layout of the compress path up to the encoder outputs (depends on n only).
@@ -604,7 +596,7 @@ CPlan make_cplan(uint64_t n, bool want_order, size_t reserved, bool ext) {
     c.o_counts = pl.add(4 * n);
     c.o_over_v = pl.add(4 * n);
     c.o_over_u = pl.add(4 * n);
-    c.lb_units = plan_lb(pl, c.tiles, 3);
+    c.lb_units = plan_lb(pl, c.tiles, 1);
     c.lb_enc = plan_lb(pl, c.tiles, 4);
     if (ext) {
         const uint64_t nb = cdiv(n, kParamBlock);
@@ -729,8 +721,8 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
         f.small(c, st0 + offsetof(PointStats, nonfinite), offsetof(Small, first_rep), 0);
         f.small(c, offsetof(Small, first_rep), offsetof(Small, bins), ~0u);
         f.small(c, offsetof(Small, bins), offsetof(Small, codes), 0);
-        lb_clear(c, f, cp.lb_units, 3);
-        lb_clear(c, f, cp.lb_enc, 4);
+        lb_clear(c, f, cp.lb_units);
+        lb_clear(c, f, cp.lb_enc);
         launch_fill(f.a, st);
     }
     if (cin) {
@@ -923,7 +915,6 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     Plan pe;
     pe.total = pl.total;
     const size_t o_w_gr = pe.add(4 * words_for(bits_gr));
-    const LookBackState lbs = lb_state(c, lb_enc);
     auto job = [&](int ch, int kind, const void* in, uint64_t count, int k, size_t o_words, uint64_t bits) {
         EncodeJob j{};
         j.kind = kind;
@@ -932,7 +923,7 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
         j.n = count;
         j.words = at<uint32_t>(c, o_words);
         j.cap_bits = 32 * words_for(bits);
-        j.lb = LookBackState{lbs.flag + ch * lb_enc.tiles, lbs.agg + ch * lb_enc.tiles, lbs.inc + ch * lb_enc.tiles};
+        j.status = lb_state(c, lb_enc, ch);
         j.tile_counter = SMALL_FIELD(c, tile_counters[20 + ch]);
         j.total_bits = SMALL_FIELD(c, totals[ch]);
         return j;
@@ -1524,7 +1515,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     const size_t o_counts = pl.add(4 * U + 8);
     const size_t o_xw = h.ext ? pl.add(x_nb) : 0, o_xk = h.ext ? pl.add(x_nb) : 0, o_xoff = h.ext ? pl.add(8 * x_nb) : 0,
                  o_xpay = h.ext ? pl.add(4 * (cdiv(x_bits, 32) + 2)) : 0, o_rv = h.ext ? pl.add(8 * U + 8) : 0;
-    const LB lb_scan = plan_lb(pl, cdiv(std::max<uint64_t>(NB, 1), kScanTile), 4);
+    const LB lb_scan = plan_lb(pl, cdiv(std::max<uint64_t>(NB, 1), kScanTile), 3);
     struct TabOff {
         size_t root, tree, sym;
     };
@@ -1550,13 +1541,19 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         o_dinc[i] = pl.add(16 * dtiles[i]);
     }
     const uint64_t rtiles = cdiv(std::max<uint64_t>(U, 1), kScanTile);
-    const size_t o_rflag = pl.add(4 * rtiles * 5), o_ragg = pl.add(16 * rtiles * 5), o_rinc = pl.add(16 * rtiles * 5);
+    const LB lb_rec = plan_lb(pl, rtiles, 3);
     if (pl.total > c->arena.cap) return fail(XNYZ_ERR_OOM, "__grow__:" + std::to_string(pl.total));
 
-    TRY(memset_small(c, offsetof(Small, err), sizeof(uint32_t), 0));
-    TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
-    TRY(memset_small(c, offsetof(Small, fallback), sizeof(uint32_t) * 8 * 2, 0));  // fallback + redone
-    TRY(memset_small(c, offsetof(Small, codewords), sizeof(unsigned long long) * 8, 0));
+    {
+        Fills f;
+        f.small(c, offsetof(Small, counters), offsetof(Small, first_rep), 0);  // error word, totals, codewords, ..
+        f.small(c, offsetof(Small, tile_counters), offsetof(Small, sort_hist), 0);
+        for (int i = 0; i < 4; ++i) f.add(at<uint8_t>(c, o_dinc[i]), 16 * dtiles[i], 0);
+        lb_clear(c, f, lb_scan);
+        lb_clear(c, f, lb_rec);
+        if (!h.direct) f.add(at<uint8_t>(c, o_isst), align_up(U, 4), 0);  // block-start marks
+        launch_fill(f.a, st);
+    }
     auto upload = [&](const HuffTables& t, const TabOff& o) -> xnyz_status {
         if (!t.root.empty())
             CUDA_TRY(cudaMemcpyAsync(at<uint32_t>(c, o.root), t.root.data(), 4 * t.root.size(), cudaMemcpyHostToDevice, st));
@@ -1582,8 +1579,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         const uint32_t* w0 = words_of(h.streams[0], b0);
         const uint32_t* w1 = words_of(h.streams[1], b1);
         Prof pr(c, "block_streams", 1, (w_blk + w_cnt) * NB / 8.0 + 8.0 * NB + 5.0 * std::min(NB, U));
-        TRY(lb_clear(c, lb_scan, 2));
-        CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_isst), 0, U + 8, st));
         launch_block_streams(w0, b0, w_blk, w1, b1, w_cnt, NB, U, at<unsigned long long>(c, o_blk),
                              at<uint8_t>(c, o_isst), at<uint32_t>(c, o_stb), lb_state(c, lb_scan),
                              SMALL_FIELD(c, tile_counters[20]), SMALL_FIELD(c, count_total), SMALL_FIELD(c, err), st);
@@ -1676,9 +1671,8 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     bool counts_summed = false;
     for (auto& j : jobs)
         if (rle && j.slot == 3 && j.width == 4 && !j.fill && (j.fixed_len || !j.tables)) counts_summed = true;
-    // the self-synchronising and the entry-table decoder (their state cleared first)
+    // the self-synchronising decoder (its state is zero on entry) and the entry-table decoder
     auto launch_sync = [&](const DecodeJob& j, cudaStream_t js, unsigned long long* sum_out) -> xnyz_status {
-        CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_dinc[j.slot]), 0, 16 * dtiles[j.slot], js));
         launch_decode_sync(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.byte_symbols, j.nsym, j.width, j.out,
                            at<uint8_t>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
                            SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, redone[j.slot]),
@@ -1706,7 +1700,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         Prof pr(c, j.kind == kCodeGolombRice ? "decode_golomb_rice" : (j.kind == kCodeHuffman ? "decode_huffman" : "decode_exp_golomb"),
                 1, j.total_bits / 8.0 + static_cast<double>(j.nsym) * j.width, js);
         const bool sum = counts_summed && j.slot == 3;
-        if (sum) CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, totals), 0, sizeof(unsigned long long) * 8, js));
         unsigned long long* sum_out = sum ? SMALL_FIELD(c, totals[0]) : nullptr;
         if (j.fixed_len) {
             if (j.nsym * static_cast<uint64_t>(j.fixed_len) > j.total_bits)
@@ -1755,6 +1748,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, redone[j.slot]), 0, 4, st));
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, tile_counters[30 + j.slot]), 0, 4, st));
             if (why == 4u) {
+                CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_dinc[j.slot]), 0, 16 * dtiles[j.slot], st));
                 TRY(launch_sync(j, st, nullptr));
             } else if (!(why & 1u) && !j.tables) {
                 j.tables = true;
@@ -1822,12 +1816,10 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     ri.nblocks = NB;
     ri.counts = at<int32_t>(c, o_counts);
     ri.rep_val = h.ext ? at<unsigned long long>(c, o_rv) : nullptr;
-    CUDA_TRY(cudaMemsetAsync(at<uint32_t>(c, o_rflag), 0, 4 * rtiles * 5, st));
     float* out = at<float>(c, o_out);
     Prof pr_rec(c, "recover_units", 1,
                 (h.direct ? 1.0 : 7.0) * U + 8.0 * P + (rle ? 4.0 * U : 0.0) + 12.0 * static_cast<double>(nout));
-    launch_recover_units(ri, U, nout, rp, c->d_small->hil_inv, at<uint32_t>(c, o_rflag),
-                         at<unsigned long long>(c, o_ragg), at<unsigned long long>(c, o_rinc),
+    launch_recover_units(ri, U, nout, rp, c->d_small->hil_inv, lb_state(c, lb_rec),
                          SMALL_FIELD(c, tile_counters[40]), out, SMALL_FIELD(c, err), st);
     CUDA_TRY(cudaGetLastError());
     pr_rec.end();
@@ -2445,7 +2437,7 @@ xnyz_status xnyz_expand_cells(xnyz_ctx* c, const int32_t* cells, const int32_t* 
         CUDA_TRY(cudaMemcpyAsync(at<int32_t>(c, o_counts), counts, 4 * n, cudaMemcpyHostToDevice, st));
     }
     CUDA_TRY(cudaMemcpyAsync(at<float>(c, o_off), offset, 12, cudaMemcpyHostToDevice, st));
-    TRY(lb_clear(c, lb, 1));
+    CUDA_TRY(cudaMemsetAsync(lb_state(c, lb), 0, kScanStatusBytes * lb.tiles, st));
     TRY(memset_small(c, offsetof(Small, err), sizeof(uint32_t), 0));
     TRY(memset_small(c, offsetof(Small, tile_counters), sizeof(uint32_t) * 64, 0));
     TRY(memset_small(c, offsetof(Small, totals), sizeof(unsigned long long) * 8, 0));

@@ -124,72 +124,35 @@ __device__ __forceinline__ T block_exclusive(T v, T identity, Op op, T* scratch,
 }
 
 // ------------------------------------------------------------- look-back ----------------
-// Single-pass chained scan state for one u64 channel: per tile a flag (0 empty,
-// 1 aggregate published, 2 inclusive prefix published) and the two values.  Values are
-// written before their flag with a fence in between; readers read the flag first.
-struct LookBack64 {
-    u32* flag;
-    u64* agg;
-    u64* inc;
-};
-
 __device__ __forceinline__ u32 ld_volatile(const u32* p) { return *(const volatile u32*)p; }
 __device__ __forceinline__ u64 ld_volatile(const u64* p) { return *(const volatile u64*)p; }
 __device__ __forceinline__ void st_volatile(u32* p, u32 v) { *(volatile u32*)p = v; }
 __device__ __forceinline__ void st_volatile(u64* p, u64 v) { *(volatile u64*)p = v; }
 
-// Generic single-thread look-back for an associative `op` over T (T is u64 or a small
-// struct of u64 fields, accessed through load/store helpers).  Returns the exclusive
-// prefix of `tile` and publishes its inclusive prefix.
-template <typename T, typename Op, typename Load, typename Store>
-__device__ T lookback(u32* flag, T* agg, T* inc, u32 tile, T mine, T identity, Op op, Load load, Store store,
-                      u32* err) {
-    if (tile == 0) {
-        store(&inc[0], mine);
-        __threadfence();
-        st_volatile(&flag[0], 2u);
-        return identity;
-    }
-    store(&agg[tile], mine);
-    __threadfence();
-    st_volatile(&flag[tile], 1u);
-    T acc = identity;
-    i64 t = (i64)tile - 1;
-    u32 spins = 0;
-    while (t >= 0) {
-        u32 f = ld_volatile(&flag[t]);
-        if (f == 0u) {
-            if (++spins > kSpinLimit) {
-                atomicOr(err, kErrTimeout);
-                break;
-            }
-            if (spins > 64) __nanosleep(100);
-            continue;
-        }
-        __threadfence();
-        if (f == 2u) {
-            acc = op(load(&inc[t]), acc);
-            break;
-        }
-        acc = op(load(&agg[t]), acc);
-        --t;
-    }
-    store(&inc[tile], op(acc, mine));
-    __threadfence();
-    st_volatile(&flag[tile], 2u);
-    return acc;
+// Single-pass chained scans.  A tile publishes its state as one 128-bit word, stored and loaded
+// whole, so that neither side needs a fence: lo and the low 62 bits of hi hold the value, the top
+// two bits of hi the flag (0 empty, 1 the tile's aggregate, 2 inclusive prefix).  What a value means
+// is up to the operator.
+using Status = unsigned __int128;
+struct Pair {
+    u64 lo, hi;
+};
+__device__ __forceinline__ void st_status(Status* p, Pair v, u32 flag) {
+    const Status x = ((Status)(v.hi | ((u64)flag << 62)) << 64) | v.lo;
+    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(x) : "memory");
+}
+__device__ __forceinline__ Pair ld_status(const Status* p, u32& flag) {
+    Status x;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(x) : "l"(p) : "memory");
+    const u64 hi = (u64)(x >> 64);
+    flag = (u32)(hi >> 62);
+    return Pair{(u64)x, hi & ((1ull << 62) - 1)};
 }
 
-struct LoadU64 {
-    __device__ __forceinline__ u64 operator()(const u64* p) const { return ld_volatile(p); }
+// Two sums side by side (lo wraps modulo 2^64, hi stays below 2^62).
+struct PairAdd {
+    __device__ __forceinline__ Pair operator()(Pair a, Pair b) const { return Pair{a.lo + b.lo, a.hi + b.hi}; }
 };
-struct StoreU64 {
-    __device__ __forceinline__ void operator()(u64* p, u64 v) const { st_volatile(p, v); }
-};
-
-__device__ __forceinline__ u64 lookback_add(LookBack64 lb, u32 tile, u64 mine, u32* err) {
-    return lookback(lb.flag, lb.agg, lb.inc, tile, mine, (u64)0, AddOp{}, LoadU64{}, StoreU64{}, err);
-}
 
 // Segmented sum element: `head` = a segment starts inside, `sum` = sum since the last
 // segment start (or of everything if no start).  combine(a, b) = a followed by b.
@@ -202,58 +165,47 @@ struct SegOp {
         return Seg{a.head | b.head, b.head ? b.sum : a.sum + b.sum};
     }
 };
-struct LoadSeg {
-    __device__ __forceinline__ Seg operator()(const Seg* p) const {
-        return Seg{ld_volatile(&p->head), ld_volatile(&p->sum)};
-    }
-};
-struct StoreSeg {
-    __device__ __forceinline__ void operator()(Seg* p, Seg v) const {
-        st_volatile(&p->head, v.head);
-        st_volatile(&p->sum, v.sum);
-    }
-};
 
-// Warp-cooperative look-back: called by all 32 lanes of one warp, returns the exclusive
-// prefix of `tile` to every lane and publishes its inclusive prefix.  Each step inspects 32
-// predecessors at once (lane i: tile - 1 - i - 32 * step), waits until all of them have
-// published something, then combines the aggregates up to the nearest inclusive prefix.
-// `op` need not commute: earlier tiles are combined first.
-__device__ __forceinline__ u64 shfl_down_t(u64 v, int d) { return __shfl_down_sync(kFullMask, v, d); }
-__device__ __forceinline__ Seg shfl_down_t(Seg v, int d) {
-    return Seg{__shfl_down_sync(kFullMask, v.head, d), __shfl_down_sync(kFullMask, v.sum, d)};
-}
-__device__ __forceinline__ u64 shfl_t(u64 v, int l) { return __shfl_sync(kFullMask, v, l); }
-__device__ __forceinline__ Seg shfl_t(Seg v, int l) {
-    return Seg{__shfl_sync(kFullMask, v.head, l), __shfl_sync(kFullMask, v.sum, l)};
-}
-
-template <typename T, typename Op, typename Load, typename Store>
-__device__ T warp_lookback(u32* flag, T* agg, T* inc, u32 tile, T mine, T identity, Op op, Load load, Store store,
-                           u32* err) {
+// Exclusive prefix of `tile` (to every lane), publishing its inclusive prefix; called by all 32 lanes
+// of one warp.  Each step reads the states of 128 predecessors, four per lane and the nearest first,
+// all in flight together, waits until those up to the nearest inclusive prefix have been published
+// and combines them, earlier tiles first (`op` need not commute; {0, 0} is its identity).  A wide
+// window matters: with all tiles of a wave publishing at about the same time, the prefixes spread
+// by the window per step.
+template <typename Op>
+__device__ Pair chain_lookback(Status* status, u32 tile, Pair mine, Op op, u32* err) {
     const int lane = (int)(threadIdx.x & 31u);
     if (tile == 0) {
-        if (lane == 0) {
-            store(&inc[0], mine);
-            __threadfence();
-            st_volatile(&flag[0], 2u);
-        }
-        __syncwarp();
-        return identity;
+        if (lane == 0) st_status(&status[0], mine, 2u);
+        return Pair{0, 0};
     }
-    if (lane == 0) {
-        store(&agg[tile], mine);
-        __threadfence();
-        st_volatile(&flag[tile], 1u);
-    }
-    T acc = identity;
+    if (lane == 0) st_status(&status[tile], mine, 1u);
+    Pair acc{0, 0};
     i64 top = (i64)tile - 1;
     u32 spins = 0;
     bool failed = false;
     while (true) {
-        const i64 p = top - lane;
-        const u32 f = p >= 0 ? ld_volatile(&flag[p]) : 2u;
-        if (__any_sync(kFullMask, f == 0u)) {
+        Pair v[4];
+        u32 f[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const i64 q = top - 4 * lane - j;
+            f[j] = 2u;
+            v[j] = Pair{0, 0};
+            if (q >= 0) v[j] = ld_status(&status[q], f[j]);
+        }
+        Pair r{0, 0};  // my tiles from my nearest inclusive one on
+        bool fin = false, empty = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (fin) continue;
+            r = op(v[j], r);
+            fin = f[j] == 2u;
+            empty |= f[j] == 0u;
+        }
+        const u32 m2 = __ballot_sync(kFullMask, fin);
+        const int last = m2 ? __ffs(m2) - 1 : 31;
+        if (__any_sync(kFullMask, empty && lane <= last)) {
             if (++spins > kSpinLimit) {
                 failed = true;
                 break;
@@ -261,33 +213,25 @@ __device__ T warp_lookback(u32* flag, T* agg, T* inc, u32 tile, T mine, T identi
             if (spins > 64) __nanosleep(100);
             continue;
         }
-        __threadfence();
-        T v = identity;
-        if (p >= 0) v = f == 2u ? load(&inc[p]) : load(&agg[p]);
-        const u32 m2 = __ballot_sync(kFullMask, f == 2u);
-        const int last = m2 ? __ffs(m2) - 1 : 31;
-        T r = lane <= last ? v : identity;
+        if (lane > last) r = Pair{0, 0};
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const T o = shfl_down_t(r, d);  // lane + d: an earlier tile
+            const Pair o{__shfl_down_sync(kFullMask, r.lo, d), __shfl_down_sync(kFullMask, r.hi, d)};  // earlier tiles
             if (lane + d < 32) r = op(o, r);
         }
-        acc = op(shfl_t(r, 0), acc);
+        acc = op(Pair{__shfl_sync(kFullMask, r.lo, 0), __shfl_sync(kFullMask, r.hi, 0)}, acc);
         if (m2) break;
-        top -= 32;
+        top -= 128;
     }
     if (lane == 0) {
         if (failed) atomicOr(err, kErrTimeout);
-        store(&inc[tile], op(acc, mine));
-        __threadfence();
-        st_volatile(&flag[tile], 2u);
+        st_status(&status[tile], op(acc, mine), 2u);
     }
-    __syncwarp();
     return acc;
 }
 
-__device__ __forceinline__ u64 warp_lookback_add(LookBack64 lb, u32 tile, u64 mine, u32* err) {
-    return warp_lookback(lb.flag, lb.agg, lb.inc, tile, mine, (u64)0, AddOp{}, LoadU64{}, StoreU64{}, err);
+__device__ __forceinline__ u64 chain_add(void* status, u32 tile, u64 mine, u32* err) {
+    return chain_lookback(static_cast<Status*>(status), tile, Pair{mine, 0}, PairAdd{}, err).lo;
 }
 
 // Dynamic tile index: tiles are claimed in launch order, so a tile's predecessors have

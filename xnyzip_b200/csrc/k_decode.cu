@@ -31,41 +31,22 @@ __device__ __forceinline__ u64 udiv(u64 x, const U64Div& d) {
 // bit-unpack the block-id deltas and block-count deltas, inclusive prefix sums of both
 // (u64, wrapping), the exclusive prefix of the counts (first unit of each block), and the
 // per-unit block-start marks of recover_from_lcp_meta (block_quantizer.hpp:167-176).
-// The count channel carries (sum of deltas, blocks, sum of counts) so that the prefix of the
-// counts and the prefix of their prefix come out of one chained scan:
-//   (A1, N1, B1) then (A2, N2, B2) = (A1 + A2, N1 + N2, B1 + B2 + N2 * A1).
+// Within a tile the count channel carries (sum of deltas, blocks, sum of counts):
+//   (A1, N1, B1) then (A2, N2, B2) = (A1 + A2, N1 + N2, B1 + B2 + N2 * A1);
+// across tiles one chained scan gives the tile's true first count, and so its true sum of counts,
+// which the next one chains.
 struct Tri {
     u64 a, n, b;
 };
 struct TriOp {
     __device__ __forceinline__ Tri operator()(Tri x, Tri y) const { return Tri{x.a + y.a, x.n + y.n, x.b + y.b + y.n * x.a}; }
 };
-struct LoadTri {
-    __device__ __forceinline__ Tri operator()(const Tri* p) const {
-        return Tri{ld_volatile(&p->a), ld_volatile(&p->n), ld_volatile(&p->b)};
-    }
-};
-struct StoreTri {
-    __device__ __forceinline__ void operator()(Tri* p, Tri v) const {
-        st_volatile(&p->a, v.a);
-        st_volatile(&p->n, v.n);
-        st_volatile(&p->b, v.b);
-    }
-};
-// found by argument-dependent lookup from warp_lookback
-__device__ __forceinline__ Tri shfl_down_t(Tri v, int d) {
-    return Tri{__shfl_down_sync(kFullMask, v.a, d), __shfl_down_sync(kFullMask, v.n, d),
-               __shfl_down_sync(kFullMask, v.b, d)};
-}
-__device__ __forceinline__ Tri shfl_t(Tri v, int l) {
-    return Tri{__shfl_sync(kFullMask, v.a, l), __shfl_sync(kFullMask, v.n, l), __shfl_sync(kFullMask, v.b, l)};
-}
 
 __global__ void __launch_bounds__(kThreads) block_streams_kernel(const u32* __restrict__ wb, u64 bb, int width_b,
                                                                  const u32* __restrict__ wc, u64 bc, int width_c,
                                                                  u64 nb, u64 units, u64* __restrict__ blk_out,
                                                                  u8* __restrict__ is_start, u32* __restrict__ start_block,
-                                                                 LookBackState lb, u32* tile_counter,
+                                                                 ScanStatus status, u32* tile_counter,
                                                                  unsigned long long* count_total, u32* err) {
     constexpr int kWarps = kThreads / 32;
     __shared__ u32 slot;
@@ -141,17 +122,17 @@ __global__ void __launch_bounds__(kThreads) block_streams_kernel(const u32* __re
     }
     __syncthreads();
     if (tid < 32) {
-        LookBack64 l{lb.flag, lb.agg, lb.inc};
-        const u64 r = warp_lookback_add(l, tile, wsb[kWarps], err);
+        const u64 r = chain_add(status, tile, wsb[kWarps], err);
         if (tid == 0) base_b = r;
     } else if (tid < 64) {
-        Tri* ag = reinterpret_cast<Tri*>(lb.agg + ntiles);
-        Tri* in = reinterpret_cast<Tri*>(lb.inc + ntiles);
-        const Tri r = warp_lookback(lb.flag + ntiles, ag, in, tile, wtc[kWarps], Tri{0, 0, 0}, TriOp{}, LoadTri{},
-                                    StoreTri{}, err);
+        Status* st = static_cast<Status*>(status) + ntiles;
+        const Tri mine = wtc[kWarps];
+        const u64 cnt0 = chain_add(st, tile, mine.a, err);
+        const u64 sum = mine.b + mine.n * cnt0;
+        const u64 first = chain_add(st + ntiles, tile, sum, err);
         if (tid == 32) {
-            base_c = r;
-            if (tile == ntiles - 1) *count_total = TriOp{}(r, wtc[kWarps]).b;
+            base_c = Tri{cnt0, 0, first};
+            if (tile == ntiles - 1) *count_total = first + sum;
         }
     }
     __syncthreads();
@@ -194,12 +175,22 @@ struct RecoverArgs {
     u64 nout;
     RecoverParams rp;
     const u8* hinv;
-    u32* flag;   // [5][ntiles]
-    u64* agg;    // [5][ntiles][2]
-    u64* inc;    // [5][ntiles][2]
+    Status* status;  // [3][ntiles]: zero symbols; counts; segments (block mode) or SFC sums
     u32* tile_counter;
     float* out;
     u32* err;
+};
+
+// Block mode's segmented sums in one chained scan.  lo: repos sum since the last repos head; hi: block
+// index (bits 0..31) and quad sum modulo 8 (32..34) since the last block start, whether a block starts
+// (35) and whether a repos head is inside (36).
+struct SegPair {
+    __device__ __forceinline__ Pair operator()(Pair a, Pair b) const {
+        const bool hq = (b.hi >> 35) & 1u, hr = (b.hi >> 36) & 1u;
+        const u64 quad = ((hq ? 0ull : a.hi >> 32) + (b.hi >> 32)) & 7u;
+        const u64 blk = ((hq ? 0ull : a.hi) + b.hi) & 0xffffffffull;
+        return Pair{(hr ? 0ull : a.lo) + b.lo, blk | (quad << 32) | ((a.hi | b.hi) & (3ull << 35))};
+    }
 };
 
 // Quad index step of a packed quad symbol (see recover_units_kernel): q - 1 modulo 8, 0 for
@@ -290,8 +281,7 @@ __global__ void __launch_bounds__(kThreads, 6) recover_units_kernel(RecoverArgs 
         if (tid == 0) warps_exclusive<kThreads / 32>(wz, 0ull, AddOp{});
         __syncthreads();
         if (w == 0) {
-            LookBack64 l{a.flag, a.agg, a.inc};
-            const u64 r = warp_lookback_add(l, tile, wz[kWarps], a.err);
+            const u64 r = chain_add(a.status, tile, wz[kWarps], a.err);
             if (tid == 0) base_zero = r;
         }
     } else if (tid < kWarps) {
@@ -360,33 +350,23 @@ __global__ void __launch_bounds__(kThreads, 6) recover_units_kernel(RecoverArgs 
     __syncthreads();
     // one warp per chained scan
     if (w == 0) {
+        Status* st = a.status + 2 * ntiles;
         if (DIRECT) {
-            LookBack64 l{a.flag + 4 * ntiles, a.agg + 8ull * ntiles, a.inc + 8ull * ntiles};
-            const u64 r = warp_lookback_add(l, tile, wd[kWarps], a.err);
+            const u64 r = chain_add(st, tile, wd[kWarps], a.err);
             if (tid == 0) base_sfc = r;
         } else {
-            Seg* ag = reinterpret_cast<Seg*>(a.agg + 8ull * ntiles);
-            Seg* in = reinterpret_cast<Seg*>(a.inc + 8ull * ntiles);
-            const Seg r = warp_lookback(a.flag + 4 * ntiles, ag, in, tile, wr[kWarps], Seg{0, 0}, SegOp{}, LoadSeg{},
-                                        StoreSeg{}, a.err);
-            if (tid == 0) base_rep = r;
+            const Seg q = wq[kWarps], b = wb[kWarps], r = wr[kWarps];
+            const Pair mine{r.sum, (b.sum & 0xffffffffull) | ((q.sum & 7u) << 32) | (q.head << 35) | (r.head << 36)};
+            const Pair p = chain_lookback(st, tile, mine, SegPair{}, a.err);
+            if (tid == 0) {
+                base_rep = Seg{0, p.lo};
+                base_quad = Seg{0, (p.hi >> 32) & 7u};
+                base_blk = Seg{0, p.hi & 0xffffffffull};
+            }
         }
     } else if (w == 1 && rle) {
-        LookBack64 l{a.flag + ntiles, a.agg + 2ull * ntiles, a.inc + 2ull * ntiles};
-        const u64 r = warp_lookback_add(l, tile, wc[kWarps], a.err);
+        const u64 r = chain_add(a.status + ntiles, tile, wc[kWarps], a.err);
         if (tid == 32) base_count = r;
-    } else if (w == 2 && !DIRECT) {
-        Seg* ag = reinterpret_cast<Seg*>(a.agg + 4ull * ntiles);
-        Seg* in = reinterpret_cast<Seg*>(a.inc + 4ull * ntiles);
-        const Seg r = warp_lookback(a.flag + 2 * ntiles, ag, in, tile, wq[kWarps], Seg{0, 0}, SegOp{}, LoadSeg{},
-                                    StoreSeg{}, a.err);
-        if (tid == 64) base_quad = r;
-    } else if (w == 3 && !DIRECT) {
-        Seg* ag = reinterpret_cast<Seg*>(a.agg + 6ull * ntiles);
-        Seg* in = reinterpret_cast<Seg*>(a.inc + 6ull * ntiles);
-        const Seg r = warp_lookback(a.flag + 3 * ntiles, ag, in, tile, wb[kWarps], Seg{0, 0}, SegOp{}, LoadSeg{},
-                                    StoreSeg{}, a.err);
-        if (tid == 96) base_blk = r;
     }
     if (!rle && tid == 0) base_count = 0;
     __syncthreads();
@@ -518,12 +498,12 @@ inline int grid_cap(u64 n) {
 
 void launch_block_streams(const uint32_t* words_blk, uint64_t base_blk, int width_blk, const uint32_t* words_cnt,
                           uint64_t base_cnt, int width_cnt, uint64_t nblocks, uint64_t units,
-                          unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, LookBackState lb,
+                          unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, ScanStatus status,
                           uint32_t* tile_counter, unsigned long long* count_total, uint32_t* err, cudaStream_t st) {
     const unsigned tiles = (unsigned)((nblocks + kTile - 1) / kTile);
     if (!tiles) return;
     block_streams_kernel<<<tiles, kThreads, 0, st>>>(words_blk, base_blk, width_blk, words_cnt, base_cnt, width_cnt,
-                                                     nblocks, units, blk_ids, is_start, start_block, lb, tile_counter,
+                                                     nblocks, units, blk_ids, is_start, start_block, status, tile_counter,
                                                      count_total, err);
 }
 
@@ -537,8 +517,7 @@ void launch_count_total(const int32_t* counts, uint64_t n, unsigned long long* t
     if (n) count_total_kernel<<<grid_cap(n), kThreads, 0, st>>>(counts, n, total);
 }
 void launch_recover_units(const RecoverInputs& in, uint64_t units, uint64_t nout, RecoverParams rp,
-                          const uint8_t* hilbert_inv_tab, uint32_t* flag, unsigned long long* agg,
-                          unsigned long long* inc, uint32_t* tile_counter, float* out, uint32_t* err,
+                          const uint8_t* hilbert_inv_tab, ScanStatus status, uint32_t* tile_counter, float* out, uint32_t* err,
                           cudaStream_t st) {
     RecoverArgs a;
     a.rep_sym = in.rep_sym;
@@ -556,9 +535,7 @@ void launch_recover_units(const RecoverInputs& in, uint64_t units, uint64_t nout
     a.nout = nout;
     a.rp = rp;
     a.hinv = hilbert_inv_tab;
-    a.flag = flag;
-    a.agg = agg;
-    a.inc = inc;
+    a.status = static_cast<Status*>(status);
     a.tile_counter = tile_counter;
     a.out = out;
     a.err = err;

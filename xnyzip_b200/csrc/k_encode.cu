@@ -61,7 +61,7 @@ __device__ __forceinline__ void hist_add_masked(u32* masks, u32* hist, u32* firs
 template <bool DIRECT>
 __global__ void __launch_bounds__(kThreads) units_kernel(const u64* __restrict__ keys, u64 n, int rle,
                                                          BlockKeyParams bkp, DirectKeyParams dkp, UnitOutputs out,
-                                                         LookBackState lb, u32* tile_counter, u32* err) {
+                                                         ScanStatus status, u32* tile_counter, u32* err) {
     __shared__ u64 sk[kTile + 1];
     __shared__ u64 scratch[16];
     __shared__ u32 slot;
@@ -152,14 +152,16 @@ __global__ void __launch_bounds__(kThreads) units_kernel(const u64* __restrict__
     const u64 mine = (u64)h | ((u64)p << 21) | ((u64)b << 42);
     u64 tot;
     const u64 ex = block_exclusive<kThreads>(mine, 0ull, AddOp{}, scratch, tot);
-    if (tid < 96) {  // warps 0, 1, 2: one chained scan each
-        const int ch = tid >> 5;
-        const u64 part = (tot >> (21 * ch)) & ((1ull << 21) - 1);
-        LookBack64 l{lb.flag + ch * ntiles, lb.agg + ch * ntiles, lb.inc + ch * ntiles};
-        const u64 before = warp_lookback_add(l, tile, part, err);
-        if ((tid & 31) == 0) {
-            sbase[ch] = before;
-            if (tile == ntiles - 1) out.counters[ch] = before + part;
+    if (tid < 32) {  // the three counts (below 2^31) in one chained scan
+        constexpr u64 kF = (1ull << 21) - 1;
+        const Pair part{(tot & kF) | (((tot >> 21) & kF) << 32), tot >> 42};
+        const Pair before = chain_lookback(static_cast<Status*>(status), tile, part, PairAdd{}, err);
+        if (tid == 0) {
+            const u64 be[3] = {before.lo & 0xffffffffull, before.lo >> 32, before.hi};
+            for (int ch = 0; ch < 3; ++ch) {
+                sbase[ch] = be[ch];
+                if (tile == ntiles - 1) out.counters[ch] = be[ch] + ((tot >> (21 * ch)) & kF);
+            }
         }
     }
     __syncthreads();
@@ -465,8 +467,7 @@ union EncodeShared {
 
 __device__ __forceinline__ u64 tile_bit_base(const EncodeJob& j, u32 tile, u64 tot, u64* sbase, u32* err) {
     if (threadIdx.x < 32) {
-        LookBack64 l{j.lb.flag, j.lb.agg, j.lb.inc};
-        const u64 before = warp_lookback_add(l, tile, tot, err);
+        const u64 before = chain_add(j.status, tile, tot, err);
         if (threadIdx.x == 0) {
             *sbase = before;
             if (tile == j.blocks - 1) *j.total_bits = before + tot;
@@ -821,16 +822,16 @@ inline int persistent_grid(u64 n) {
 }  // namespace
 
 void launch_units_block(const unsigned long long* keys, uint64_t n, int rle, BlockKeyParams kp, UnitOutputs out,
-                        LookBackState lb, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
+                        ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
     const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
     if (!tiles) return;
-    units_kernel<false><<<tiles, kThreads, 0, st>>>(keys, n, rle, kp, DirectKeyParams{}, out, lb, tile_counter, err);
+    units_kernel<false><<<tiles, kThreads, 0, st>>>(keys, n, rle, kp, DirectKeyParams{}, out, status, tile_counter, err);
 }
 void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, DirectKeyParams kp, UnitOutputs out,
-                         LookBackState lb, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
+                         ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
     const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
     if (!tiles) return;
-    units_kernel<true><<<tiles, kThreads, 0, st>>>(keys, n, rle, BlockKeyParams{}, kp, out, lb, tile_counter, err);
+    units_kernel<true><<<tiles, kThreads, 0, st>>>(keys, n, rle, BlockKeyParams{}, kp, out, status, tile_counter, err);
 }
 void launch_count_stats(const uint32_t* unit_pos, uint64_t units, const unsigned long long* units_dev, uint64_t n,
                         int32_t* counts, CountStats cs, cudaStream_t st) {

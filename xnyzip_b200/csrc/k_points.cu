@@ -325,7 +325,7 @@ __global__ void gather_i32_kernel(const i32* __restrict__ src, const u32* __rest
 // counts[i] times, recovered and unshifted; output positions by a chained scan of the counts.
 __global__ void __launch_bounds__(kThreads) expand_cells_kernel(const i32* __restrict__ cells,
                                                                 const i32* __restrict__ counts, u64 n, QuantParams q,
-                                                                const float* __restrict__ off3, LookBackState lb,
+                                                                const float* __restrict__ off3, ScanStatus status,
                                                                 u32* tile_counter, float* __restrict__ out, u64 cap,
                                                                 unsigned long long* total, u32* err) {
     constexpr int kItems = 16, kTile = kThreads * kItems;
@@ -340,8 +340,7 @@ __global__ void __launch_bounds__(kThreads) expand_cells_kernel(const i32* __res
     u64 tot;
     const u64 ex = block_exclusive<kThreads>(s, 0ull, AddOp{}, scratch, tot);
     if (threadIdx.x < 32) {
-        LookBack64 l{lb.flag, lb.agg, lb.inc};
-        const u64 r = warp_lookback_add(l, tile, tot, err);
+        const u64 r = chain_add(status, tile, tot, err);
         if (threadIdx.x == 0) {
             sbase = r;
             if (tile == gridDim.x - 1) *total = r + tot;
@@ -475,10 +474,10 @@ void launch_gather_i32(const int32_t* src, const uint32_t* idx, uint64_t n, int3
     if (n) gather_i32_kernel<<<grid_for(n), kThreads, 0, st>>>(src, idx, n, dst);
 }
 void launch_expand_cells(const int32_t* cells, const int32_t* counts, uint64_t n, QuantParams q, const float* off3,
-                         LookBackState lb, uint32_t* tile_counter, float* out, uint64_t cap,
+                         ScanStatus status, uint32_t* tile_counter, float* out, uint64_t cap,
                          unsigned long long* total, uint32_t* err, cudaStream_t st) {
     const unsigned tiles = (unsigned)((n + kThreads * 16 - 1) / (kThreads * 16));
-    if (tiles) expand_cells_kernel<<<tiles, kThreads, 0, st>>>(cells, counts, n, q, off3, lb, tile_counter, out, cap, total, err);
+    if (tiles) expand_cells_kernel<<<tiles, kThreads, 0, st>>>(cells, counts, n, q, off3, status, tile_counter, out, cap, total, err);
 }
 void launch_quantize_cells(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, int32_t* cells,
                            cudaStream_t st) {

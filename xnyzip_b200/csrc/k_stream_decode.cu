@@ -908,7 +908,7 @@ struct SyncArgs {
     u64 nsym;
     int out_width;
     void* out;
-    unsigned __int128* status;  // per tile (tile_status)
+    Status* status;  // per tile (tile_state)
     u32* tile_counter;
     u32* err;
     u32* need_fallback;
@@ -921,20 +921,11 @@ __host__ __device__ inline size_t sync_smem(int S, int rb, int mb) {
     return 8 * kSyncThreads + (rb ? (8ull << mb) + (4ull << rb) : 0) + 4 * (size_t)(kSyncThreads * S / 32 + kSyncHalo);
 }
 
-// A block's published state, read and written as one 128-bit word so that no fence is needed:
-// bits 0..61 codewords (of the block; through the block once final), 62..63 flag (1 assumed, 2
-// final), 64..95 assumed entry and 96..127 exit, relative to the block's and the next block's
-// first bit.
-__device__ __forceinline__ unsigned __int128 tile_status(u32 flag, u64 codewords, u64 entry, u64 exit) {
-    return ((unsigned __int128)((exit << 32) | entry) << 64) | (codewords | ((u64)flag << 62));
-}
-__device__ __forceinline__ void st_status(unsigned __int128* p, unsigned __int128 v) {
-    asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
-}
-__device__ __forceinline__ unsigned __int128 ld_status(const unsigned __int128* p) {
-    unsigned __int128 v;
-    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
-    return v;
+// A block's published state (device_common.cuh: Status): lo = the exit relative to the next block's
+// first bit << 32 | the assumed entry relative to the block's, hi = codewords (of the block; through
+// the block once final) and the flag (1 assumed, 2 final).
+__device__ __forceinline__ Pair tile_state(u64 codewords, u64 entry, u64 exit) {
+    return Pair{(exit << 32) | entry, codewords};
 }
 
 // A thread's run of 32-bit words out[first], out[first + 1], ..: four at a time as one 16-byte
@@ -1201,7 +1192,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
         u32 why = kNotConverged;
         u64 E = assumed - tile_at, C = 0;
         if (tile > 0) {
-            if (lane == 0 && !failed) st_status(&a.status[tile], tile_status(1u, total, assumed - tile_at, exit_of()));
+            if (lane == 0 && !failed) st_status(&a.status[tile], tile_state(total, assumed - tile_at, exit_of()), 1u);
             // 128 blocks per step, four per lane (the nearest first)
             long long top = (long long)tile - 1;
             u64 pend = 0;
@@ -1212,10 +1203,11 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const long long q = top - 4 * (long long)lane - j;
-                    const unsigned __int128 v = q >= 0 ? ld_status(&a.status[q]) : (unsigned __int128)2u << 62;
-                    n[j] = (u64)v & ((1ull << 62) - 1);
-                    f[j] = (u32)((u64)v >> 62);
-                    ex[j] = (u64)(v >> 64);
+                    f[j] = 2u;
+                    Pair v{0, 0};
+                    if (q >= 0) v = ld_status(&a.status[q], f[j]);
+                    n[j] = v.hi;
+                    ex[j] = v.lo;
                 }
                 // my four up to my first final one, chained to the next lane's first exit
                 const u64 xnext = __shfl_down_sync(kFullMask, ex[0] >> 32, 1);
@@ -1268,7 +1260,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
             }
             const bool same = E == assumed - tile_at;
             if (!failed && !same && atomicAdd(a.redone, 1u) >= kMaxRedo) atomicOr(a.need_fallback, kNotConverged);
-            if (failed || same) st_status(&a.status[tile], tile_status(2u, C + total, 0ull, exit_of() & 0xffffffffull));
+            if (failed || same) st_status(&a.status[tile], tile_state(C + total, 0ull, exit_of() & 0xffffffffull), 2u);
             s_entry = failed ? assumed : tile_at + E;
             s_first = C;
         }
@@ -1283,7 +1275,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
                 atomicOr(a.need_fallback, kNotConverged);
                 __threadfence();
             }
-            st_status(&a.status[tile], tile_status(2u, s_first + total, 0ull, exit_of() & 0xffffffffull));
+            st_status(&a.status[tile], tile_state(s_first + total, 0ull, exit_of() & 0xffffffffull), 2u);
         }
     }
     if (tile == gridDim.x - 1 && t == 0) *a.total_codewords = s_first + total;
@@ -1550,7 +1542,7 @@ void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uin
     a.nsym = nsym;
     a.out_width = out_width;
     a.out = out;
-    a.status = static_cast<unsigned __int128*>(status);
+    a.status = static_cast<Status*>(status);
     a.tile_counter = tile_counter;
     a.err = err;
     a.need_fallback = need_fallback;

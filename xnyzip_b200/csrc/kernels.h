@@ -70,11 +70,9 @@ struct UnitOutputs {
     unsigned long long* rep_val;    // optional: repos / sfc delta value per unit (extended container)
 };
 
-struct LookBackState {
-    uint32_t* flag;
-    unsigned long long* agg;
-    unsigned long long* inc;
-};
+// State of a chained scan: 16 bytes per tile, zeroed (device_common.cuh: chain_lookback).
+using ScanStatus = void*;
+constexpr size_t kScanStatusBytes = 16;
 
 // Count-stream statistics (-rle).
 constexpr int kCountDense = 4096;
@@ -113,13 +111,13 @@ void launch_keys_direct(const float* xyz, uint64_t n, QuantParams q, const Point
                         uint32_t* hist, cudaStream_t st);
 // Cell tables: block keys from int32 cells; per-axis min / max of cells (stats->min_cell /
 // max_cell, initialised by the caller); dst[i] = src[idx[i]]; expansion + recover + unshift
-// (lb: flag, agg, inc of ceil(n / 4096) tiles; *total receives the point count).
+// (status: ceil(n / 4096) tiles; *total receives the point count).
 void launch_keys_cells(const int32_t* cells, uint64_t n, BlockKeyParams kp, const uint8_t* hilbert_tab,
                        unsigned long long* keys, uint32_t* payload, int passes, uint32_t* hist, cudaStream_t st);
 void launch_cells_stats(const int32_t* cells, uint64_t n, PointStats* stats, cudaStream_t st);
 void launch_gather_i32(const int32_t* src, const uint32_t* idx, uint64_t n, int32_t* dst, cudaStream_t st);
 void launch_expand_cells(const int32_t* cells, const int32_t* counts, uint64_t n, QuantParams q, const float* off3,
-                         LookBackState lb, uint32_t* tile_counter, float* out, uint64_t cap,
+                         ScanStatus status, uint32_t* tile_counter, float* out, uint64_t cap,
                          unsigned long long* total, uint32_t* err, cudaStream_t st);
 void launch_quantize_cells(const float* xyz, uint64_t n, QuantParams q, const PointStats* stats, int32_t* cells,
                            cudaStream_t st);
@@ -146,9 +144,9 @@ void launch_sort_small(const unsigned long long* kin, unsigned long long* kout, 
 // --- compress segments + encoders -------------------------------------------------------
 constexpr int kUnitTile = 4096;
 void launch_units_block(const unsigned long long* keys, uint64_t n, int rle, BlockKeyParams kp, UnitOutputs out,
-                        LookBackState lb, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
+                        ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
 void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, DirectKeyParams kp, UnitOutputs out,
-                         LookBackState lb, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
+                         ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
 // unit_pos null: counts[] is the input (cell tables), else counts[] receives the run lengths.
 void launch_count_stats(const uint32_t* unit_pos, uint64_t units, const unsigned long long* units_dev, uint64_t n,
                         int32_t* counts, CountStats cs, cudaStream_t st);
@@ -211,7 +209,7 @@ struct EncodeJob {
     uint32_t blocks;  // set by launch_encode
     uint32_t* words;
     uint64_t cap_bits;
-    LookBackState lb;
+    ScanStatus status;
     uint32_t* tile_counter;
     unsigned long long* total_bits;
 };
@@ -345,16 +343,15 @@ struct RecoverInputs {
 };
 // Block streams of block mode in one pass: bit-unpack (widths <= 64), inclusive prefix sums of
 // the block-id and block-count deltas, block-start marks (is_start zeroed by the caller).
-// lb: flag [2 * tiles], agg and inc [4 * tiles] u64; tiles = ceil(nblocks / 4096).
+// status: [3][tiles], tiles = ceil(nblocks / 4096).
 void launch_block_streams(const uint32_t* words_blk, uint64_t base_blk, int width_blk, const uint32_t* words_cnt,
                           uint64_t base_cnt, int width_cnt, uint64_t nblocks, uint64_t units,
-                          unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, LookBackState lb,
+                          unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, ScanStatus status,
                           uint32_t* tile_counter, unsigned long long* count_total, uint32_t* err, cudaStream_t st);
-// flag: [5 * tiles]; agg, inc: [10 * tiles]; tiles = ceil(units / 4096)
+// status: [3][tiles], tiles = ceil(units / 4096)
 void launch_recover_units(const RecoverInputs& in, uint64_t units, uint64_t nout, RecoverParams rp,
-                          const uint8_t* hilbert_inv_tab, uint32_t* flag, unsigned long long* agg,
-                          unsigned long long* inc, uint32_t* tile_counter, float* out, uint32_t* err,
-                          cudaStream_t st);
+                          const uint8_t* hilbert_inv_tab, ScanStatus status, uint32_t* tile_counter, float* out,
+                          uint32_t* err, cudaStream_t st);
 
 
 // --- block-parameter coding (extended container) and its predictor ------------------------
