@@ -59,9 +59,6 @@ xnyz_status fail(xnyz_status s, const std::string& msg) {
     } while (0)
 
 constexpr size_t kAlign = 256;
-// First 8 bytes of an extended container ("XNYZBX01"): the reference container follows,
-// except that the repos / SFC-delta stream is block-coded (k_blocks.cu).
-constexpr uint64_t kExtMagic = 0x313058425a594e58ull;
 inline size_t align_up(size_t v, size_t a = kAlign) { return (v + a - 1) / a * a; }
 inline uint64_t cdiv(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 inline int bitlen(uint64_t v) { return v ? 64 - __builtin_clzll(v) : 0; }
@@ -130,6 +127,9 @@ struct xnyz_ctx {
     uint32_t sort_epoch = 0;
     uint8_t* h_stage = nullptr;  // pinned staging for containers
     size_t h_stage_cap = 0;
+    uint8_t* h_tab = nullptr;  // pinned staging for decode tables
+    size_t h_tab_cap = 0;
+    uint8_t* h_head = nullptr;  // pinned, written by the header kernel (kHeaderBytes)
     uint8_t* d_container = nullptr;  // device container returned by xnyz_compress_device
     size_t d_container_cap = 0;
     uint8_t* d_blob = nullptr;  // host bytes of a container whose header is large
@@ -182,16 +182,17 @@ xnyz_status ensure_arena(xnyz_ctx* c, size_t bytes) {
     return XNYZ_OK;
 }
 
-xnyz_status ensure_host_stage(xnyz_ctx* c, size_t bytes) {
-    if (c->h_stage_cap >= bytes) return XNYZ_OK;
-    if (c->h_stage) cudaFreeHost(c->h_stage);
-    c->h_stage = nullptr;
-    c->h_stage_cap = 0;
-    const size_t want = align_up(bytes + bytes / 8, 1 << 20);
-    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_stage), want, cudaHostAllocDefault));
-    c->h_stage_cap = want;
+xnyz_status ensure_pinned(uint8_t*& buf, size_t& cap, size_t bytes, size_t unit = 1 << 16) {
+    if (cap >= bytes) return XNYZ_OK;
+    if (buf) cudaFreeHost(buf);
+    buf = nullptr;
+    cap = 0;
+    const size_t want = align_up(bytes + bytes / 8, unit);
+    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&buf), want, cudaHostAllocDefault));
+    cap = want;
     return XNYZ_OK;
 }
+xnyz_status ensure_host_stage(xnyz_ctx* c, size_t bytes) { return ensure_pinned(c->h_stage, c->h_stage_cap, bytes, 1 << 20); }
 
 // The buffer of the container that xnyz_compress_device returns (+ 64 bytes of zero padding).
 xnyz_status ensure_container(xnyz_ctx* c, size_t bytes) {
@@ -1151,7 +1152,7 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     HostPhase hp6(c, "c6_container");
     // ---- 9. container (Appendix: block_compressor.hpp:56-215, block_compressor_rle.hpp:125-314) ----
     Container& K = R.cont;
-    if (ext) K.pod<uint64_t>(kExtMagic);
+    if (ext) K.pod<uint64_t>(kExtendedMagic);
     K.pod<uint64_t>(U);
     if (adaptive) {  // params: the adaptive quantizer's three steps (block_compressor.hpp:63-66)
         K.pod<uint64_t>(3);
@@ -1293,7 +1294,7 @@ xnyz_status parse_header(Read rd, uint64_t len, bool rle, Header& h) {
     uint64_t np = 0;
     uint8_t hb = 0, db = 0;
     if (!get(&h.units, 8)) return fail(XNYZ_ERR_BAD_STREAM, "truncated container header");
-    if (h.units == kExtMagic) {
+    if (h.units == kExtendedMagic) {
         h.ext = true;
         if (!get(&h.units, 8)) return fail(XNYZ_ERR_BAD_STREAM, "truncated container header");
     }
@@ -1523,10 +1524,13 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     if (!h.ext) TRY(build_huff_tables(pm_sym, ht_sym));
     if (!h.direct) TRY(build_huff_tables(pm_quad, ht_quad));
     if (rle && !pm_cnt.exp_golomb) TRY(build_huff_tables(pm_cnt, ht_cnt));
+    // all decode tables side by side, uploaded in one copy
+    const size_t tab0 = align_up(pl.total);
     auto plan_tab = [&](const HuffTables& t) {
         return TabOff{pl.add(4 * t.root.size()), pl.add(4 * t.tree.size()), pl.add(8 * t.symvals.size() + 8)};
     };
     const TabOff to_sym = plan_tab(ht_sym), to_quad = plan_tab(ht_quad), to_cnt = plan_tab(ht_cnt);
+    const size_t tab_bytes = pl.total - tab0;
     // decode look-back state per stream (up to 4 streams), for either decoder
     const uint64_t dbits[4] = {s_gr.data_len * 8, s_sym.data_len * 8, h.direct ? 0 : h.streams[5].data_len * 8,
                                rle ? s_cnt->data_len * 8 : 0};
@@ -1554,19 +1558,16 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         if (!h.direct) f.add(at<uint8_t>(c, o_isst), align_up(U, 4), 0);  // block-start marks
         launch_fill(f.a, st);
     }
-    auto upload = [&](const HuffTables& t, const TabOff& o) -> xnyz_status {
-        if (!t.root.empty())
-            CUDA_TRY(cudaMemcpyAsync(at<uint32_t>(c, o.root), t.root.data(), 4 * t.root.size(), cudaMemcpyHostToDevice, st));
-        if (!t.tree.empty())
-            CUDA_TRY(cudaMemcpyAsync(at<uint32_t>(c, o.tree), t.tree.data(), 4 * t.tree.size(), cudaMemcpyHostToDevice, st));
-        if (!t.symvals.empty())
-            CUDA_TRY(cudaMemcpyAsync(at<unsigned long long>(c, o.sym), t.symvals.data(), 8 * t.symvals.size(),
-                                     cudaMemcpyHostToDevice, st));
-        return XNYZ_OK;
+    TRY(ensure_pinned(c->h_tab, c->h_tab_cap, tab_bytes));
+    auto place = [&](const HuffTables& t, const TabOff& o) {
+        std::memcpy(c->h_tab + (o.root - tab0), t.root.data(), 4 * t.root.size());
+        std::memcpy(c->h_tab + (o.tree - tab0), t.tree.data(), 4 * t.tree.size());
+        std::memcpy(c->h_tab + (o.sym - tab0), t.symvals.data(), 8 * t.symvals.size());
     };
-    TRY(upload(ht_sym, to_sym));
-    TRY(upload(ht_quad, to_quad));
-    TRY(upload(ht_cnt, to_cnt));
+    place(ht_sym, to_sym);
+    place(ht_quad, to_quad);
+    place(ht_cnt, to_cnt);
+    if (tab_bytes) CUDA_TRY(cudaMemcpyAsync(at<uint8_t>(c, tab0), c->h_tab, tab_bytes, cudaMemcpyHostToDevice, st));
 
     hd1.end();
     HostPhase hd2(c, "d2_launch");
@@ -1898,6 +1899,7 @@ xnyz_status xnyz_create(xnyz_ctx** out, int device, void* stream) {
     CUDA_TRY(cudaMemcpy(c->d_small->hil_inv, hilbert_machines().inv.data(), 256, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_small), sizeof(Small), cudaHostAllocDefault));
     std::memset(c->h_small, 0, sizeof(Small));
+    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_head), kHeaderBytes, cudaHostAllocDefault));
     CUDA_TRY(cudaEventCreate(&c->ev0));
     CUDA_TRY(cudaEventCreate(&c->ev1));
     CUDA_TRY(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
@@ -1918,6 +1920,8 @@ xnyz_status xnyz_destroy(xnyz_ctx* c) {
     if (c->d_small) cudaFree(c->d_small);
     if (c->h_small) cudaFreeHost(c->h_small);
     if (c->h_stage) cudaFreeHost(c->h_stage);
+    if (c->h_tab) cudaFreeHost(c->h_tab);
+    if (c->h_head) cudaFreeHost(c->h_head);
     if (c->d_container) cudaFree(c->d_container);
     if (c->d_blob) cudaFree(c->d_blob);
     if (c->d_model) cudaFree(c->d_model);
@@ -2246,11 +2250,12 @@ xnyz_status xnyz_decompress_device(xnyz_ctx* c, const uint8_t* dev_container, ui
         return fail(XNYZ_ERR_INVALID_ARG, "quantizer must be 0 (cube), 1 (truncated octahedron) or 2 (adaptive)");
     CUDA_TRY(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
-    // The kernels read up to 16 bytes past a stream's end; containers from
-    // xnyz_compress_device carry 64 bytes of padding.  Others are copied into the arena.
+    // The kernels read the streams as aligned 4-byte words, at most 12 bytes past a stream's end,
+    // which is where the next stream's lengths or the container's offset lie: a container on a
+    // 4-byte boundary is decoded in place, any other is copied to one.
     const uint8_t* d_cont = dev_container;
     size_t reserved = 0;
-    if (dev_container != c->d_container) {
+    if (reinterpret_cast<uintptr_t>(dev_container) & 3u) {
         reserved = align_up(len + 64);
         TRY(ensure_arena(c, reserved));
         CUDA_TRY(cudaMemcpyAsync(c->arena.base, dev_container, len, cudaMemcpyDeviceToDevice, st));
@@ -2259,16 +2264,39 @@ xnyz_status xnyz_decompress_device(xnyz_ctx* c, const uint8_t* dev_container, ui
     }
     Header h;
     HostPhase hph(c, "d0_header_device");
-    // The header's fields are read through a 64 KB window of the container copied to the host
-    // at once: a small container's whole header costs one copy, a large one a copy per stream
-    // (each stream's lengths and meta follow the previous stream's data), instead of a copy
-    // and a synchronisation per field.
+    // A small container comes over whole.  In a large one each stream's lengths and meta follow the
+    // previous stream's data: a kernel walks them and writes them to pinned memory (18 us; a copy
+    // and a wait per stream took 130 us for 1M points).  Whatever it did not collect (a meta beyond
+    // its room, damaged lengths) is read through 64 KB windows.
+    constexpr uint64_t kWindow = 64u << 10;
+    const HeaderPieces* hp = reinterpret_cast<const HeaderPieces*>(c->h_head);
+    const bool whole = len <= kHeaderBytes / 2;
+    if (whole) {
+        CUDA_TRY(cudaMemcpyAsync(c->h_head, d_cont, len, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+    } else {
+        launch_header(d_cont, len, rle != 0, c->h_head, st);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(st));
+    }
     std::vector<uint8_t> win;
     uint64_t win_off = 0;
     xnyz_status s = parse_header(
         [&](uint64_t off, uint64_t bytes, void* dst) {
+            if (whole) {
+                std::memcpy(dst, c->h_head + off, bytes);
+                return true;
+            } else {
+                for (uint32_t i = 0; i < hp->count; ++i) {
+                    const auto& p = hp->piece[i];
+                    if (off >= p.off && off + bytes <= p.off + p.len) {
+                        std::memcpy(dst, c->h_head + sizeof(HeaderPieces) + p.at + (off - p.off), bytes);
+                        return true;
+                    }
+                }
+            }
             if (win.empty() || off < win_off || off + bytes > win_off + win.size()) {
-                const uint64_t want = std::min<uint64_t>(len - off, std::max<uint64_t>(bytes, 64u << 10));
+                const uint64_t want = std::min<uint64_t>(len - off, std::max<uint64_t>(bytes, kWindow));
                 win.resize(want);
                 win_off = off;
                 if (cudaMemcpyAsync(win.data(), d_cont + off, want, cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -141,6 +141,63 @@ __global__ void __launch_bounds__(kThreads) block_streams_kernel(const u32* __re
     pass(blk, cnt, start);
 }
 
+// ---------------------------------------------------------------- header --------------
+// One block: thread 0 walks the streams' lengths (a chain of one read each), then all threads copy
+// the pieces.
+__global__ void __launch_bounds__(kThreads) header_kernel(const u8* __restrict__ c, u64 len, u64 magic, int rle,
+                                                          u8* __restrict__ out) {
+    __shared__ HeaderPieces hp;
+    constexpr u32 kRoom = (u32)(kHeaderBytes - sizeof(HeaderPieces));
+    if (threadIdx.x == 0) {
+        auto u64_at = [&](u64 p) {
+            u64 v = 0;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) v |= (u64)__ldg(c + p + b) << (8 * b);
+            return v;
+        };
+        u32 used = 0;
+        hp.count = 0;
+        hp.unused = 0;
+        auto take = [&](u64 off, u64 n) {
+            const u32 m = (u32)min(n, (u64)(kRoom - used));
+            hp.piece[hp.count++] = {off, m, used};
+            used += m;
+        };
+        u64 p = 0;
+        bool ok = len >= 64;
+        if (ok) {
+            if (u64_at(0) == magic) p = 8;
+            const u64 np = u64_at(p + 8);  // quantizer parameters (4 bytes each)
+            p += 16;
+            ok = np <= (len - p) / 4 && len - p - 4 * np >= 14;
+            if (ok) {
+                p += 4 * np + 13;
+                const int ns = (__ldg(c + p) ? 2 : 6) + rle;  // the direct-mode flag ends the fixed fields
+                ++p;
+                u64 from = 0;  // a piece holds the fixed fields or nothing, a stream's lengths and its meta
+                for (int i = 0; i < ns && ok; ++i) {
+                    ok = len - p >= 16;
+                    if (!ok) break;
+                    const u64 dl = u64_at(p), ml = u64_at(p + 8);
+                    p += 16;
+                    ok = ml <= len - p && dl <= len - p - ml;
+                    take(from, p - from + (ok ? ml : 0));
+                    p += ok ? ml + dl : 0;
+                    from = p;
+                }
+                if (ok && len - p >= 12) take(p, 12);
+            }
+        }
+    }
+    __syncthreads();
+    u8* bytes = out + sizeof(HeaderPieces);
+    for (u32 i = 0; i < hp.count; ++i)
+        for (u32 b = threadIdx.x; b < hp.piece[i].len; b += kThreads)
+            bytes[hp.piece[i].at + b] = __ldg(c + hp.piece[i].off + b);
+    for (u32 b = threadIdx.x; b < sizeof(HeaderPieces) / 4; b += kThreads)
+        reinterpret_cast<u32*>(out)[b] = reinterpret_cast<const u32*>(&hp)[b];
+}
+
 // ---------------------------------------------------------------- helpers --------------
 __global__ void fill_u32_kernel(u32* p, u64 n, u32 v) {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) p[i] = v;
@@ -496,6 +553,9 @@ inline int grid_cap(u64 n) {
 
 }  // namespace
 
+void launch_header(const uint8_t* cont, uint64_t len, int rle, uint8_t* out, cudaStream_t st) {
+    header_kernel<<<1, kThreads, 0, st>>>(cont, len, kExtendedMagic, rle ? 1 : 0, out);
+}
 void launch_block_streams(const uint32_t* words_blk, uint64_t base_blk, int width_blk, const uint32_t* words_cnt,
                           uint64_t base_cnt, int width_cnt, uint64_t nblocks, uint64_t units,
                           unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, ScanStatus status,

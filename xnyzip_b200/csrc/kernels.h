@@ -341,6 +341,22 @@ struct RecoverInputs {
     const int32_t* counts;         // -rle
     const unsigned long long* rep_val;  // extended container: repos / sfc delta per unit (replaces rep_sym + patches)
 };
+// Collects a container's header bytes (the fixed fields, every stream's lengths and meta, the trailing
+// offset) into pinned host memory at `out`: HeaderPieces, then the bytes.  Stops at lengths that leave
+// the container.
+struct HeaderPieces {
+    uint32_t count, unused;
+    struct {
+        uint64_t off;      // in the container
+        uint32_t len, at;  // bytes collected, and where after the struct
+    } piece[10];
+};
+constexpr size_t kHeaderBytes = 32768;
+// First 8 bytes of an extended container ("XNYZBX01"): the reference container follows,
+// except that the repos / SFC-delta stream is block-coded (k_blocks.cu).
+constexpr uint64_t kExtendedMagic = 0x313058425a594e58ull;
+void launch_header(const uint8_t* cont, uint64_t len, int rle, uint8_t* out, cudaStream_t st);
+
 // Block streams of block mode in one pass: bit-unpack (widths <= 64), inclusive prefix sums of
 // the block-id and block-count deltas, block-start marks (is_start zeroed by the caller).
 // status: [3][tiles], tiles = ceil(nblocks / 4096).
