@@ -74,7 +74,7 @@ struct Small {
     uint32_t over_n;
     uint32_t max_dense;
     uint32_t err;
-    uint32_t pad;
+    uint32_t empty_blocks;
     uint32_t fallback[8];
     uint32_t redone[8];  // decoder blocks that assumed a wrong entry, per stream
     unsigned long long max2[2];
@@ -92,6 +92,7 @@ struct Small {
     ByteCodes codes[2];
     uint32_t dense_bits[kCountDense];
     uint8_t dense_len[kCountDense];
+    alignas(16) uint16_t hil_inv2[2048];
     uint8_t hil_fwd[256];
     uint8_t hil_inv[256];
     float offset_in[4];
@@ -1510,13 +1511,13 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     // ---- arena plan ----
     Plan pl;
     pl.total = reserved;
-    const size_t o_blk = pl.add(8 * NB + 8);
+    const size_t o_cx = pl.add(4 * NB + 8), o_cy = pl.add(4 * NB + 8), o_cz = pl.add(4 * NB + 8);
     const size_t o_patch = pl.add(8 * P + 8);
-    const size_t o_rep = pl.add(U + 8), o_quad = pl.add(U + 8), o_isst = pl.add(U + 8), o_stb = pl.add(4 * U + 8);
-    const size_t o_counts = pl.add(4 * U + 8);
+    const size_t o_rep = pl.add(U + 16), o_quad = pl.add(U + 16), o_isst = pl.add(U + 16);
+    const size_t o_counts = pl.add(4 * U + 64);
     const size_t o_xw = h.ext ? pl.add(x_nb) : 0, o_xk = h.ext ? pl.add(x_nb) : 0, o_xoff = h.ext ? pl.add(8 * x_nb) : 0,
                  o_xpay = h.ext ? pl.add(4 * (cdiv(x_bits, 32) + 2)) : 0, o_rv = h.ext ? pl.add(8 * U + 8) : 0;
-    const LB lb_scan = plan_lb(pl, cdiv(std::max<uint64_t>(NB, 1), kScanTile), 3);
+    const LB lb_scan = plan_lb(pl, cdiv(std::max<uint64_t>(NB, 1), kBlockStreamTile), 3);
     struct TabOff {
         size_t root, tree, sym;
     };
@@ -1544,8 +1545,9 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         o_dagg[i] = pl.add(8 * ttiles[i] * kDecodeMaxL);
         o_dinc[i] = pl.add(16 * dtiles[i]);
     }
-    const uint64_t rtiles = cdiv(std::max<uint64_t>(U, 1), kScanTile);
-    const LB lb_rec = plan_lb(pl, rtiles, 3);
+    const uint64_t rtiles = cdiv(std::max<uint64_t>(U, 1), kRecoverTile);
+    const LB lb_rec = plan_lb(pl, rtiles, 1), lb_pre = plan_lb(pl, cdiv(rtiles, kPrefixTiles), 1);
+    const size_t o_prefix = pl.add(sizeof(TilePrefix) * (rtiles + 1));
     if (pl.total > c->arena.cap) return fail(XNYZ_ERR_OOM, "__grow__:" + std::to_string(pl.total));
 
     {
@@ -1555,6 +1557,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         for (int i = 0; i < 4; ++i) f.add(at<uint8_t>(c, o_dinc[i]), 16 * dtiles[i], 0);
         lb_clear(c, f, lb_scan);
         lb_clear(c, f, lb_rec);
+        lb_clear(c, f, lb_pre);
         if (!h.direct) f.add(at<uint8_t>(c, o_isst), align_up(U, 4), 0);  // block-start marks
         launch_fill(f.a, st);
     }
@@ -1575,15 +1578,20 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     // unpacked and scanned on the context's stream.
     TRY(fork_sides(c));
     // ---- block streams: bit-unpack + prefix sums ----
-    if (!h.direct && NB) {
+    // nx uses the size_t conversion of the stored int range (block_quantizer.hpp:163)
+    const uint64_t blocks_x = static_cast<uint64_t>(static_cast<int64_t>(h.rx)) / 128 + 1,
+                   blocks_y = static_cast<uint64_t>(static_cast<int64_t>(h.ry)) / 128 + 1;
+    const BlockCorners corners{at<uint32_t>(c, o_cx), at<uint32_t>(c, o_cy), at<uint32_t>(c, o_cz)};
+    auto launch_blocks = [&](bool compact) {
         uint64_t b0, b1;
         const uint32_t* w0 = words_of(h.streams[0], b0);
         const uint32_t* w1 = words_of(h.streams[1], b1);
-        Prof pr(c, "block_streams", 1, (w_blk + w_cnt) * NB / 8.0 + 8.0 * NB + 5.0 * std::min(NB, U));
-        launch_block_streams(w0, b0, w_blk, w1, b1, w_cnt, NB, U, at<unsigned long long>(c, o_blk),
-                             at<uint8_t>(c, o_isst), at<uint32_t>(c, o_stb), lb_state(c, lb_scan),
-                             SMALL_FIELD(c, tile_counters[20]), SMALL_FIELD(c, count_total), SMALL_FIELD(c, err), st);
-    }
+        Prof pr(c, "block_streams", 1, (w_blk + w_cnt) * NB / 8.0 + 12.0 * NB + 1.0 * std::min(NB, U));
+        launch_block_streams(w0, b0, w_blk, w1, b1, w_cnt, NB, U, blocks_x, blocks_y, compact, corners,
+                             at<uint8_t>(c, o_isst), lb_state(c, lb_scan), SMALL_FIELD(c, tile_counters[20]),
+                             SMALL_FIELD(c, count_total), SMALL_FIELD(c, empty_blocks), SMALL_FIELD(c, err), st);
+    };
+    if (!h.direct && NB) launch_blocks(false);
 
     // ---- entropy-coded streams ----
     std::vector<DecodeJob> jobs;
@@ -1667,17 +1675,12 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
                             at<unsigned long long>(c, o_xoff), at<unsigned long long>(c, o_rv), SMALL_FIELD(c, err),
                             xs);
     }
-    // The -rle count stream sums the point count as it decodes (totals[0], zeroed on its own
-    // stream first) unless the entry-table decoder takes it.
-    bool counts_summed = false;
-    for (auto& j : jobs)
-        if (rle && j.slot == 3 && j.width == 4 && !j.fill && (j.fixed_len || !j.tables)) counts_summed = true;
     // the self-synchronising decoder (its state is zero on entry) and the entry-table decoder
-    auto launch_sync = [&](const DecodeJob& j, cudaStream_t js, unsigned long long* sum_out) -> xnyz_status {
+    auto launch_sync = [&](const DecodeJob& j, cudaStream_t js) -> xnyz_status {
         launch_decode_sync(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.byte_symbols, j.nsym, j.width, j.out,
                            at<uint8_t>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
                            SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, redone[j.slot]),
-                           SMALL_FIELD(c, codewords[j.slot]), sum_out, js);
+                           SMALL_FIELD(c, codewords[j.slot]), js);
         return XNYZ_OK;
     };
     auto launch_tables = [&](const DecodeJob& j, cudaStream_t js) -> xnyz_status {
@@ -1700,41 +1703,55 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         cudaStream_t js = side(c, j.slot);
         Prof pr(c, j.kind == kCodeGolombRice ? "decode_golomb_rice" : (j.kind == kCodeHuffman ? "decode_huffman" : "decode_exp_golomb"),
                 1, j.total_bits / 8.0 + static_cast<double>(j.nsym) * j.width, js);
-        const bool sum = counts_summed && j.slot == 3;
-        unsigned long long* sum_out = sum ? SMALL_FIELD(c, totals[0]) : nullptr;
         if (j.fixed_len) {
             if (j.nsym * static_cast<uint64_t>(j.fixed_len) > j.total_bits)
                 return fail(XNYZ_ERR_BAD_STREAM, "Huffman stream shorter than its symbols");
             launch_decode_fixed(j.words, j.base_bits, j.total_bits, j.table, j.fixed_len, j.nsym, j.width, j.out,
-                                SMALL_FIELD(c, err), js, sum_out);
+                                SMALL_FIELD(c, err), js);
             continue;
         }
         if (j.tables) {  // (Huffman only)
             TRY(launch_tables(j, js));
             continue;
         }
-        TRY(launch_sync(j, js, sum_out));
+        TRY(launch_sync(j, js));
     }
     CUDA_TRY(cudaGetLastError());
     TRY(join_sides(c));
     hd2.end();
     HostPhase hd3(c, "d3_decode_sync");
-    // count total (for -rle) once the count stream is decoded; the fallback flags, totals,
-    // codeword counts and the error word come back in one copy.  A stream whose parallel
-    // decode gave up (rare) is decoded again sequentially and the counts re-summed.
-    auto count_total = [&]() -> xnyz_status {
-        if (!counts_summed) TRY(memset_small(c, offsetof(Small, totals), sizeof(unsigned long long) * 8, 0));
-        if (rle && U && !counts_summed) {
-            Prof pr(c, "count_total", 1, 4.0 * U);
-            launch_count_total(at<int32_t>(c, o_counts), U, SMALL_FIELD(c, totals[0]), st);
+    // the recover tiles' prefixes and the point count; the fallback flags, totals, codeword counts and
+    // the error word come back in one copy
+    auto prefixes = [&](bool again) -> xnyz_status {
+        if (again) {
+            Fills f;
+            lb_clear(c, f, lb_pre);
+            f.add(SMALL_FIELD(c, tile_counters[41]), 4, 0);
+            launch_fill(f.a, st);
+        }
+        {
+            Prof pr(c, "tile_prefix", 1, (h.ext ? 0.0 : 1.0) * U + (h.direct ? 0.0 : 1.0) * U + (rle ? 4.0 : 0.0) * U);
+            launch_tile_prefix(h.ext ? nullptr : at<uint8_t>(c, o_rep), h.direct ? nullptr : at<uint8_t>(c, o_isst),
+                               rle ? at<int32_t>(c, o_counts) : nullptr, U, at<TilePrefix>(c, o_prefix),
+                               lb_state(c, lb_pre), SMALL_FIELD(c, tile_counters[41]), SMALL_FIELD(c, totals[0]),
+                               SMALL_FIELD(c, err), st);
         }
         CUDA_TRY(cudaGetLastError());
         return fetch_small(c, offsetof(Small, err), offsetof(Small, first_rep) - offsetof(Small, err));
     };
-    TRY(count_total());
+    TRY(prefixes(false));
+    if (c->h_small->empty_blocks) {  // (never from an encoder) rank the blocks that have units
+        Fills f;
+        f.add(at<uint8_t>(c, o_isst), align_up(U, 4), 0);
+        lb_clear(c, f, lb_scan);
+        f.add(SMALL_FIELD(c, tile_counters[20]), 4, 0);
+        launch_fill(f.a, st);
+        launch_blocks(true);
+        TRY(prefixes(true));
+    }
     // A stream with wide values is decoded again with 64-bit output, one that did not fall in step
     // by the entry-table decoder, one whose bounded wait expired sequentially (each may take the
-    // next way in turn).  The counts are summed again.
+    // next way in turn).
     bool patch32 = true;
     for (int pass = 0; pass < 3; ++pass) {
         bool again = false;
@@ -1750,7 +1767,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, tile_counters[30 + j.slot]), 0, 4, st));
             if (why == 4u) {
                 CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_dinc[j.slot]), 0, 16 * dtiles[j.slot], st));
-                TRY(launch_sync(j, st, nullptr));
+                TRY(launch_sync(j, st));
             } else if (!(why & 1u) && !j.tables) {
                 j.tables = true;
                 TRY(launch_tables(j, st));
@@ -1761,8 +1778,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             again = true;
         }
         if (!again) break;
-        counts_summed = false;
-        TRY(count_total());
+        TRY(prefixes(true));
     }
     TRY(device_errors(c));
     for (auto& j : jobs)
@@ -1788,11 +1804,8 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     rp.off[0] = h.off[0];
     rp.off[1] = h.off[1];
     rp.off[2] = h.off[2];
-    // nx uses the size_t conversion of the stored int range (block_quantizer.hpp:163)
-    rp.nx = static_cast<uint64_t>(static_cast<int64_t>(h.rx)) / 128 + 1;
-    rp.ny = static_cast<uint64_t>(static_cast<int64_t>(h.ry)) / 128 + 1;
-    rp.div_nx = make_u64div(rp.nx);
-    rp.div_ny = make_u64div(rp.ny);
+    // coordinates are 0 or between 2^-39 and 2^74 bounds of a reciprocal product: no under- or overflow
+    if (q.s >= 0x1p-40f && q.s <= 0x1p40f) rp.rinv = static_cast<float>(1.0 / static_cast<double>(q.rdiv));
     rp.hilbert = h.hilbert;
     rp.hstart_inv = hm.inv_block_start;
     rp.rle = rle && !cells_out;
@@ -1806,21 +1819,21 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         rp.bits = bits;
     }
     RecoverInputs ri{};
+    ri.prefix = at<TilePrefix>(c, o_prefix);
     ri.rep_sym = at<uint8_t>(c, o_rep);
     ri.rep_patch = at<unsigned long long>(c, o_patch);
     ri.patch32 = patch32;
     ri.npatch = P;
     ri.quad_sym = at<uint8_t>(c, o_quad);
     ri.is_start = at<uint8_t>(c, o_isst);
-    ri.start_block = at<uint32_t>(c, o_stb);
-    ri.blk_ids = at<unsigned long long>(c, o_blk);
+    ri.corners = corners;
     ri.nblocks = NB;
     ri.counts = at<int32_t>(c, o_counts);
     ri.rep_val = h.ext ? at<unsigned long long>(c, o_rv) : nullptr;
     float* out = at<float>(c, o_out);
     Prof pr_rec(c, "recover_units", 1,
                 (h.direct ? 1.0 : 7.0) * U + 8.0 * P + (rle ? 4.0 * U : 0.0) + 12.0 * static_cast<double>(nout));
-    launch_recover_units(ri, U, nout, rp, c->d_small->hil_inv, lb_state(c, lb_rec),
+    launch_recover_units(ri, U, nout, rp, c->d_small->hil_inv, c->d_small->hil_inv2, lb_state(c, lb_rec),
                          SMALL_FIELD(c, tile_counters[40]), out, SMALL_FIELD(c, err), st);
     CUDA_TRY(cudaGetLastError());
     pr_rec.end();
@@ -1897,6 +1910,7 @@ xnyz_status xnyz_create(xnyz_ctx** out, int device, void* stream) {
     CUDA_TRY(cudaMemset(c->d_small, 0, sizeof(Small)));
     CUDA_TRY(cudaMemcpy(c->d_small->hil_fwd, hilbert_machines().fwd.data(), 256, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(c->d_small->hil_inv, hilbert_machines().inv.data(), 256, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(c->d_small->hil_inv2, hilbert_machines().inv2.data(), 4096, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_small), sizeof(Small), cudaHostAllocDefault));
     std::memset(c->h_small, 0, sizeof(Small));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_head), kHeaderBytes, cudaHostAllocDefault));
@@ -2250,9 +2264,10 @@ xnyz_status xnyz_decompress_device(xnyz_ctx* c, const uint8_t* dev_container, ui
         return fail(XNYZ_ERR_INVALID_ARG, "quantizer must be 0 (cube), 1 (truncated octahedron) or 2 (adaptive)");
     CUDA_TRY(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
-    // The kernels read the streams as aligned 4-byte words, at most 12 bytes past a stream's end,
-    // which is where the next stream's lengths or the container's offset lie: a container on a
-    // 4-byte boundary is decoded in place, any other is copied to one.
+    // The kernels read the streams as aligned 4-byte words, at most 12 bytes past a stream's end
+    // (the block streams in 16-byte pieces, at most 28 past it), which is where the next streams'
+    // lengths or the container's offset lie: a container on a 4-byte boundary is decoded in place,
+    // any other is copied to one.
     const uint8_t* d_cont = dev_container;
     size_t reserved = 0;
     if (reinterpret_cast<uintptr_t>(dev_container) & 3u) {

@@ -152,18 +152,8 @@ __device__ __forceinline__ Pair ld_status(const Status* p, u32& flag) {
 // Two sums side by side (lo wraps modulo 2^64, hi stays below 2^62).
 struct PairAdd {
     __device__ __forceinline__ Pair operator()(Pair a, Pair b) const { return Pair{a.lo + b.lo, a.hi + b.hi}; }
-};
-
-// Segmented sum element: `head` = a segment starts inside, `sum` = sum since the last
-// segment start (or of everything if no start).  combine(a, b) = a followed by b.
-struct Seg {
-    u64 head;  // 0 or 1
-    u64 sum;
-};
-struct SegOp {
-    __device__ __forceinline__ Seg operator()(Seg a, Seg b) const {
-        return Seg{a.head | b.head, b.head ? b.sum : a.sum + b.sum};
-    }
+    // whether nothing before a tile with this value matters to the tiles after it
+    __device__ static __forceinline__ bool closed(Pair) { return false; }
 };
 
 // Exclusive prefix of `tile` (to every lane), publishing its inclusive prefix; called by all 32 lanes
@@ -171,15 +161,13 @@ struct SegOp {
 // all in flight together, waits until those up to the nearest inclusive prefix have been published
 // and combines them, earlier tiles first (`op` need not commute; {0, 0} is its identity).  A wide
 // window matters: with all tiles of a wave publishing at about the same time, the prefixes spread
-// by the window per step.
+// by the window per step.  A tile whose value is closed (Op::closed) ends the walk as an inclusive
+// prefix does.
 template <typename Op>
 __device__ Pair chain_lookback(Status* status, u32 tile, Pair mine, Op op, u32* err) {
     const int lane = (int)(threadIdx.x & 31u);
-    if (tile == 0) {
-        if (lane == 0) st_status(&status[0], mine, 2u);
-        return Pair{0, 0};
-    }
-    if (lane == 0) st_status(&status[tile], mine, 1u);
+    if (lane == 0) st_status(&status[tile], mine, tile == 0 || Op::closed(mine) ? 2u : 1u);
+    if (tile == 0) return Pair{0, 0};
     Pair acc{0, 0};
     i64 top = (i64)tile - 1;
     u32 spins = 0;
@@ -225,7 +213,7 @@ __device__ Pair chain_lookback(Status* status, u32 tile, Pair mine, Op op, u32* 
     }
     if (lane == 0) {
         if (failed) atomicOr(err, kErrTimeout);
-        st_status(&status[tile], op(acc, mine), 2u);
+        if (!Op::closed(mine)) st_status(&status[tile], op(acc, mine), 2u);
     }
     return acc;
 }

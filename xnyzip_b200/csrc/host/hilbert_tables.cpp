@@ -146,6 +146,13 @@ HilbertMachines make() {
         next = compose(B, child_h2m[md]);
         return static_cast<int>(B[md]);
     });
+    for (uint32_t st = 0; st < 32; ++st)
+        for (uint32_t d = 0; d < 64; ++d) {
+            const uint32_t e1 = hm.inv[st * 8 + (d >> 3)], e0 = hm.inv[(e1 >> 3) * 8 + (d & 7)];
+            uint32_t v = (e0 >> 3) << 6;
+            for (int a = 0; a < 3; ++a) v |= ((((e1 >> a) & 1) << 1) | ((e0 >> a) & 1)) << (2 * a);
+            hm.inv2[st * 64 + d] = static_cast<uint16_t>(v);
+        }
     uint32_t s = 0, t = 0;
     for (int level = 20; level >= 6; --level) {
         if ((hm.fwd[s * 8] & 7) != 0 || (hm.inv[t * 8] & 7) != 0)

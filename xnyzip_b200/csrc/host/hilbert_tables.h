@@ -12,6 +12,8 @@ namespace xnyz {
 struct HilbertMachines {
     std::array<uint8_t, 256> fwd;   // Morton -> Hilbert (mortonToHilbert3)
     std::array<uint8_t, 256> inv;   // Hilbert -> Morton (hilbertToMorton3)
+    // two levels of `inv` per entry [state * 64 + two digits]: x | y << 2 | z << 4 | next state << 6
+    std::array<uint16_t, 2048> inv2;
     uint32_t fwd_block_start;       // state after levels 20..6 of zero digits (18-bit local codes)
     uint32_t inv_block_start;
     int fwd_states;

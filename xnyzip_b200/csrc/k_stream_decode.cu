@@ -914,7 +914,6 @@ struct SyncArgs {
     u32* need_fallback;
     u32* redone;
     unsigned long long* total_codewords;
-    unsigned long long* sum_out;  // 32-bit symbols: sum of max(symbol, 0), or null
 };
 
 __host__ __device__ inline size_t sync_smem(int S, int rb, int mb) {
@@ -1280,7 +1279,6 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     }
     if (tile == gridDim.x - 1 && t == 0) *a.total_codewords = s_first + total;
 
-    u64 sum = 0;
     u64 idx = s_first + before;
     if (own && entry < Bend && idx < a.nsym && !(ld_volatile(a.need_fallback) & ~kWideValue)) {
         u32 q = (u32)(entry - str.org);
@@ -1302,10 +1300,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
                         br.put(syms, n);
                         idx += n;
                     } else {
-                        for (u32 i = 0; i < n; ++i, syms >>= 8, ++idx) {
-                            wr.put(idx, syms & 0xffu);
-                            sum += syms & 0xffu;
-                        }
+                        for (u32 i = 0; i < n; ++i, syms >>= 8, ++idx) wr.put(idx, syms & 0xffu);
                     }
                     continue;
                 }
@@ -1321,7 +1316,6 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
             } else if (a.out_width == 4) {
                 wr.put(idx, (u32)v);
                 wide |= (v >> 32) != 0;
-                sum += (u64)max((i32)(u32)v, 0);
             } else {
                 static_cast<u64*>(a.out)[idx] = v;
             }
@@ -1332,10 +1326,6 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
         if (KIND == kCodeHuffman && bytes) br.finish();
         else if (a.out_width == 4 && idx > wr.first) wr.finish(idx);
         if (KIND == kCodeGolombRice && wide) atomicOr(a.need_fallback, kWideValue);
-    }
-    if (a.sum_out) {
-        sum = warp_sum(sum);
-        if (lane == 0 && sum) atomicAdd(a.sum_out, sum);
     }
 }
 
@@ -1380,10 +1370,8 @@ __global__ void decode_sequential_kernel(Args a) {
 __global__ void __launch_bounds__(256) decode_fixed_kernel(const u32* __restrict__ words, u32 base, u64 nwords,
                                                            int len, const u32* __restrict__ root,
                                                            const u64* __restrict__ symvals, u64 nsym, int width,
-                                                           void* out, bool packed_ok, u32* err,
-                                                           unsigned long long* sum_out) {
+                                                           void* out, bool packed_ok, u32* err) {
     const u64 groups = (nsym + 3) / 4;
-    u64 sum = 0;  // sum_out: the sum of max(symbol, 0) over 32-bit symbols (the -rle point count)
     auto wbe = [&](u64 k) -> u64 { return k < nwords ? (u64)__byte_perm(__ldg(words + k), 0, 0x0123) : 0ull; };
     for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += (u64)gridDim.x * blockDim.x) {
         const u64 i0 = 4 * g;
@@ -1405,7 +1393,6 @@ __global__ void __launch_bounds__(256) decode_fixed_kernel(const u32* __restrict
                 packed |= ((u32)val & 0xffu) << (8 * j);
             } else {
                 reinterpret_cast<u32*>(out)[i0 + j] = (u32)val;
-                sum += (u64)max((i32)(u32)val, 0);
             }
         }
         if (width == 1) {
@@ -1417,11 +1404,6 @@ __global__ void __launch_bounds__(256) decode_fixed_kernel(const u32* __restrict
             }
         }
         if (bad) atomicOr(err, kErrBadStream);
-    }
-    if (sum_out) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFullMask, sum, d);
-        if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(sum_out, sum);
     }
 }
 
@@ -1517,7 +1499,7 @@ SyncGeometry sync_geometry(int kind, uint64_t total_bits) {
 void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
                         bool byte_symbols, uint64_t nsym, int out_width, void* out, void* status,
                         uint32_t* tile_counter, uint32_t* err, uint32_t* need_fallback, uint32_t* redone, unsigned long long* total_codewords,
-                        unsigned long long* sum_out, cudaStream_t st) {
+                        cudaStream_t st) {
     if (kind == kCodeHuffman && (t.root_bits < 1 || t.root_bits > kMaxRootBits)) {
         atomic_flag_host_error(err, st);  // the host builds tables with 1 <= root_bits <= 11
         return;
@@ -1548,7 +1530,6 @@ void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uin
     a.need_fallback = need_fallback;
     a.redone = redone;
     a.total_codewords = total_codewords;
-    a.sum_out = out_width == 4 ? sum_out : nullptr;
     const unsigned tiles = (unsigned)g.tiles;
     // at most 16.5 KB of words, 16 KB of tables and 1 KB of exits: below the 48 KB that need no opt-in
     const int smem = (int)sync_smem(g.S, a.code.rb, a.mb);
@@ -1561,8 +1542,7 @@ void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uin
 }
 
 void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t, int len,
-                         uint64_t nsym, int out_width, void* out, uint32_t* err, cudaStream_t st,
-                         unsigned long long* sum_out) {
+                         uint64_t nsym, int out_width, void* out, uint32_t* err, cudaStream_t st) {
     if (!nsym) return;
     if (len < 1 || len > kMaxRootBits || len != t.root_bits || (out_width != 1 && out_width != 4) ||
         nsym * (uint64_t)len > total_bits) {
@@ -1574,8 +1554,7 @@ void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t tot
     if (blocks > 148 * 16) blocks = 148 * 16;
     const bool packed_ok = (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
     decode_fixed_kernel<<<(unsigned)blocks, 256, 0, st>>>(words, (u32)base_bits, nwords, len, t.root, t.symvals, nsym,
-                                                          out_width, out, packed_ok, err,
-                                                          out_width == 4 ? sum_out : nullptr);
+                                                          out_width, out, packed_ok, err);
 }
 
 void launch_decode_sequential(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits,

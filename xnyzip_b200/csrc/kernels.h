@@ -233,7 +233,6 @@ struct FillArgs {
 void launch_fill(const FillArgs& args, cudaStream_t st);
 
 // --- decompress -------------------------------------------------------------------------
-constexpr int kScanTile = 4096;  // elements per tile of the decompress-side chained scans
 
 // Parallel decoding of one unindexed prefix-code stream (Huffman, Golomb-Rice, exp-Golomb),
 // implemented in k_stream_decode.cu.
@@ -268,8 +267,7 @@ void launch_decode_stream(int kind, const uint32_t* words, uint64_t base_bits, u
 // from any bit offset.  *need_fallback (starts at 0) tells why the stream has to be decoded
 // otherwise: 1 a bounded wait expired, 2 it did not fall in step, 4 a Golomb-Rice value of 2^32 or
 // more with out_width 4.  status: 16 bytes per tile, zeroed, 16-byte aligned; *redone starts at 0.
-// out: 16-byte aligned.  byte_symbols: every symbol value is below 256.  out_width 4: *sum_out
-// (when given) grows by the sum of max(symbol, 0).
+// out: 16-byte aligned.  byte_symbols: every symbol value is below 256.
 struct SyncGeometry {
     int S;           // bits per subsequence
     int G;           // subsequences a block decodes ahead of its own
@@ -279,28 +277,27 @@ SyncGeometry sync_geometry(int kind, uint64_t total_bits);
 void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t,
                         bool byte_symbols, uint64_t nsym, int out_width, void* out, void* status,
                         uint32_t* tile_counter, uint32_t* err, uint32_t* need_fallback, uint32_t* redone,
-                        unsigned long long* total_codewords, unsigned long long* sum_out, cudaStream_t st);
+                        unsigned long long* total_codewords, cudaStream_t st);
 // One-thread decoder the host runs when a bounded wait of the parallel decoder expired.
 // A Huffman stream whose codewords all have length len (== t.root_bits <= 11): every symbol
-// from its own len bits (out_width 1: u8, 4: u32 values; with out_width 4 and sum_out, *sum_out
-// += the sum of max(value, 0) over the values, as int32).
+// from its own len bits (out_width 1: u8, 4: u32 values).
 void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t, int len,
-                         uint64_t nsym, int out_width, void* out, uint32_t* err, cudaStream_t st,
-                         unsigned long long* sum_out = nullptr);
+                         uint64_t nsym, int out_width, void* out, uint32_t* err, cudaStream_t st);
 void launch_decode_sequential(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits,
                               DecodeTable t, uint64_t nsym, int out_width, void* out,
                               unsigned long long* total_codewords, uint32_t* err, cudaStream_t st);
-void launch_count_total(const int32_t* counts, uint64_t n, unsigned long long* total, cudaStream_t st);
 void launch_fill_u8(uint8_t* p, uint64_t n, uint8_t v, cudaStream_t st);
 void launch_fill_u32(uint32_t* p, uint64_t n, uint32_t v, cudaStream_t st);
 
 // Division of any 64-bit value by an invariant divisor d >= 1 through one high multiply
 // (T. Granlund and P. Montgomery, "Division by invariant integers using multiplication",
 // PLDI 1994, section 4, figure 4.1): with l = ceil(log2 d) and m = floor(2^64 (2^l - d) / d)
-// + 1, x / d = (t + ((x - t) >> min(l, 1))) >> max(l - 1, 0) where t = mulhi(m, x).
+// + 1, x / d = (t + ((x - t) >> min(l, 1))) >> max(l - 1, 0) where t = mulhi(m, x).  For x below
+// 2^44 (all block ids but those of z = -1 cells) the same theorem with N = 44 needs no correction:
+// x / d = mulhi(x << 20, m44) >> l with m44 = ceil(2^(44 + l) / d).
 struct U64Div {
-    unsigned long long m;
-    unsigned int sh1, sh2;
+    unsigned long long m, m44;
+    unsigned int sh1, sh2, l44;
 };
 inline U64Div make_u64div(unsigned long long d) {
     unsigned int l = 0;
@@ -311,6 +308,8 @@ inline U64Div make_u64div(unsigned long long d) {
     r.m = static_cast<unsigned long long>(num / d + 1);
     r.sh1 = l < 1 ? l : 1;
     r.sh2 = l > 1 ? l - 1 : 0;
+    r.m44 = static_cast<unsigned long long>(((static_cast<unsigned __int128>(1) << (44 + l)) + d - 1) / d);
+    r.l44 = l < 63 ? l : 63;
     return r;
 }
 
@@ -318,9 +317,8 @@ inline U64Div make_u64div(unsigned long long d) {
 // -rle expansion, recover and unshift.
 struct RecoverParams {
     QuantParams q;
+    float rinv;  // 1 / q.rdiv correctly rounded, or 0: divide (a bound near the float range's ends)
     float off[3];
-    unsigned long long nx, ny;
-    U64Div div_nx, div_ny;   // make_u64div(nx), make_u64div(ny)
     int hilbert;
     unsigned int hstart_inv;  // inverse-Hilbert state after levels 20..6 of zero digits
     int rle;
@@ -328,17 +326,26 @@ struct RecoverParams {
     int bits;   // direct mode hilbert_bits
     int cells;  // write the units' int32 lattice cells instead of points (no expansion, no recover)
 };
+// Lattice corner of each block that has units, in order.
+struct BlockCorners {
+    uint32_t *x, *y, *z;
+};
+// What comes before a tile of kRecoverTile units: patches (zero symbols), block starts, outputs.
+struct TilePrefix {
+    uint32_t zeros, starts;
+    unsigned long long outputs;
+};
 struct RecoverInputs {
-    const uint8_t* rep_sym;
-    const void* rep_patch;      // Golomb-Rice decoded patches: u32 when patch32, else u64
+    const TilePrefix* prefix;      // per tile and one past the last (launch_tile_prefix)
+    const uint8_t* rep_sym;        // byte arrays: 8-byte aligned, readable 8 bytes past the end
+    const void* rep_patch;         // Golomb-Rice decoded patches: u32 when patch32, else u64
     int patch32;
     uint64_t npatch;
     const uint8_t* quad_sym;
     const uint8_t* is_start;       // block mode: 1 where a non-empty block starts
-    const uint32_t* start_block;   // block mode: block index at those units
-    const unsigned long long* blk_ids;
+    BlockCorners corners;
     uint64_t nblocks;
-    const int32_t* counts;         // -rle
+    const int32_t* counts;         // -rle: 16-byte aligned, readable 32 bytes past the end
     const unsigned long long* rep_val;  // extended container: repos / sfc delta per unit (replaces rep_sym + patches)
 };
 // Collects a container's header bytes (the fixed fields, every stream's lengths and meta, the trailing
@@ -358,17 +365,27 @@ constexpr uint64_t kExtendedMagic = 0x313058425a594e58ull;
 void launch_header(const uint8_t* cont, uint64_t len, int rle, uint8_t* out, cudaStream_t st);
 
 // Block streams of block mode in one pass: bit-unpack (widths <= 64), inclusive prefix sums of
-// the block-id and block-count deltas, block-start marks (is_start zeroed by the caller).
-// status: [3][tiles], tiles = ceil(nblocks / 4096).
+// the block-id and block-count deltas, block-start marks (is_start zeroed by the caller) and corners.
+// Sets *empty when a block has no units: then call again with `compact` (everything zeroed again).
+// The words of each stream are read from the 16-byte boundary before its first to the one after the
+// 12 bytes past its last.  status: [3][tiles], tiles = ceil(nblocks / kBlockStreamTile).
+constexpr int kBlockStreamTile = 2048;
 void launch_block_streams(const uint32_t* words_blk, uint64_t base_blk, int width_blk, const uint32_t* words_cnt,
-                          uint64_t base_cnt, int width_cnt, uint64_t nblocks, uint64_t units,
-                          unsigned long long* blk_ids, uint8_t* is_start, uint32_t* start_block, ScanStatus status,
-                          uint32_t* tile_counter, unsigned long long* count_total, uint32_t* err, cudaStream_t st);
-// status: [3][tiles], tiles = ceil(units / 4096)
+                          uint64_t base_cnt, int width_cnt, uint64_t nblocks, uint64_t units, uint64_t nx, uint64_t ny,
+                          bool compact, BlockCorners corners, uint8_t* is_start, ScanStatus status, uint32_t* tile_counter,
+                          unsigned long long* count_total, uint32_t* empty, uint32_t* err, cudaStream_t st);
+constexpr int kRecoverTile = 2048;
+// Prefixes of the recover tiles, and the outputs' number; null inputs count nothing (rep_sym: no patches,
+// is_start: direct mode, counts: -normal).  status: one word per kPrefixTiles tiles.
+constexpr int kPrefixTiles = 4;
+void launch_tile_prefix(const uint8_t* rep_sym, const uint8_t* is_start, const int32_t* counts, uint64_t units,
+                        TilePrefix* out, ScanStatus status, uint32_t* tile_counter, unsigned long long* count_total,
+                        uint32_t* err, cudaStream_t st);
+// status: [tiles], tiles = ceil(units / kRecoverTile); hilbert_inv2: two levels of the inverse
+// machine per entry ([32][64]: x | y << 2 | z << 4 | next state << 6)
 void launch_recover_units(const RecoverInputs& in, uint64_t units, uint64_t nout, RecoverParams rp,
-                          const uint8_t* hilbert_inv_tab, ScanStatus status, uint32_t* tile_counter, float* out,
-                          uint32_t* err, cudaStream_t st);
-
+                          const uint8_t* hilbert_inv_tab, const uint16_t* hilbert_inv2, ScanStatus status,
+                          uint32_t* tile_counter, float* out, uint32_t* err, cudaStream_t st);
 
 // --- block-parameter coding (extended container) and its predictor ------------------------
 constexpr int kParamBlock = 1024;     // values per block
