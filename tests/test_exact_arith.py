@@ -1,6 +1,7 @@
-"""The decoder's replacements for divisions, restated on the host: the block coordinates' division of
-ids below 2^44 by one high multiply, and the recovered coordinates' division by the rounded constants
-sqrt(3) and sqrt(5) through the reciprocal with one fused correction (every significand)."""
+"""Replacements for divisions and roundings, restated on the host: the block coordinates' division of
+ids below 2^44 by one high multiply; the recovered coordinates' division by the rounded constants
+sqrt(3) and sqrt(5) through the reciprocal with one fused correction, and the quantizers' by any step
+with two (every significand); the truncated octahedron's two lattice candidates from the floor."""
 import os
 import shutil
 import subprocess
@@ -21,9 +22,49 @@ static float div_const(float x, float d, float y) {
     const float q = x * y;
     return std::fmaf(std::fmaf(-q, d, x), y, q);
 }
+static float div_any(float x, float d, float y) {
+    float q = x * y;
+    q = std::fmaf(std::fmaf(-q, d, x), y, q);
+    return std::fmaf(std::fmaf(-q, d, x), y, q);
+}
+static long candidates(float q) {  // as the quantizer defines them, and from floor(q)
+    const float e = std::round(q * 0.5f) * 2.0f, o = std::round((q - 1.0f) * 0.5f) * 2.0f + 1.0f;
+    const int f = (int)std::floor(q);
+    const float e2 = (float)(f + (f & 1)), o2 = q <= 0x1p-25f ? -1.0f : (float)(f | 1);
+    return (e != e2) + (o != o2);
+}
 int main() {
     std::mt19937_64 rng(11);
     long bad = 0;
+    for (int i = 0; i < 16; ++i) {
+        // 1, just above 1, just below 2, and steps of any significand and size
+        const unsigned m = i == 0 ? 0u : i == 1 ? 1u : i == 2 ? 0x7ffffeu : (unsigned)(rng() & 0x7fffffu);
+        if (m == 0x7fffffu) continue;
+        const unsigned db = (i < 4 ? 127u : 127u - 42u + (unsigned)(rng() % 85)) << 23 | m;
+        float d, x;
+        std::memcpy(&d, &db, 4);
+        const float y = (float)(1.0 / (double)d);
+        for (unsigned b = 0x3f800000u; b < 0x40000000u; ++b) {
+            std::memcpy(&x, &b, 4);
+            if (div_any(x, d, y) != x / d) ++bad;
+        }
+        for (int e : {-60, -31, 17, 59})
+            for (int k = 0; k < 100000; ++k) {
+                x = std::ldexp((float)((rng() >> 40) | (1 << 23)), e - 23);
+                if (div_any(x, d, y) != x / d) ++bad;
+            }
+        if (div_any(0.0f, d, y) != 0.0f) ++bad;
+    }
+    for (unsigned b = 0; b < 0x4b700000u; b += b < 0x3c000000u ? 997u : 13u) {  // 0 to 2^24 - 2^20
+        float q;
+        std::memcpy(&q, &b, 4);
+        bad += candidates(q);
+    }
+    for (float c = 0x1p-26f; c < 16000000.0f; c = c < 0.5f ? c * 2.0f : c < 4096.0f ? c + 0.5f : c * 1.0009f) {
+        const float k = c < 0.5f ? c : std::round(c * 2.0f) * 0.5f;
+        for (float q : {k, std::nextafterf(k, 0.0f), std::nextafterf(k, 1e9f)}) bad += candidates(q);
+    }
+    if (candidates(-0.0f)) ++bad;
     for (int i = 0; i < 400; ++i) {
         const u64 d = i < 40 ? (u64)i + 1 : i < 64 ? 1ull << (i - 39) : (rng() >> (39 + rng() % 25)) + 1;
         const auto m = xnyz::dev::make_u64div(d);

@@ -93,6 +93,7 @@ struct Small {
     uint32_t dense_bits[kCountDense];
     uint8_t dense_len[kCountDense];
     alignas(16) uint16_t hil_inv2[2048];
+    alignas(16) uint16_t hil_fwd2[2048];
     uint8_t hil_fwd[256];
     uint8_t hil_inv[256];
     float offset_in[4];
@@ -334,6 +335,14 @@ QuantParams make_quant(int quantizer, float l2) {
     q.div = static_cast<float>(static_cast<double>(2.0f * l2) / std::sqrt(k));
     q.s = l2;
     q.rdiv = static_cast<float>(std::sqrt(k));
+    // Division by multiplication (device_common.cuh).  Recovered coordinates are 0 or between 2^-39 and
+    // 2^74: no under- or overflow.  A divisor whose significand is all ones is left out.
+    uint32_t bits;
+    std::memcpy(&bits, &q.div, 4);
+    if (q.s >= 0x1p-40f && q.s <= 0x1p40f) {
+        q.rinv = static_cast<float>(1.0 / static_cast<double>(q.rdiv));
+        if ((bits & 0x7fffffu) != 0x7fffffu) q.inv = static_cast<float>(1.0 / static_cast<double>(q.div));
+    }
     return q;
 }
 
@@ -802,7 +811,7 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
             return fail(XNYZ_ERR_UNSUPPORTED, "block ids need more than 43 bits");
         const int B = bitlen(static_cast<uint64_t>(cells - 1));
         bkp.nx = static_cast<uint64_t>(nx);
-        bkp.ny = static_cast<uint64_t>(ny);
+        bkp.nxy = static_cast<uint64_t>(nx * ny);
         bkp.hilbert = hil;
         bkp.hstart = hm.fwd_block_start;
         key_bits = B + 21;
@@ -834,13 +843,13 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     {
         Prof pr(c, "keys", 1, 20.0 * n + (want_order ? 4.0 * n : 0.0));
         if (cin)
-            launch_keys_cells(cin->cells, n, bkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0], passes,
+            launch_keys_cells(cin->cells, n, bkp, c->d_small->hil_fwd2, sb.keys[0], sb.vals[0], passes,
                               c->d_small->sort_hist, st);
         else if (direct)
             launch_keys_direct(d_xyz, n, q, SMALL_FIELD(c, stats), dkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0],
                                passes, c->d_small->sort_hist, st);
         else
-            launch_keys_cells(cells_tmp, n, bkp, c->d_small->hil_fwd, sb.keys[0], sb.vals[0], passes,
+            launch_keys_cells(cells_tmp, n, bkp, c->d_small->hil_fwd2, sb.keys[0], sb.vals[0], passes,
                               c->d_small->sort_hist, st);
     }
     int res = 0;
@@ -1804,8 +1813,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     rp.off[0] = h.off[0];
     rp.off[1] = h.off[1];
     rp.off[2] = h.off[2];
-    // coordinates are 0 or between 2^-39 and 2^74 bounds of a reciprocal product: no under- or overflow
-    if (q.s >= 0x1p-40f && q.s <= 0x1p40f) rp.rinv = static_cast<float>(1.0 / static_cast<double>(q.rdiv));
     rp.hilbert = h.hilbert;
     rp.hstart_inv = hm.inv_block_start;
     rp.rle = rle && !cells_out;
@@ -1911,6 +1918,7 @@ xnyz_status xnyz_create(xnyz_ctx** out, int device, void* stream) {
     CUDA_TRY(cudaMemcpy(c->d_small->hil_fwd, hilbert_machines().fwd.data(), 256, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(c->d_small->hil_inv, hilbert_machines().inv.data(), 256, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(c->d_small->hil_inv2, hilbert_machines().inv2.data(), 4096, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(c->d_small->hil_fwd2, hilbert_machines().fwd2.data(), 4096, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_small), sizeof(Small), cudaHostAllocDefault));
     std::memset(c->h_small, 0, sizeof(Small));
     CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->h_head), kHeaderBytes, cudaHostAllocDefault));

@@ -236,6 +236,23 @@ __device__ __forceinline__ u32 claim_tile(u32* counter, u32* smem_slot) {
 // rdiv = float(sqrt(5 or 3)) (recover: ((v * 2) * s) / rdiv).
 using dev::QuantParams;
 
+// x / d correctly rounded, given y = RN(1 / d): one fused correction of x y (P. Markstein, IBM J. Res.
+// Dev. 34(1), 1990).  Used for the two constants sqrt(3) and sqrt(5) rounded to float, for which every
+// significand has been compared with IEEE division, and for |x| far from underflow and overflow.
+__device__ __forceinline__ float div_const(float x, float d, float y) {
+    const float q = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
+}
+
+// x / d correctly rounded for any divisor whose significand is not all ones, given y = RN(1 / d): two
+// corrections, the first of which makes the quotient faithful (P. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, 1990).  x is 0 or in [2^-60, 2^60], d in [2^-42, 2^42]: the remainders are exact.
+__device__ __forceinline__ float div_any(float x, float d, float y) {
+    float q = __fmul_rn(x, y);
+    q = __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
+    return __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
+}
+
 // static_cast<int>(float) as compiled for x86-64 (cvttss2si): truncation toward zero and
 // 0x80000000 for NaN or values outside the int range.
 __device__ __forceinline__ i32 f2i_x86(float f) {
@@ -409,20 +426,6 @@ __device__ __forceinline__ void hilbert_xyz6(const u8* tab, u32 code, u32 state,
         z |= ((e >> 2) & 1u) << l;
         state = e >> 3;
     }
-}
-
-// hilbert_apply(tab, morton3(x, y, z), 5, state) for x, y, z below 64: the input digit of
-// level l is bit l of x, y and z, so the interleave is done as the levels are consumed.
-__device__ __forceinline__ u32 hilbert_code6(const u8* tab, u32 x, u32 y, u32 z, u32 state) {
-    u32 out = 0;
-#pragma unroll
-    for (int l = 5; l >= 0; --l) {
-        const u32 d = ((x >> l) & 1u) | (((y >> l) & 1u) << 1) | (((z >> l) & 1u) << 2);
-        const u32 e = tab[state * 8 + d];
-        out |= (e & 7u) << (3 * l);
-        state = e >> 3;
-    }
-    return out;
 }
 
 // ------------------------------------------------------------- bit writers --------------

@@ -152,6 +152,9 @@ HilbertMachines make() {
             uint32_t v = (e0 >> 3) << 6;
             for (int a = 0; a < 3; ++a) v |= ((((e1 >> a) & 1) << 1) | ((e0 >> a) & 1)) << (2 * a);
             hm.inv2[st * 64 + d] = static_cast<uint16_t>(v);
+            auto digit = [&](int bit) { return ((d >> bit) & 1) | ((d >> (2 + bit) & 1) << 1) | ((d >> (4 + bit) & 1) << 2); };
+            const uint32_t f1 = hm.fwd[st * 8 + digit(1)], f0 = hm.fwd[(f1 >> 3) * 8 + digit(0)];
+            hm.fwd2[st * 64 + d] = static_cast<uint16_t>(((f1 & 7) << 3) | (f0 & 7) | ((f0 >> 3) << 6));
         }
     uint32_t s = 0, t = 0;
     for (int level = 20; level >= 6; --level) {

@@ -14,6 +14,8 @@ struct HilbertMachines {
     std::array<uint8_t, 256> inv;   // Hilbert -> Morton (hilbertToMorton3)
     // two levels of `inv` per entry [state * 64 + two digits]: x | y << 2 | z << 4 | next state << 6
     std::array<uint16_t, 2048> inv2;
+    // two levels of `fwd` per entry [state * 64 + x | y << 2 | z << 4]: both digits | next state << 6
+    std::array<uint16_t, 2048> fwd2;
     uint32_t fwd_block_start;       // state after levels 20..6 of zero digits (18-bit local codes)
     uint32_t inv_block_start;
     int fwd_states;

@@ -470,19 +470,11 @@ struct SegPair {
 };
 constexpr u64 kSegQuad = 1ull << 35, kSegRep = 1ull << 36;
 
-// x / d correctly rounded, given y = RN(1 / d): one fused correction of x y (P. Markstein, IBM J. Res.
-// Dev. 34(1), 1990).  Used for the two constants sqrt(3) and sqrt(5) rounded to float, for which every
-// significand has been compared with IEEE division, and for |x| far from underflow and overflow.
-__device__ __forceinline__ float div_const(float x, float d, float y) {
-    const float q = __fmul_rn(x, y);
-    return __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
-}
-
 // recover + unshift (device_common.cuh: recover), the divisions by the constant as above when allowed;
 // v * 2 * s is v * (2 s), doubling being exact.
 __device__ __forceinline__ void recover_point(const RecoverParams& p, i32 cx, i32 cy, i32 cz, float& x, float& y,
                                               float& z) {
-    if (!p.rinv || p.q.quantizer == 2) {
+    if (!p.q.rinv || p.q.quantizer == 2) {
         recover(p.q, cx, cy, cz, p.off[0], p.off[1], p.off[2], x, y, z);
         return;
     }
@@ -498,7 +490,7 @@ __device__ __forceinline__ void recover_point(const RecoverParams& p, i32 cx, i3
         f[2] = __fadd_rn(__int2float_rn(cz), 0.5f);
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) f[a] = div_const(__fmul_rn(f[a], 2.0f * p.q.s), p.q.rdiv, p.rinv);
+    for (int a = 0; a < 3; ++a) f[a] = div_const(__fmul_rn(f[a], 2.0f * p.q.s), p.q.rdiv, p.q.rinv);
     x = __fadd_rn(f[0], p.off[0]);
     y = __fadd_rn(f[1], p.off[1]);
     z = __fadd_rn(f[2], p.off[2]);

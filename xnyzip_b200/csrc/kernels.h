@@ -16,6 +16,8 @@ struct QuantParams {
     float div;      // float(double(2*l2)/sqrt(3|5))
     float s;        // l2 as float
     float rdiv;     // float(sqrt(3|5))
+    float inv;      // 1 / div correctly rounded, or 0: divide (quotients_exact)
+    float rinv;     // 1 / rdiv correctly rounded, or 0: divide (a bound near the float range's ends)
     float step[3];  // adaptive: per-axis steps (decompression: from the container)
     const float* step_dev;  // adaptive compression: the steps in device memory (PointStats::step)
 };
@@ -38,7 +40,7 @@ struct PointStats {
 // z = -1 (the truncated-octahedron edge case) carry `defect_flag` and the id minus
 // `defect_base` so that they sort after all other cells in the reference's id order.
 struct BlockKeyParams {
-    unsigned long long nx, ny;
+    unsigned long long nx, nxy;      // blocks per row, per layer (nx < 2^25)
     unsigned long long defect_flag;  // 0 if no z = -1 cells
     unsigned long long defect_base;  // ((2^64-1)/64/2) * nx * ny  (mod 2^64)
     int hilbert;
@@ -112,7 +114,7 @@ void launch_keys_direct(const float* xyz, uint64_t n, QuantParams q, const Point
 // Cell tables: block keys from int32 cells; per-axis min / max of cells (stats->min_cell /
 // max_cell, initialised by the caller); dst[i] = src[idx[i]]; expansion + recover + unshift
 // (status: ceil(n / 4096) tiles; *total receives the point count).
-void launch_keys_cells(const int32_t* cells, uint64_t n, BlockKeyParams kp, const uint8_t* hilbert_tab,
+void launch_keys_cells(const int32_t* cells, uint64_t n, BlockKeyParams kp, const uint16_t* hilbert_fwd2,
                        unsigned long long* keys, uint32_t* payload, int passes, uint32_t* hist, cudaStream_t st);
 void launch_cells_stats(const int32_t* cells, uint64_t n, PointStats* stats, cudaStream_t st);
 void launch_gather_i32(const int32_t* src, const uint32_t* idx, uint64_t n, int32_t* dst, cudaStream_t st);
@@ -317,7 +319,6 @@ inline U64Div make_u64div(unsigned long long d) {
 // -rle expansion, recover and unshift.
 struct RecoverParams {
     QuantParams q;
-    float rinv;  // 1 / q.rdiv correctly rounded, or 0: divide (a bound near the float range's ends)
     float off[3];
     int hilbert;
     unsigned int hstart_inv;  // inverse-Hilbert state after levels 20..6 of zero digits
