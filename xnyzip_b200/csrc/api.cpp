@@ -591,7 +591,7 @@ struct CPlan {
 };
 CPlan make_cplan(uint64_t n, bool want_order, size_t reserved, bool ext) {
     CPlan c{};
-    c.tiles = cdiv(n, kUnitTile);
+    c.tiles = cdiv(n, kEncTile);
     Plan pl;
     pl.total = reserved;
     c.o_k0 = pl.add(8 * n);
@@ -607,7 +607,7 @@ CPlan make_cplan(uint64_t n, bool want_order, size_t reserved, bool ext) {
     c.o_counts = pl.add(4 * n);
     c.o_over_v = pl.add(4 * n);
     c.o_over_u = pl.add(4 * n);
-    c.lb_units = plan_lb(pl, c.tiles, 1);
+    c.lb_units = plan_lb(pl, cdiv(n, unit_tile(n)), 1);
     c.lb_enc = plan_lb(pl, c.tiles, 4);
     if (ext) {
         const uint64_t nb = cdiv(n, kParamBlock);

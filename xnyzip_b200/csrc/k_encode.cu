@@ -26,7 +26,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;
-static_assert(kTile == kUnitTile && kTile == kEncTile, "tile size");
+static_assert(kTile == kEncTile, "tile size");
 
 __device__ __forceinline__ void block_key_fields(u64 k, const BlockKeyParams& kp, u64& id, u32& quad, u32& sfc) {
     id = (kp.defect_flag && k >= kp.defect_flag) ? (((k - kp.defect_flag) >> 21) + kp.defect_base) : (k >> 21);
@@ -38,207 +38,188 @@ __device__ __forceinline__ u64 direct_key_sfc(u64 k, const DirectKeyParams& kp) 
     return (kp.defect_flag && k >= kp.defect_flag) ? (kp.defect_high | (k - kp.defect_flag)) : k;
 }
 
-// Warp-aggregated histogram update with first-occurrence tracking; the lowest lane of a
-// group of equal symbols holds the smallest unit index (units grow with the lane).  The groups are
-// found through a per-warp bit mask in shared memory (one atomicOr per lane) instead of match.any,
-// which serialises on the address-divergence pipe.  `masks` is zero on entry and on return.
-__device__ __forceinline__ void hist_add_masked(u32* masks, u32* hist, u32* first, bool valid, u32 sym, u32 unit) {
-    const u32 lane = lane_id();
-    if (valid) atomicOr(&masks[sym], 1u << lane);
-    __syncwarp();
-    if (valid) {
-        const u32 peers = masks[sym];
-        if (lane == (u32)(__ffs(peers) - 1)) {
-            atomicAdd(&hist[sym], (u32)__popc(peers));
-            atomicMin(&first[sym], unit);
-        }
-    }
-    __syncwarp();
-    if (valid) masks[sym] = 0u;
-    __syncwarp();
+__device__ __forceinline__ void copy_async16(void* smem, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((u32)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
 }
 
-template <bool DIRECT>
+// Units from the sorted keys.  Warp w owns keys [32 ITEMS w, 32 ITEMS (w + 1)) of the tile, 32 consecutive
+// ones (one per lane) per round, so that a round's outputs land in consecutive units.  The first pass
+// classifies each key against the one before it and counts; the second places, tallies and writes.  What
+// a key came to (repos delta, flags, quad delta) stays in one register in between.
+//
+// Bound by instructions, then by the chain: classified twice, with the histogram's equal symbols found
+// by masks in shared memory, a key took 308 instructions and 64M keys 718 us; this 572 (3.3 TB/s).  (The
+// hardware merges equal addresses of a shared increment; the first unit of a symbol is only touched when
+// it gets smaller.)  Tiles of 2048 keys take 725 us for 64M: the chain.  Tiles of 1024 below kUnitSmall,
+// since a tile's rounds are serial: 1013 keys 19 -> 10 us, 120k 17 -> 13 (1M, tiles of 4096: 30 -> 22).
+template <bool DIRECT, int ITEMS>
 __global__ void __launch_bounds__(kThreads) units_kernel(const u64* __restrict__ keys, u64 n, int rle,
                                                          BlockKeyParams bkp, DirectKeyParams dkp, UnitOutputs out,
-                                                         ScanStatus status, u32* tile_counter, u32* err) {
-    __shared__ u64 sk[kTile + 1];
-    __shared__ u64 scratch[16];
+                                                         Status* status, u32* tile_counter, u32* err) {
+    constexpr int kT = kThreads * ITEMS, kW = kThreads / 32;
+    __shared__ __align__(16) u64 sk[kT + 2];  // [1] the key before the tile, [2 + e] key e
     __shared__ u32 slot;
+    __shared__ u32 hrep[256], frep[256], hquad[8], fquad[8];
+    __shared__ u32 wtot[kW];           // units | patches << 10 | blocks << 20 of each warp
     __shared__ u64 sbase[3];
-    __shared__ u32 hrep[256], frep[256], hquad[16], fquad[16];
-    __shared__ u32 mrep[kThreads / 32][256];
-    __shared__ u64 psum[kThreads / 32];
+    __shared__ unsigned long long psum;
 
     const u32 tile = claim_tile(tile_counter, &slot);
-    const u32 ntiles = gridDim.x;
-    const u64 base = (u64)tile * kTile;
-    const u32 cnt = (u32)min((u64)kTile, n - base);
-    const int tid = threadIdx.x;
-    if (tid == 0) sk[0] = base ? keys[base - 1] : 0ull;
-    for (int i = 0; i < kItems; ++i) {
-        const u32 e = (u32)i * kThreads + tid;
-        if (e < cnt) sk[1 + e] = keys[base + e];
+    const u64 base = (u64)tile * kT;
+    const u32 cnt = (u32)min((u64)kT, n - base);
+    const int tid = threadIdx.x, w = tid >> 5;
+    const u32 lane = lane_id(), lt = lanemask_lt();
+#pragma unroll
+    for (int i = 0; i < ITEMS / 2; ++i) {
+        const u32 e = ((u32)i * kThreads + tid) * 2u;
+        if (e + 1 < cnt) copy_async16(&sk[2 + e], keys + base + e);
+        else if (e < cnt) sk[2 + e] = keys[base + e];
     }
+    // the very first key differs from its predecessor in every bit: a head that starts a block
+    if (tid == 0) sk[1] = base ? keys[base - 1] : ~keys[0];
     hrep[tid] = 0;
     frep[tid] = 0xffffffffu;
-    if (tid < 16) {
+    if (tid < 8) {
         hquad[tid] = 0;
         fquad[tid] = 0xffffffffu;
     }
-    for (int i = tid; i < (kThreads / 32) * 256; i += kThreads) (&mrep[0][0])[i] = 0u;
+    if (tid == 0) psum = 0;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
-    // Element e of the tile: flags (bit0 head, bit1 patch, bit2 new block, bits 8..15 quad
-    // delta), repos / SFC delta and block id.  Computed in pass A for the counts and again in
-    // pass B from the staged keys (cheaper than holding 16 of each in registers).
-    auto classify = [&](u32 e, u64& val, u64& idv) -> u32 {
-        val = 0;
-        idv = 0;
-        if (e >= cnt) return 0u;
-        const u64 j = base + e;
-        const u64 k = sk[1 + e], kp = sk[e];
-        const bool head = !rle || j == 0 || k != kp;
-        if (!head) return 0u;
-        u32 f = 1u;
-        if (DIRECT) {
-            const u64 s = direct_key_sfc(k, dkp);
-            const u64 d = j == 0 ? s : s - direct_key_sfc(kp, dkp);
-            val = d;
-            if (d > 254u) f |= 2u;
-        } else {
-            u64 id, idp = 0;
-            u32 quad, sfc, quadp = 0, sfcp = 0;
-            block_key_fields(k, bkp, id, quad, sfc);
-            if (j > 0) block_key_fields(kp, bkp, idp, quadp, sfcp);
-            const bool nb = (j == 0) || id != idp;
-            u32 qd;
-            u64 r;
-            if (nb) {
-                qd = quad;
-                r = sfc;
-                f |= 4u;
-            } else if (quad != quadp) {
-                qd = quad - quadp;
-                r = sfc;
-            } else {
-                qd = 0;
-                r = (u64)sfc - (u64)sfcp;
-            }
-            val = r;
-            idv = id;
-            if (r > 254u) f |= 2u;
-            f |= (qd & 0xffu) << 8;
-        }
-        return f;
+    const u32 e0 = (u32)w * (32u * ITEMS) + lane;
+    auto sfc_delta = [&](u32 e) -> u64 {  // direct mode
+        const u64 s = direct_key_sfc(sk[2 + e], dkp);
+        return base + e ? s - direct_key_sfc(sk[1 + e], dkp) : s;
     };
-    // Warp w owns elements [512 w, 512 w + 512) of the tile, taken 32 consecutive elements
-    // (one per lane) per round: staged keys are read without bank conflicts, and the
-    // outputs of a round land in consecutive units, so the stores coalesce.
-    const int w = tid >> 5;
-    const u32 lane = lane_id();
-    const u32 wfirst = (u32)w * (32u * kItems);
-    // Pass A: count heads, patches and new blocks of my 16 elements.
-    u32 h = 0, p = 0, b = 0;
-    for (int r = 0; r < kItems; ++r) {
-        u64 v, id;
-        const u32 f = classify(wfirst + (u32)r * 32u + lane, v, id);
-        h += f & 1u;
-        p += (f >> 1) & 1u;
-        b += (f >> 2) & 1u;
+    constexpr u32 kHead = 1u << 18, kPatch = 1u << 19, kBlock = 1u << 20;
+    u32 info[ITEMS];  // repos delta (18 bits), flags, quad delta << 21; 0: no unit
+    u32 sums = 0;
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const u32 e = e0 + 32u * r;
+        info[r] = 0;
+        if (e < cnt) {
+            const u64 k = sk[2 + e], x = k ^ sk[1 + e];
+            if (!rle || x || (base + e) == 0) {
+                u32 f = kHead;
+                if (DIRECT) {
+                    if (sfc_delta(e) > 254u) f |= kPatch;
+                } else {
+                    const u32 lo = (u32)k, before = lo ^ (u32)x;
+                    const bool block = (x >> 21) != 0, moved = (x >> 18) != 0;
+                    const u32 d = moved ? lo & 0x3ffffu : lo - before;
+                    const u32 quad = ((lo >> 18) & 7u) - (block ? 0u : (before >> 18) & 7u);
+                    f |= d | (quad << 21) | (d > 254u ? kPatch : 0u) | (block ? kBlock : 0u);
+                }
+                info[r] = f;
+                sums += 1u + (f & kPatch ? 1u << 10 : 0u) + (f & kBlock ? 1u << 20 : 0u);
+            }
+        }
     }
-    // Packed three-field exclusive scan: each field <= 4096 per tile, 21 bits apiece.  Lane
-    // 0's exclusive prefix is the count over the earlier warps' elements.
-    const u64 mine = (u64)h | ((u64)p << 21) | ((u64)b << 42);
-    u64 tot;
-    const u64 ex = block_exclusive<kThreads>(mine, 0ull, AddOp{}, scratch, tot);
-    if (tid < 32) {  // the three counts (below 2^31) in one chained scan
-        constexpr u64 kF = (1ull << 21) - 1;
-        const Pair part{(tot & kF) | (((tot >> 21) & kF) << 32), tot >> 42};
-        const Pair before = chain_lookback(static_cast<Status*>(status), tile, part, PairAdd{}, err);
-        if (tid == 0) {
-            const u64 be[3] = {before.lo & 0xffffffffull, before.lo >> 32, before.hi};
-            for (int ch = 0; ch < 3; ++ch) {
-                sbase[ch] = be[ch];
-                if (tile == ntiles - 1) out.counters[ch] = be[ch] + ((tot >> (21 * ch)) & kF);
+    sums = __reduce_add_sync(kFullMask, sums);  // (at most 512 each)
+    if (lane == 0) wtot[w] = sums;
+    __syncthreads();
+    u32 mu = 0, mp = 0, mb = 0;  // the warp's first unit, patch and block in the tile
+#pragma unroll
+    for (int i = 0; i < kW; ++i) {
+        const u32 t = wtot[i];
+        if (i < w) {
+            mu += t & 0x3ffu;
+            mp += (t >> 10) & 0x3ffu;
+            mb += t >> 20;
+        }
+    }
+    if (w == kW - 1) {  // the three counts (below 2^31) in one chained scan
+        const u32 tu = mu + (sums & 0x3ffu), tp = mp + ((sums >> 10) & 0x3ffu), tb = mb + (sums >> 20);
+        const Pair b = chain_lookback(status, tile, Pair{(u64)tu | ((u64)tp << 32), tb}, PairAdd{}, err);
+        if (lane == 0) {
+            sbase[0] = b.lo & 0xffffffffull;
+            sbase[1] = b.lo >> 32;
+            sbase[2] = b.hi;
+            if (tile == gridDim.x - 1) {
+                out.counters[0] = sbase[0] + tu;
+                out.counters[1] = sbase[1] + tp;
+                out.counters[2] = sbase[2] + tb;
             }
         }
     }
     __syncthreads();
 
-    const u64 wex = __shfl_sync(kFullMask, ex, 0);
-    u64 uu = sbase[0] + (wex & ((1ull << 21) - 1));
-    u64 pp = sbase[1] + ((wex >> 21) & ((1ull << 21) - 1));
-    u64 bb = sbase[2] + ((wex >> 42) & ((1ull << 21) - 1));
-    const u32 lt = lanemask_lt();
+    const u64 ubase = sbase[0];
+    u8* const rep_sym = out.rep_sym + ubase;
+    u8* const quad_sym = out.quad_sym + ubase;
+    u32* const unit_pos = out.unit_pos + ubase;
+    u64* const rep_val = out.rep_val ? (u64*)out.rep_val + ubase : nullptr;
+    u64* const patch64 = static_cast<u64*>(out.patches) + sbase[1];
+    u32* const patch32 = static_cast<u32*>(out.patches) + sbase[1];
+    u64* const blk_id = (u64*)out.blk_id + sbase[2];
+    u32* const blk_unit = out.blk_unit + sbase[2];
     u64 mysum = 0;
-    // quad symbols are 1..8 (qd = 0..7): lane v < 8 counts symbol v + 1 from three ballots of
-    // its bits, and keeps the unit of its first occurrence
-    u32 qn = 0, qf = 0xffffffffu;
-    for (int r = 0; r < kItems; ++r) {
-        const u32 e = wfirst + (u32)r * 32u + lane;
-        u64 vi, idi;
-        const u32 f = classify(e, vi, idi);
-        const bool head = f & 1u;
-        const bool patch = head && ((f >> 1) & 1u);
-        const bool nblk = head && ((f >> 2) & 1u);
-        const u32 hm = __ballot_sync(kFullMask, head), pm = __ballot_sync(kFullMask, patch),
-                  bm = __ballot_sync(kFullMask, nblk);
-        const u64 u = uu + __popc(hm & lt);
-        const u32 sym = head ? (patch ? 0u : (u32)vi + 1u) : 0u;
-        const u32 qsym = ((f >> 8) & 0xffu) + 1u;
+    u32 q0 = 0, q1 = 0;  // units of my quad deltas 0..3 and 4..7, one byte each
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const u32 e = e0 + 32u * r, f = info[r];
+        const bool head = f != 0, patch = f & kPatch, block = !DIRECT && (f & kBlock);
+        const u32 hm = __ballot_sync(kFullMask, head), pm = __ballot_sync(kFullMask, patch);
+        const u32 bm = DIRECT ? 0u : __ballot_sync(kFullMask, block);
         if (head) {
-            out.rep_sym[u] = (u8)sym;
-            if (out.rep_val) out.rep_val[u] = vi;
-            if (!DIRECT) out.quad_sym[u] = (u8)qsym;
+            const u32 u = mu + __popc(hm & lt);
+            const u64 val = DIRECT ? sfc_delta(e) : (u64)(f & 0x3ffffu);
+            const u32 sym = patch ? 0u : (u32)val + 1u;
+            rep_sym[u] = (u8)sym;
+            if (rep_val) rep_val[u] = val;
+            if (rle) unit_pos[u] = (u32)(base + e);
             if (patch) {
-                const u64 at = pp + __popc(pm & lt);
-                if (DIRECT) static_cast<u64*>(out.patches)[at] = vi;
-                else static_cast<u32*>(out.patches)[at] = (u32)vi;  // 18-bit codes
-                mysum += vi;
+                const u32 at = mp + __popc(pm & lt);
+                if (DIRECT) patch64[at] = val;
+                else patch32[at] = (u32)val;  // 18-bit codes
+                mysum += val;
             }
-            if (!DIRECT && nblk) {
-                const u64 bi = bb + __popc(bm & lt);
-                out.blk_id[bi] = idi;
-                out.blk_unit[bi] = (u32)u;
+            atomicAdd(&hrep[sym], 1u);
+            if (u < *(volatile u32*)&frep[sym]) atomicMin(&frep[sym], u);
+            if (!DIRECT) {
+                const u32 qd = f >> 21;
+                quad_sym[u] = (u8)(qd + 1u);
+                const u32 one = 1u << (8u * (qd & 3u));
+                if (qd < 4u) q0 += one;
+                else q1 += one;
+                if (u < *(volatile u32*)&fquad[qd]) atomicMin(&fquad[qd], u);
+                if (block) {
+                    const u32 at = mb + __popc(bm & lt);
+                    u64 id;
+                    u32 quad, sfc;
+                    block_key_fields(sk[2 + e], bkp, id, quad, sfc);
+                    blk_id[at] = id;
+                    blk_unit[at] = (u32)ubase + u;
+                }
             }
-            if (rle) out.unit_pos[u] = (u32)(base + e);
         }
-        hist_add_masked(mrep[w], hrep, frep, head, sym, (u32)u);
-        if (!DIRECT) {
-            const u32 qb = qsym - 1u;
-            const u32 b0 = __ballot_sync(kFullMask, head && (qb & 1u)), b1 = __ballot_sync(kFullMask, head && (qb & 2u)),
-                      b2 = __ballot_sync(kFullMask, head && (qb & 4u));
-            const u32 mv = hm & ((lane & 1u) ? b0 : ~b0) & ((lane & 2u) ? b1 : ~b1) & ((lane & 4u) ? b2 : ~b2);
-            if (lane < 8u && mv) {
-                qn += (u32)__popc(mv);
-                if (qf == 0xffffffffu) qf = (u32)(uu + (u32)__popc(hm & ((1u << (__ffs(mv) - 1)) - 1u)));
-            }
+        mu += __popc(hm);
+        mp += __popc(pm);
+        mb += __popc(bm);
+    }
+    if (!DIRECT) {
+        const u32 t[4] = {__reduce_add_sync(kFullMask, q0 & 0xff00ffu), __reduce_add_sync(kFullMask, (q0 >> 8) & 0xff00ffu),
+                          __reduce_add_sync(kFullMask, q1 & 0xff00ffu), __reduce_add_sync(kFullMask, (q1 >> 8) & 0xff00ffu)};
+        if (lane < 8u) {  // delta v: byte v % 4 of its word, the low or high half of t
+            const u32 x = lane & 4u ? (lane & 1u ? t[3] : t[2]) : (lane & 1u ? t[1] : t[0]);
+            const u32 c = lane & 2u ? x >> 16 : x & 0xffffu;
+            if (c) atomicAdd(&hquad[lane], c);
         }
-        uu += __popc(hm);
-        pp += __popc(pm);
-        bb += __popc(bm);
     }
-    if (!DIRECT && lane < 8u && qn) {
-        atomicAdd(&hquad[lane + 1], qn);
-        atomicMin(&fquad[lane + 1], qf);
-    }
-    for (int d = 16; d > 0; d >>= 1) mysum += __shfl_xor_sync(kFullMask, mysum, d);
-    if (lane_id() == 0) psum[tid >> 5] = mysum;
+    mysum = warp_sum(mysum);
+    if (lane == 0 && mysum) atomicAdd(&psum, mysum);
     __syncthreads();
-    if (tid == 0) {
-        u64 s = 0;
-        for (int w = 0; w < kThreads / 32; ++w) s += psum[w];
-        if (s) atomicAdd(&out.counters[3], s);
-    }
-    if (hrep[tid]) {
-        atomicAdd(&out.hist_rep[tid], (u64)hrep[tid]);
-        atomicMin(&out.first_rep[tid], frep[tid]);
-    }
-    if (!DIRECT && tid < 16 && hquad[tid]) {
-        atomicAdd(&out.hist_quad[tid], (u64)hquad[tid]);
-        atomicMin(&out.first_quad[tid], fquad[tid]);
-    }
+    if (tid == 0 && psum) atomicAdd(&out.counters[3], psum);
+    // (first units come down with the tiles, nearly in order: read before each minimum)
+    auto flush = [&](unsigned long long* hist, u32* first, u32 c, u32 f) {
+        atomicAdd(hist, (unsigned long long)c);
+        f += (u32)ubase;
+        if (f < __ldcg(first)) atomicMin(first, f);
+    };
+    if (hrep[tid]) flush(out.hist_rep + tid, out.first_rep + tid, hrep[tid], frep[tid]);
+    if (!DIRECT && tid < 8 && hquad[tid]) flush(out.hist_quad + tid + 1, out.first_quad + tid + 1, hquad[tid], fquad[tid]);
 }
 
 // -rle: count of each unit = distance to the next unit's first point, and the counts' histogram with
@@ -821,17 +802,23 @@ inline int persistent_grid(u64 n) {
 
 }  // namespace
 
+template <bool DIRECT>
+static void launch_units(const unsigned long long* keys, uint64_t n, int rle, const BlockKeyParams& bkp,
+                         const DirectKeyParams& dkp, UnitOutputs out, ScanStatus status, uint32_t* tile_counter,
+                         uint32_t* err, cudaStream_t st) {
+    const unsigned tiles = (unsigned)((n + unit_tile(n) - 1) / unit_tile(n));
+    if (!tiles) return;
+    auto k = unit_tile(n) == kUnitTile ? units_kernel<DIRECT, kUnitTile / kThreads> : units_kernel<DIRECT, kUnitTileSmall / kThreads>;
+    k<<<tiles, kThreads, 0, st>>>(reinterpret_cast<const u64*>(keys), n, rle, bkp, dkp, out, static_cast<Status*>(status),
+                                  tile_counter, err);
+}
 void launch_units_block(const unsigned long long* keys, uint64_t n, int rle, BlockKeyParams kp, UnitOutputs out,
                         ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
-    if (!tiles) return;
-    units_kernel<false><<<tiles, kThreads, 0, st>>>(keys, n, rle, kp, DirectKeyParams{}, out, status, tile_counter, err);
+    launch_units<false>(keys, n, rle, kp, DirectKeyParams{}, out, status, tile_counter, err, st);
 }
 void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, DirectKeyParams kp, UnitOutputs out,
                          ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
-    if (!tiles) return;
-    units_kernel<true><<<tiles, kThreads, 0, st>>>(keys, n, rle, BlockKeyParams{}, kp, out, status, tile_counter, err);
+    launch_units<true>(keys, n, rle, BlockKeyParams{}, kp, out, status, tile_counter, err, st);
 }
 void launch_count_stats(const uint32_t* unit_pos, uint64_t units, const unsigned long long* units_dev, uint64_t n,
                         int32_t* counts, CountStats cs, cudaStream_t st) {

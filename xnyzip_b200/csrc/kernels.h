@@ -144,7 +144,9 @@ void launch_sort_small(const unsigned long long* kin, unsigned long long* kout, 
                        uint64_t n, int passes, cudaStream_t st);
 
 // --- compress segments + encoders -------------------------------------------------------
-constexpr int kUnitTile = 4096;
+constexpr int kUnitTile = 4096, kUnitTileSmall = 1024;
+constexpr uint64_t kUnitSmall = 1ull << 19;
+inline uint64_t unit_tile(uint64_t n) { return n < kUnitSmall ? kUnitTileSmall : kUnitTile; }
 void launch_units_block(const unsigned long long* keys, uint64_t n, int rle, BlockKeyParams kp, UnitOutputs out,
                         ScanStatus status, uint32_t* tile_counter, uint32_t* err, cudaStream_t st);
 void launch_units_direct(const unsigned long long* keys, uint64_t n, int rle, DirectKeyParams kp, UnitOutputs out,
