@@ -1,4 +1,4 @@
-// zstd frames decoded on the GPU, one frame per warp (zstd_dec.cuh), for callers that hold
+// zstd frames decoded on the GPU, one frame per block (zstd_dec.cuh), for callers that hold
 // many container frames in device memory: no host round trip.
 #include "kernels.h"
 #include "zstd_dec.cuh"
@@ -8,27 +8,37 @@ namespace dev {
 
 namespace {
 
-// One frame per warp: the lanes decode it together (zd::WarpTeam).
-__global__ void __launch_bounds__(128) zstd_frames_kernel(const uint8_t* const* src, const uint64_t* src_len,
-                                                          uint8_t* const* dst, const uint64_t* cap, long long* out_len,
-                                                          zd::Workspace* ws, uint64_t count) {
-    const uint64_t f = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (f >= count) return;  // the same for every lane of the warp
-    const zd::WarpTeam team{(int)(threadIdx.x & 31)};
-    const long long r = zd::decode_frame(src[f], src_len[f], dst[f], cap[f], ws[f], team);
+struct Workspace : zd::Tables {
+    zd::u8* lit;
+};
+
+// One frame per block of 128 threads (zd::BlockTeam), the tables in shared memory; registers for six
+// blocks per SM, so that 768 frames run at once.  Bound by latency: the frames with the most sequences (6170
+// in 28 KB) are last, for whom the states' chain takes 160 clocks a sequence and the copies, beside it in
+// other warps, about as much.  One warp per frame, whose lanes walked the sequences together, byte loads for
+// the bits, tables in global memory and one copy after another took 6.9 ms for 768 frames of 27 KB (81 KB of
+// content); this takes 1.4 ms.
+__global__ void __launch_bounds__(zd::BlockTeam::size, 6) zstd_frames_kernel(const uint8_t* const* src, const uint64_t* src_len,
+                                                                          uint8_t* const* dst, const uint64_t* cap,
+                                                                          long long* out_len, uint8_t* literals) {
+    __shared__ Workspace ws;
+    __shared__ int slot;
+    const uint64_t f = blockIdx.x;
+    const zd::BlockTeam team{(int)threadIdx.x, &slot};
+    if (team.rank == 0) ws.lit = literals + f * (zd::kMaxBlock + 32);
+    __syncthreads();
+    const long long r = zd::decode_frame(src[f], src_len[f], dst[f], cap[f], ws, team);
     if (team.rank == 0) out_len[f] = r;
 }
 
 }  // namespace
 
-size_t zstd_workspace_bytes() { return sizeof(zd::Workspace); }
+size_t zstd_workspace_bytes() { return zd::kMaxBlock + 32; }
 
 void launch_zstd_frames(const uint8_t* const* src, const uint64_t* src_len, uint8_t* const* dst, const uint64_t* cap,
                         long long* out_len, void* workspace, uint64_t count, cudaStream_t st) {
     if (!count) return;
-    const unsigned blocks = (unsigned)((count + 3) / 4);  // four frames (warps) per block
-    zstd_frames_kernel<<<blocks, 128, 0, st>>>(src, src_len, dst, cap, out_len,
-                                              static_cast<zd::Workspace*>(workspace), count);
+    zstd_frames_kernel<<<(unsigned)count, zd::BlockTeam::size, 0, st>>>(src, src_len, dst, cap, out_len, static_cast<uint8_t*>(workspace));
 }
 
 }  // namespace dev
