@@ -74,31 +74,6 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
-// Segmented inclusive sums over one round of 32 consecutive elements (lane order): lane i
-// gets the sum of v over [h, i] with h the last head lane at or before i, or carry plus the
-// sum over [0, i] when there is none (SegOp's semantics; carry = the running segment sum).
-template <typename T>
-__device__ __forceinline__ T warp_seg_incl(u32 heads, T v, T carry) {
-    const T incl = warp_incl_add(v);
-    const u32 le = heads & (lanemask_lt() | (1u << lane_id()));
-    const T before = __shfl_sync(kFullMask, incl - v, le ? 31 - __clz(le) : 0);
-    return le ? incl - before : carry + incl;
-}
-
-// Exclusive prefix over the block's warps of per-warp aggregates held in v[0..WARPS); the
-// tile total goes to v[WARPS].  One thread.
-template <int WARPS, typename T, typename Op>
-__device__ __forceinline__ void warps_exclusive(T* v, T identity, Op op) {
-    T run = identity;
-    for (int i = 0; i < WARPS; ++i) {
-        const T x = v[i];
-        v[i] = run;
-        run = op(run, x);
-    }
-    v[WARPS] = run;
-}
-
-
 // Block-wide exclusive scan (THREADS a multiple of 32, <= 1024).  `total` receives the
 // block aggregate.  `scratch` holds THREADS/32 + 1 elements of shared memory.
 template <int THREADS, typename T, typename Op>
@@ -415,19 +390,6 @@ __device__ __forceinline__ void hilbert_xyz(const u8* tab, u64 code, int top, u3
     }
 }
 
-// hilbert_xyz for top = 5 and a code below 2^18 (the 6 levels of one 64^3 quadrant).
-__device__ __forceinline__ void hilbert_xyz6(const u8* tab, u32 code, u32 state, u32& x, u32& y, u32& z) {
-    x = y = z = 0;
-#pragma unroll
-    for (int l = 5; l >= 0; --l) {
-        const u32 e = tab[state * 8 + ((code >> (3 * l)) & 7u)];
-        x |= (e & 1u) << l;
-        y |= ((e >> 1) & 1u) << l;
-        z |= ((e >> 2) & 1u) << l;
-        state = e >> 3;
-    }
-}
-
 // ------------------------------------------------------------- bit writers --------------
 // Stream words are 32-bit; the output buffer must be zeroed and 4-byte aligned.
 // MSB-first streams: stream bit p is bit (7 - p%8) of byte p/8; a 32-bit word k then holds
@@ -454,24 +416,6 @@ __device__ __forceinline__ void warp_or_word(u32* words, u64 word, u32 bits, boo
     int na = __shfl_down_sync(kFullMask, act, 1);
     bool last = (lane == 31) || !na || nw != word;
     if (active && last && v) atomicOr(&words[word], v);
-}
-
-// Writes `nbits` (<= 64) bits of `val` (its low bits, most significant first) at stream
-// position `pos` of an MSB-first stream.
-__device__ __forceinline__ void warp_write_msb(u32* words, u64 pos, u64 val, u32 nbits) {
-    const bool act = nbits != 0;
-    const u64 k0 = pos >> 5;
-    const u32 o = (u32)(pos & 31u);
-    // 96-bit window W[k0] W[k0+1] W[k0+2]; the value occupies [o, o + nbits).
-    unsigned __int128 chunk = 0;
-    if (act) {
-        const u64 v = nbits == 64 ? val : (val & ((1ull << nbits) - 1));
-        chunk = (unsigned __int128)v << (96u - o - nbits);
-    }
-    const u32 w0 = (u32)(chunk >> 64), w1 = (u32)(chunk >> 32), w2 = (u32)chunk;
-    warp_or_word(words, k0, __byte_perm(w0, 0, 0x0123), act);
-    if (__any_sync(kFullMask, act && w1 != 0u)) warp_or_word(words, k0 + 1, __byte_perm(w1, 0, 0x0123), act);
-    if (__any_sync(kFullMask, act && w2 != 0u)) warp_or_word(words, k0 + 2, __byte_perm(w2, 0, 0x0123), act);
 }
 
 // One thread's run of consecutive codes of an MSB-first stream, from stream bit `pos` on
@@ -608,43 +552,6 @@ __device__ __forceinline__ void warp_write_lsb(u32* words, u64 pos, u64 val, u32
     warp_or_word(words, k0, w0, act);
     if (__any_sync(kFullMask, act && w1 != 0u)) warp_or_word(words, k0 + 1, w1, act);
     if (__any_sync(kFullMask, act && w2 != 0u)) warp_or_word(words, k0 + 2, w2, act);
-}
-
-// Single-lane writer of `count` one-bits at `pos` of an LSB-first stream (long unary runs
-// of the Golomb-Rice code).  Whole words inside the run belong to this run alone.
-__device__ __forceinline__ void write_ones_lsb(u32* words, u64 pos, u64 count) {
-    while (count > 0) {
-        const u64 k = pos >> 5;
-        const u32 o = (u32)(pos & 31u);
-        const u32 take = (u32)min((u64)(32u - o), count);
-        const u32 mask = (take == 32u ? 0xffffffffu : ((1u << take) - 1u)) << o;
-        if (mask == 0xffffffffu)
-            words[k] = 0xffffffffu;
-        else
-            atomicOr(&words[k], mask);
-        pos += take;
-        count -= take;
-    }
-}
-
-// ------------------------------------------------------------- bit readers --------------
-// Streams are padded with >= 16 zero bytes so these may read past the last word.
-__device__ __forceinline__ u32 load_be_word(const u32* w, u64 k) { return __byte_perm(__ldg(&w[k]), 0, 0x0123); }
-
-// 32 bits of an MSB-first stream starting at bit `pos`, first bit in bit 31.
-__device__ __forceinline__ u32 peek_msb32(const u32* w, u64 pos) {
-    const u64 k = pos >> 5;
-    const u32 o = (u32)(pos & 31u);
-    const u32 a = load_be_word(w, k), b = load_be_word(w, k + 1);
-    return o ? ((a << o) | (b >> (32u - o))) : a;
-}
-// 64 bits of an LSB-first stream starting at bit `pos`, first bit in bit 0.
-__device__ __forceinline__ u64 peek_lsb64(const u32* w, u64 pos) {
-    const u64 k = pos >> 5;
-    const u32 o = (u32)(pos & 31u);
-    const u64 a = __ldg(&w[k]), b = __ldg(&w[k + 1]), c = __ldg(&w[k + 2]);
-    const unsigned __int128 x = (unsigned __int128)a | ((unsigned __int128)b << 32) | ((unsigned __int128)c << 64);
-    return (u64)(x >> o);
 }
 
 __device__ __forceinline__ u32 bitlen64(u64 v) { return v ? 64u - (u32)__clzll((long long)v) : 0u; }
