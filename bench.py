@@ -919,7 +919,7 @@ def zstd_measure(ctx, stream, dev, points=4_000_000, piece=1 << 16, count=6360, 
             "host_libzstd_GB_s": {"1": round(cpu1 / 1e9, 3), str(threads): round(cpun / 1e9, 3)},
             "workload": f"pre-zstd container of a {points}-point terrain cloud (TO 0.01, Hilbert, -rle) in "
                         f"{piece}-byte pieces, each a libzstd level-3 frame, repeated to {count} frames; "
-                        "one warp per frame"}
+                        "one block of 128 threads per frame"}
 
 
 # ---------------------------------------------------------------------- CPU baselines ---
