@@ -1363,44 +1363,68 @@ __global__ void decode_sequential_kernel(Args a) {
 }
 
 // A Huffman stream whose codewords all have one length `len` (<= kMaxRootBits): symbol i is
-// bits [i len, (i + 1) len) of the stream, one primary-table lookup each, so the stream needs
-// neither entry tables nor look-back.  Thread g decodes symbols 4g .. 4g + 3 from one 64-bit
-// window (4 len <= 44 bits) and stores u8 symbols four at a time.  A chunk that is no
-// codeword sets kErrBadStream, as the chained decoder does.
+// bits [i len, (i + 1) len) of the stream, one table lookup each, so the stream needs neither entry
+// tables nor look-back.  A thread decodes 16 symbols, from one 64-bit window (SHORT: len <= 4) or from
+// one per four symbols, through a table of values in shared memory, and stores them in 16-byte pieces.
+// Bound by instructions: four symbols per thread through the global table took 64 per symbol; the three
+// Huffman streams of 64M terrain points (two of them of one length) took 427 us, with this 262.  A chunk
+// that is no codeword sets kErrBadStream, as the chained decoder does.
+template <bool SHORT, int WIDTH>
 __global__ void __launch_bounds__(256) decode_fixed_kernel(const u32* __restrict__ words, u32 base, u64 nwords,
                                                            int len, const u32* __restrict__ root,
-                                                           const u64* __restrict__ symvals, u64 nsym, int width,
-                                                           void* out, bool packed_ok, u32* err) {
-    const u64 groups = (nsym + 3) / 4;
-    auto wbe = [&](u64 k) -> u64 { return k < nwords ? (u64)__byte_perm(__ldg(words + k), 0, 0x0123) : 0ull; };
+                                                           const u64* __restrict__ symvals, u64 nsym,
+                                                           void* out, bool aligned, u32* err) {
+    __shared__ uint2 tab[1 << kMaxRootBits];  // value, and whether no codeword
+    for (u32 i = threadIdx.x; i < 1u << len; i += blockDim.x) {
+        const u32 e = __ldg(root + i), v = e & 0xffffffu;
+        tab[i] = make_uint2(symvals ? (u32)__ldg(symvals + v) : v, (e >> 24) != (u32)len);
+    }
+    __syncthreads();
+    constexpr int kPer = SHORT ? 16 : 4;
+    auto wbe = [&](u64 k) -> u32 {
+        const u32 w = __byte_perm(__ldg(words + (k < nwords ? k : nwords - 1)), 0, 0x0123);
+        return k < nwords ? w : 0u;
+    };
+    const u64 groups = (nsym + 15) / 16;
     for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += (u64)gridDim.x * blockDim.x) {
-        const u64 i0 = 4 * g;
-        const int cnt = (int)min((u64)4, nsym - i0);
-        const u64 q = (u64)base + i0 * (u64)len;
-        const u64 k = q >> 5;
-        const u32 o = (u32)(q & 31u);
-        u64 win = ((wbe(k) << 32) | wbe(k + 1)) << o;
-        if (o) win |= wbe(k + 2) >> (32u - o);
-        bool bad = false;
-        u32 packed = 0;
-        for (int j = 0; j < cnt; ++j) {
-            const u32 code = (u32)(win >> (64 - len));
-            win <<= len;
-            const u32 e = __ldg(root + code);
-            if ((e >> 24) != (u32)len) bad = true;
-            const u64 val = symvals ? __ldg(symvals + (e & 0xffffffu)) : (u64)(e & 0xffffffu);
-            if (width == 1) {
-                packed |= ((u32)val & 0xffu) << (8 * j);
-            } else {
-                reinterpret_cast<u32*>(out)[i0 + j] = (u32)val;
+        const u32 cnt = (u32)min((u64)16, nsym - 16 * g);
+        u32 v[16], bad = 0;
+#pragma unroll
+        for (int p = 0; p < 16; p += kPer) {
+            const u64 q = (u64)base + (16 * g + p) * (u64)len, k = q >> 5;
+            const u32 o = (u32)q & 31u, w0 = wbe(k), w1 = wbe(k + 1), w2 = wbe(k + 2);
+            u32 hi = __funnelshift_l(w1, w0, o), lo = __funnelshift_l(w2, w1, o);
+#pragma unroll
+            for (int j = p; j < p + kPer; ++j) {
+                const uint2 e = tab[hi >> (32 - len)];
+                hi = __funnelshift_l(lo, hi, len);
+                lo <<= len;
+                v[j] = e.x;
+                bad |= (u32)j < cnt ? e.y : 0u;
             }
         }
-        if (width == 1) {
-            u8* o8 = reinterpret_cast<u8*>(out) + i0;
-            if (cnt == 4 && packed_ok) {
-                *reinterpret_cast<u32*>(o8) = packed;
+        if (WIDTH == 1) {
+            u32 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                w[j] = __byte_perm(__byte_perm(v[4 * j], v[4 * j + 1], 0x0040), __byte_perm(v[4 * j + 2], v[4 * j + 3], 0x0040), 0x5410);
+            u8* o8 = static_cast<u8*>(out) + 16 * g;
+            if (cnt == 16u && aligned) {
+                *reinterpret_cast<uint4*>(o8) = make_uint4(w[0], w[1], w[2], w[3]);
             } else {
-                for (int j = 0; j < cnt; ++j) o8[j] = (u8)(packed >> (8 * j));
+#pragma unroll
+                for (u32 j = 0; j < 16; ++j)
+                    if (j < cnt) o8[j] = (u8)v[j];
+            }
+        } else {
+            u32* o32 = static_cast<u32*>(out) + 16 * g;
+            if (cnt == 16u && aligned) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(o32 + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            } else {
+#pragma unroll
+                for (u32 j = 0; j < 16; ++j)
+                    if (j < cnt) o32[j] = v[j];
             }
         }
         if (bad) atomicOr(err, kErrBadStream);
@@ -1550,11 +1574,12 @@ void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t tot
         return;
     }
     const u64 nwords = (base_bits + total_bits + 31) / 32;
-    u64 blocks = (nsym / 4 + 256) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    const bool packed_ok = (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
-    decode_fixed_kernel<<<(unsigned)blocks, 256, 0, st>>>(words, (u32)base_bits, nwords, len, t.root, t.symvals, nsym,
-                                                          out_width, out, packed_ok, err);
+    const u64 threads = (nsym + 15) / 16, want = (threads + 255) / 256;
+    const unsigned blocks = (unsigned)(want < 148 * 8 ? want : 148 * 8);
+    const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    auto k = out_width == 1 ? (len <= 4 ? decode_fixed_kernel<true, 1> : decode_fixed_kernel<false, 1>)
+                            : (len <= 4 ? decode_fixed_kernel<true, 4> : decode_fixed_kernel<false, 4>);
+    k<<<blocks, 256, 0, st>>>(words, (u32)base_bits, nwords, len, t.root, t.symvals, nsym, out, aligned, err);
 }
 
 void launch_decode_sequential(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits,
