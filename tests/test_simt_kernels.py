@@ -1,0 +1,45 @@
+"""The library on the CPU (simt_host.py): its kernels with the warps of a block, and the lanes of a
+warp, taking their turns in either order between barriers, against the oracle."""
+import pytest
+
+import simt_host
+
+ORDERS = [0, 1, 2, 3]
+
+
+@pytest.mark.parametrize("order", ORDERS)
+def test_containers_in_either_order(oracle, order):
+    """One-block and chained sorts, block and direct mode, both curves and containers."""
+    simt_host.run(f"""
+from oracle import Oracle
+o = Oracle()
+simt.simt_order({order})
+ctx = X.Context(0)
+for n in (40, 1013, 9000):
+    x = np.random.default_rng(n).uniform(0, 30, (n, 3)).astype(np.float32)
+    for q, name, hil, rle, thr in ((1, "to", 1, 1, 0), (0, "cube", 0, 0, 0), (0, "cube", 1, 0, 1024)):
+        raw = ctx.compress(x, q, 0.05, hil, rle, thr, use_zstd=False)
+        no_fault()
+        assert raw == o.compress(x, name, 0.05, hil, rle, thr, zstd=False)
+        got = ctx.decompress(raw, q, 0.05, rle, is_zstd=False)
+        no_fault()
+        assert got.tobytes() == o.decompress(raw, name, 0.05, rle, zstd=False).tobytes()
+""")
+
+
+@pytest.mark.parametrize("order", ORDERS)
+@pytest.mark.parametrize("n", [30_000, 60_000, 200_000])
+def test_blocks_that_decode_again(oracle, order, n):
+    """Runs of the codeword 11 of the code 0, 10, 11, some thousand long: a block that starts inside
+    one reads from the wrong bit as consistently as from the right one, assumes a wrong entry, and
+    decodes again once the block before it has told."""
+    simt_host.run(f"""
+from oracle import Oracle
+from test_gpu_stream_decode import container
+simt.simt_order({order})
+sym = np.where(np.random.default_rng({n}).random({n}) < 1 / 3000, 1, 3)
+raw = container(sym, {{1: 1, 2: 2, 3: 2}})
+got = X.Context(0).decompress(raw, 0, 0.05, 0, is_zstd=False)
+no_fault()
+assert got.tobytes() == Oracle().decompress(raw, "cube", 0.05, 0, zstd=False).tobytes()
+""")

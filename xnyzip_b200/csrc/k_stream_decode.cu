@@ -1078,7 +1078,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     constexpr int TT = kSyncThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ u32 slot;
-    __shared__ u64 s_entry, s_first, s_wsum[TT / 32];
+    __shared__ u64 s_assumed, s_entry, s_first, s_wsum[TT / 32];
     u64* sx = reinterpret_cast<u64*>(smem_raw);
     u32* mlen = reinterpret_cast<u32*>(sx + TT);
     u32* msym = mlen + (KIND == kCodeHuffman ? (1 << a.mb) : 0);
@@ -1179,9 +1179,9 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     };
     sum_counts();
     const int last_t = (int)min((long long)TT - 1, (long long)a.nsub - 1 - ((long long)tile * (TT - G) - G));
-    if (t == G) s_entry = entry;
+    if (t == G) s_assumed = entry;
     __syncthreads();
-    const u64 assumed = s_entry;
+    const u64 assumed = s_assumed;  // (read by slower warps while warp 0 already writes s_entry)
 
     // first bit of this block's own subsequences and of the next block's
     const u64 tile_at = (u64)tile * (u64)(TT - G) * (u64)S, next_at = tile_at + (u64)(TT - G) * (u64)S;
