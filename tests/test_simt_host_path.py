@@ -1,0 +1,63 @@
+"""The host path of the library on the CPU (simt_host.py): what a failed call leaves behind, with
+streams that run their work as late as they may."""
+import pytest
+
+import simt_host
+
+PARTS = """
+import struct
+from oracle import Oracle
+o = Oracle()
+
+def streams(raw, rle):
+    '''Container -> (head, [[meta, data], ..], tail).'''
+    units, params = struct.unpack_from("<QQ", raw, 0)
+    at = 16 + 4 * params + 14
+    head, out = raw[:at], []
+    for _ in range((2 if raw[at - 1] else 6) + rle):
+        dl, ml = struct.unpack_from("<QQ", raw, at)
+        out.append([raw[at + 16:at + 16 + ml], raw[at + 16 + ml:at + 16 + ml + dl]])
+        at += 16 + ml + dl
+    assert len(raw) == at + 12
+    return head, out, raw[at:]
+
+def joined(head, parts, tail):
+    return head + b"".join(struct.pack("<QQ", len(d), len(m)) + m + d for m, d in parts) + tail
+"""
+
+
+@pytest.mark.parametrize("damage", ["counts too short", "quads too short", "no quad codes", "no count codes"])
+def test_failed_decompress_leaves_no_work_behind(oracle, damage):
+    """A stream that the host finds damaged after others have been queued: nothing may read the caller's
+    container, or write the context's workspace, once the call has returned."""
+    simt_host.run(PARTS + f"""
+damage = {damage!r}
+ctx = X.Context(0)
+rng = np.random.default_rng(3)
+x = rng.uniform(0, 400, (6000, 3)).astype(np.float32)
+x = np.concatenate([x, x[:3000]])  # counts 1 and 2: one bit each
+raw = o.compress(x, "to", 0.05, 1, 1, 0, zstd=False)
+head, s, tail = streams(raw, 1)
+which = 6 if "count" in damage else 5
+if "short" in damage:
+    if which == 5:  # eight codes of three bits
+        s[5][0] = struct.pack(">I", 8) + b"".join(struct.pack(">BBI", i + 1, 3, i) for i in range(8))
+    s[which][1] = s[which][1][:100]
+else:
+    s[which] = [struct.pack(">I", 0), b""]
+bad = joined(head, s, tail)
+p = device(bad)
+try:
+    ctx.decompress_device(p, len(bad), 1, 0.05, 1)
+    raise SystemExit("accepted")
+except X.XnyzError as e:
+    assert e.status == 2, e
+assert simt.simt_pending() == 0
+simt.simt_device_free(p)
+y = rng.uniform(0, 300, (5000, 3)).astype(np.float32)
+for _ in range(2):
+    raw = ctx.compress(y, 1, 0.05, 1, 1, use_zstd=False)
+    assert raw == o.compress(y, "to", 0.05, 1, 1, zstd=False)
+    assert ctx.decompress(raw, 1, 0.05, 1, is_zstd=False).tobytes() == o.decompress(raw, "to", 0.05, 1, zstd=False).tobytes()
+    no_fault()
+""")

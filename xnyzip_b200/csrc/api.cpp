@@ -1587,27 +1587,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     place(ht_cnt, to_cnt);
     if (tab_bytes) CUDA_TRY(cudaMemcpyAsync(at<uint8_t>(c, tab0), c->h_tab, tab_bytes, cudaMemcpyHostToDevice, st));
 
-    hd1.end();
-    HostPhase hd2(c, "d2_launch");
-    // The entropy-coded streams decode on the side streams while the block streams are
-    // unpacked and scanned on the context's stream.
-    TRY(fork_sides(c));
-    // ---- block streams: bit-unpack + prefix sums ----
-    // nx uses the size_t conversion of the stored int range (block_quantizer.hpp:163)
-    const uint64_t blocks_x = static_cast<uint64_t>(static_cast<int64_t>(h.rx)) / 128 + 1,
-                   blocks_y = static_cast<uint64_t>(static_cast<int64_t>(h.ry)) / 128 + 1;
-    const BlockCorners corners{at<uint32_t>(c, o_cx), at<uint32_t>(c, o_cy), at<uint32_t>(c, o_cz)};
-    auto launch_blocks = [&](bool compact) {
-        uint64_t b0, b1;
-        const uint32_t* w0 = words_of(h.streams[0], b0);
-        const uint32_t* w1 = words_of(h.streams[1], b1);
-        Prof pr(c, "block_streams", 1, (w_blk + w_cnt) * NB / 8.0 + 12.0 * NB + 1.0 * std::min(NB, U));
-        launch_block_streams(w0, b0, w_blk, w1, b1, w_cnt, NB, U, blocks_x, blocks_y, compact, corners,
-                             at<uint8_t>(c, o_isst), lb_state(c, lb_scan), SMALL_FIELD(c, tile_counters[20]),
-                             SMALL_FIELD(c, count_total), SMALL_FIELD(c, empty_blocks), SMALL_FIELD(c, err), st);
-    };
-    if (!h.direct && NB) launch_blocks(false);
-
     // ---- entropy-coded streams ----
     std::vector<DecodeJob> jobs;
     auto huff_job = [&](const StreamRef& s, const ParsedMeta& pm, const HuffTables& t, const TabOff& o, int width,
@@ -1634,6 +1613,8 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         bool same = !pm.codes.empty();
         for (const auto& ce : pm.codes) same = same && ce.len == t.max_len;
         if (same && t.max_len == t.root_bits) j.fixed_len = t.max_len;
+        if (!j.fill && j.nsym * static_cast<uint64_t>(j.fixed_len) > j.total_bits)
+            return fail(XNYZ_ERR_BAD_STREAM, "Huffman stream shorter than its symbols");
         int g = 0;
         for (const auto& ce : pm.codes) g = std::gcd(g, static_cast<int>(ce.len));
         j.tables = g > 1;
@@ -1674,6 +1655,27 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             TRY(huff_job(*s_cnt, pm_cnt, ht_cnt, to_cnt, 4, at<int32_t>(c, o_counts), 3));
         }
     }
+    hd1.end();
+    HostPhase hd2(c, "d2_launch");
+    // The entropy-coded streams decode on the side streams while the block streams are
+    // unpacked and scanned on the context's stream.
+    TRY(fork_sides(c));
+    // ---- block streams: bit-unpack + prefix sums ----
+    // nx uses the size_t conversion of the stored int range (block_quantizer.hpp:163)
+    const uint64_t blocks_x = static_cast<uint64_t>(static_cast<int64_t>(h.rx)) / 128 + 1,
+                   blocks_y = static_cast<uint64_t>(static_cast<int64_t>(h.ry)) / 128 + 1;
+    const BlockCorners corners{at<uint32_t>(c, o_cx), at<uint32_t>(c, o_cy), at<uint32_t>(c, o_cz)};
+    auto launch_blocks = [&](bool compact) {
+        uint64_t b0, b1;
+        const uint32_t* w0 = words_of(h.streams[0], b0);
+        const uint32_t* w1 = words_of(h.streams[1], b1);
+        Prof pr(c, "block_streams", 1, (w_blk + w_cnt) * NB / 8.0 + 12.0 * NB + 1.0 * std::min(NB, U));
+        launch_block_streams(w0, b0, w_blk, w1, b1, w_cnt, NB, U, blocks_x, blocks_y, compact, corners,
+                             at<uint8_t>(c, o_isst), lb_state(c, lb_scan), SMALL_FIELD(c, tile_counters[20]),
+                             SMALL_FIELD(c, count_total), SMALL_FIELD(c, empty_blocks), SMALL_FIELD(c, err), st);
+    };
+    if (!h.direct && NB) launch_blocks(false);
+
     if (h.ext && U) {
         // block-coded stream: copy its parts to aligned buffers, then decode every block
         cudaStream_t xs = side(c, 0);
@@ -1719,8 +1721,6 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         Prof pr(c, j.kind == kCodeGolombRice ? "decode_golomb_rice" : (j.kind == kCodeHuffman ? "decode_huffman" : "decode_exp_golomb"),
                 1, j.total_bits / 8.0 + static_cast<double>(j.nsym) * j.width, js);
         if (j.fixed_len) {
-            if (j.nsym * static_cast<uint64_t>(j.fixed_len) > j.total_bits)
-                return fail(XNYZ_ERR_BAD_STREAM, "Huffman stream shorter than its symbols");
             launch_decode_fixed(j.words, j.base_bits, j.total_bits, j.table, j.fixed_len, j.nsym, j.width, j.out,
                                 SMALL_FIELD(c, err), js);
             continue;
@@ -1857,8 +1857,8 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     return XNYZ_OK;
 }
 
-xnyz_status decompress_run(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, const Header& h, int quantizer, float l2,
-                           bool rle, size_t reserved, float** d_out, uint64_t* n_out, int32_t** cells_out = nullptr) {
+xnyz_status decompress_attempts(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, const Header& h, int quantizer,
+                                float l2, bool rle, size_t reserved, float** d_out, uint64_t* n_out, int32_t** cells_out) {
     // The container may live in the arena's reserved prefix; growing keeps that prefix.
     for (int attempt = 0; attempt < 3; ++attempt) {
         xnyz_status s = decompress_core(c, d_cont, len, h, quantizer, l2, rle, reserved, d_out, n_out, cells_out);
@@ -1881,6 +1881,18 @@ xnyz_status decompress_run(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, con
         }
     }
     return fail(XNYZ_ERR_OOM, "workspace growth did not converge");
+}
+
+// A call that fails waits for what it has queued, on the side streams too: it reads the caller's container
+// and writes the workspace of the next call.
+xnyz_status decompress_run(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, const Header& h, int quantizer, float l2,
+                           bool rle, size_t reserved, float** d_out, uint64_t* n_out, int32_t** cells_out = nullptr) {
+    const xnyz_status s = decompress_attempts(c, d_cont, len, h, quantizer, l2, rle, reserved, d_out, n_out, cells_out);
+    if (s != XNYZ_OK) {
+        for (cudaStream_t side : c->side) cudaStreamSynchronize(side);
+        cudaStreamSynchronize(c->stream);
+    }
+    return s;
 }
 
 }  // namespace
