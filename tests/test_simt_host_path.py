@@ -61,3 +61,33 @@ for _ in range(2):
     assert ctx.decompress(raw, 1, 0.05, 1, is_zstd=False).tobytes() == o.decompress(raw, "to", 0.05, 1, zstd=False).tobytes()
     no_fault()
 """)
+
+
+def test_sort_after_a_failed_allocation(oracle):
+    """The sort's status words cannot grow for a large cloud: that call fails, and the next smaller one,
+    for which the old words sufficed, allocates its own."""
+    simt_host.run(PARTS + """
+ctx = X.Context(0)
+rng = np.random.default_rng(3)
+x = rng.uniform(0, 300, (60_000, 3)).astype(np.float32)
+
+def same(n):
+    raw = ctx.compress(x[:n], 1, 0.05, 1, 1, use_zstd=False)
+    no_fault()
+    assert raw == o.compress(x[:n], "to", 0.05, 1, 1, zstd=False)
+
+same(9000)
+try:  # grows the workspace: 128 KB a frame
+    ctx.zstd_decompress_device([device(b"no frame")] * 100, [8] * 100, [device(bytes(8))] * 100, [8] * 100)
+except X.XnyzError:
+    pass
+simt.simt_malloc_limit(100_000)
+try:
+    ctx.compress(x, 1, 0.05, 1, 1, use_zstd=False)
+    raise SystemExit("allocated")
+except X.XnyzError as e:
+    assert e.status == 4, e
+simt.simt_malloc_limit(1 << 40)
+same(9000)
+same(60_000)
+""")

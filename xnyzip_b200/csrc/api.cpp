@@ -386,6 +386,7 @@ xnyz_status radix_sort(xnyz_ctx* c, SortBufs& b, uint64_t n, int passes, uint32_
         CUDA_TRY(cudaStreamSynchronize(c->stream));
         if (c->sort_status) cudaFree(c->sort_status);
         c->sort_status = nullptr;
+        c->sort_status_cap = 0;  // (the allocation may fail)
         const size_t want = need + need / 4 + 4096;
         CUDA_TRY(cudaMalloc(&c->sort_status, want * sizeof(unsigned long long)));
         CUDA_TRY(cudaMemsetAsync(c->sort_status, 0, want * sizeof(unsigned long long), c->stream));
