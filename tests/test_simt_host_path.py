@@ -91,3 +91,24 @@ simt.simt_malloc_limit(1 << 40)
 same(9000)
 same(60_000)
 """)
+
+
+@pytest.mark.parametrize("rle,threshold", [(1, 0), (0, 0), (0, 1024)])
+def test_streams_whose_waits_run_out(oracle, rle, threshold):
+    """The stream decoders' status words get lost, so that every block but the first waits in vain
+    (64 times instead of seconds): the streams are decoded by one thread, and the result is right."""
+    simt_host.run(PARTS + f"""
+ctx = X.Context(0)
+x = np.random.default_rng(9).uniform(0, 40, (30_000, 3)).astype(np.float32)
+raw = o.compress(x, "to", 0.05, 1, {rle}, {threshold}, zstd=False)
+want = o.decompress(raw, "to", 0.05, {rle}, zstd=False).tobytes()
+simt.simt_drop_status(b"decode_sync_kernel")
+assert ctx.decompress(raw, 1, 0.05, {rle}, is_zstd=False).tobytes() == want
+kernels = simt.simt_kernels().decode()
+assert "decode_sequential_kernel" in kernels, kernels
+simt.simt_drop_status(b"")
+simt.simt_clear()
+assert ctx.decompress(raw, 1, 0.05, {rle}, is_zstd=False).tobytes() == want
+assert "decode_sequential_kernel" not in simt.simt_kernels().decode()
+no_fault()
+""")

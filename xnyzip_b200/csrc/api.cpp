@@ -77,6 +77,7 @@ struct Small {
     uint32_t empty_blocks;
     uint32_t fallback[8];
     uint32_t redone[8];  // decoder blocks that assumed a wrong entry, per stream
+    uint32_t stream_err[8];  // the entropy decoders' error words, of the last attempt at each stream
     unsigned long long max2[2];
     unsigned long long totals[8];
     unsigned long long codewords[8];
@@ -311,15 +312,15 @@ xnyz_status join_sides(xnyz_ctx* c) {
     return XNYZ_OK;
 }
 
-// The device error word as last copied to the host.
-xnyz_status device_errors(xnyz_ctx* c) {
-    const uint32_t e = c->h_small->err;
+xnyz_status device_error(uint32_t e) {
     if (e & 1u) return fail(XNYZ_ERR_TIMEOUT, "a bounded device wait expired");
     if (e & 2u) return fail(XNYZ_ERR_BAD_STREAM, "malformed bit stream");
     if (e & 4u) return fail(XNYZ_ERR_BAD_STREAM, "stream content exceeds its declared sizes");
     if (e & 8u) return fail(XNYZ_ERR_TIMEOUT, "a scatter position fell outside its array after a wait expired");
     return XNYZ_OK;
 }
+// The device error word as last copied to the host.
+xnyz_status device_errors(xnyz_ctx* c) { return device_error(c->h_small->err); }
 
 xnyz_status check_device_errors(xnyz_ctx* c) {
     TRY(fetch_small(c, offsetof(Small, err), sizeof(uint32_t)));
@@ -1697,7 +1698,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
     auto launch_sync = [&](const DecodeJob& j, cudaStream_t js) -> xnyz_status {
         launch_decode_sync(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.byte_symbols, j.nsym, j.width, j.out,
                            at<uint8_t>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
-                           SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, redone[j.slot]),
+                           SMALL_FIELD(c, stream_err[j.slot]), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, redone[j.slot]),
                            SMALL_FIELD(c, codewords[j.slot]), js);
         return XNYZ_OK;
     };
@@ -1706,7 +1707,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         launch_decode_stream(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.L, j.nsym, j.width, j.out,
                              at<uint32_t>(c, o_dflag[j.slot]), at<unsigned long long>(c, o_dagg[j.slot]),
                              at<unsigned long long>(c, o_dinc[j.slot]), SMALL_FIELD(c, tile_counters[30 + j.slot]),
-                             SMALL_FIELD(c, err), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, codewords[j.slot]),
+                             SMALL_FIELD(c, stream_err[j.slot]), SMALL_FIELD(c, fallback[j.slot]), SMALL_FIELD(c, codewords[j.slot]),
                              js);
         return XNYZ_OK;
     };
@@ -1723,7 +1724,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
                 1, j.total_bits / 8.0 + static_cast<double>(j.nsym) * j.width, js);
         if (j.fixed_len) {
             launch_decode_fixed(j.words, j.base_bits, j.total_bits, j.table, j.fixed_len, j.nsym, j.width, j.out,
-                                SMALL_FIELD(c, err), js);
+                                SMALL_FIELD(c, stream_err[j.slot]), js);
             continue;
         }
         if (j.tables) {  // (Huffman only)
@@ -1780,6 +1781,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
             }
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, fallback[j.slot]), 0, 4, st));
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, redone[j.slot]), 0, 4, st));
+            CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, stream_err[j.slot]), 0, 4, st));
             CUDA_TRY(cudaMemsetAsync(SMALL_FIELD(c, tile_counters[30 + j.slot]), 0, 4, st));
             if (why == 4u) {
                 CUDA_TRY(cudaMemsetAsync(at<uint8_t>(c, o_dinc[j.slot]), 0, 16 * dtiles[j.slot], st));
@@ -1789,7 +1791,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
                 TRY(launch_tables(j, st));
             } else {
                 launch_decode_sequential(j.kind, j.words, j.base_bits, j.total_bits, j.table, j.nsym, j.width, j.out,
-                                         SMALL_FIELD(c, codewords[j.slot]), SMALL_FIELD(c, err), st);
+                                         SMALL_FIELD(c, codewords[j.slot]), SMALL_FIELD(c, stream_err[j.slot]), st);
             }
             again = true;
         }
@@ -1797,6 +1799,7 @@ xnyz_status decompress_core(xnyz_ctx* c, const uint8_t* d_cont, uint64_t len, co
         TRY(prefixes(true));
     }
     TRY(device_errors(c));
+    for (auto& j : jobs) TRY(device_error(c->h_small->stream_err[j.slot]));
     for (auto& j : jobs)
         if (!j.fill && !j.fixed_len && c->h_small->codewords[j.slot] < j.nsym)
             return fail(XNYZ_ERR_BAD_STREAM, "stream " + std::to_string(j.slot) + " holds " +

@@ -18,8 +18,8 @@
 //
 // The block's stream words (plus a halo) and the Huffman primary table are staged in shared
 // memory; codewords are read through a 64-bit register bit buffer refilled one word at a
-// time.  Waits are bounded (kSpinLimit): a block that gives up sets kErrTimeout and the
-// host's fallback flag and returns.
+// time.  Waits are bounded (kSpinLimit): a block that gives up sets the host's fallback flag and
+// returns; that is no error yet, since the host then has one thread decode the stream.
 #include "device_common.cuh"
 #include "kernels.h"
 
@@ -43,6 +43,10 @@ constexpr int kMaxL = kDecodeMaxL;
 constexpr int kMaxRootBits = 11;
 constexpr u32 kOOD = 0xffu;             // exit outside the next subsequence's entry range
 constexpr u64 kFar = 1ull << 20;        // length given to an invalid Huffman code: ends the chain
+// Why the host has to decode a stream otherwise (kernels.h: launch_decode_sync).
+constexpr u32 kWaitExpired = 1u;
+constexpr u32 kNotConverged = 2u;
+constexpr u32 kWideValue = 4u;
 static_assert(kDecodeSubBits % 32 == 0 && kDecodeSubBitsGR % 32 == 0 && T % 32 == 0 && T <= 1024 &&
                   WIN <= kDecodeSubBits && WIN <= kDecodeSubBitsGR && kDecodeSubBits <= kDecodeSubBitsGR,
               "decode geometry");
@@ -776,10 +780,7 @@ __global__ void __launch_bounds__(T) decode_stream_kernel(Args a) {
         const u32 tabX = Es < 32u ? mx0 : mx1;
         const bool fast = !failed && Ei != kOOD && tabX != kOOD;
         if (t == 0) {
-            if (failed) {
-                atomicOr(a.err, kErrTimeout);
-                atomicOr(a.need_fallback, 1u);
-            }
+            if (failed) atomicOr(a.need_fallback, kWaitExpired);
             if (fast) {
                 st_volatile(&a.inc[(u64)tile * 2], (u64)tabX);
                 st_volatile(&a.inc[(u64)tile * 2 + 1], C + (Es < 32u ? mc0 : mc1));
@@ -892,8 +893,6 @@ constexpr int kSyncThreads = 128;
 constexpr int kSyncHalo = 8;
 constexpr int kMaxRounds = 64;
 constexpr u32 kMaxRedo = 256;
-constexpr u32 kNotConverged = 2u;
-constexpr u32 kWideValue = 4u;
 constexpr int kMaxMultiBits = 10;
 
 struct SyncArgs {
@@ -1233,8 +1232,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
                     const u32 given_up = __shfl_sync(kFullMask, lane == 0 ? ld_volatile(a.need_fallback) : 0u, 0);
                     if (++spins > kSpinLimit) {
                         failed = true;
-                        why = 1u;
-                        if (lane == 0) atomicOr(a.err, kErrTimeout);
+                        why = kWaitExpired;
                     } else if ((given_up & ~kWideValue) != 0u) {
                         failed = true;
                     }
