@@ -15,6 +15,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 #ifdef __CUDACC__
 #define ZD_HD __host__ __device__ __forceinline__
@@ -78,7 +79,7 @@ struct Tables {
     u32 state[3], rep[3];
     // a chunk's bytes: the values of those from outside, and the byte of the chunk that each repeats (or itself)
     u64 q_value[kChunkBytes / 8 + 2];
-    u64 q_from[(kChunkBytes / 8 + 2) * 2];
+    alignas(8) u16 q_from[kChunkBytes + 16];
     int msg[4];
 };
 struct Workspace : Tables {
@@ -955,7 +956,7 @@ ZD_HD void run_chunk(WS& ws, int first, int last, u8* dst, const u8* lit, const 
     }
     const u32 lead = (u32)((u64)dst & 7u), groups = (lead + total + 7u) / 8u;
     u8* const value = reinterpret_cast<u8*>(ws.q_value);
-    u16* const from = reinterpret_cast<u16*>(ws.q_from);
+    u16* const from = ws.q_from;
     bool inside = false;  // some byte of mine repeats one of the chunk
     for (u32 g = (u32)team.rank; g < groups; g += (u32)team.size) {
         const u32 lo = 8u * g > lead ? 8u * g - lead : 0u, hi = 8u * g + 8u - lead < total ? 8u * g + 8u - lead : total;
@@ -986,8 +987,8 @@ ZD_HD void run_chunk(WS& ws, int first, int last, u8* dst, const u8* lit, const 
             else f1 |= (u64)f8[j] << (16u * (j - 4u));
         }
         ws.q_value[g] = v;
-        ws.q_from[2 * g] = f0;
-        ws.q_from[2 * g + 1] = f1;
+        memcpy(__builtin_assume_aligned(from + 8u * g, 8), &f0, 8);
+        memcpy(__builtin_assume_aligned(from + 8u * g + 4u, 8), &f1, 8);
     }
     team.sync();
     // a byte's source may meanwhile have been replaced by a later one on the same way: as good
