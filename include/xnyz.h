@@ -113,7 +113,7 @@ xnyz_status xnyz_compress(xnyz_ctx* ctx, const float* xyz, uint64_t n, int xyz_i
 
 /* Compress into a device-resident container.  `xyz` is a device pointer; the container
  * stays in the context's workspace and is described by (*dev_container, *container_len)
- * until the next call on the context. */
+ * until the next call on the context (which may have written to it even if it fails). */
 xnyz_status xnyz_compress_device(xnyz_ctx* ctx, const float* xyz, uint64_t n, const xnyz_params* params,
                                  const uint8_t** dev_container, uint64_t* container_len, xnyz_compress_info* info);
 
@@ -159,7 +159,10 @@ xnyz_status xnyz_decompress_into(xnyz_ctx* ctx, const uint8_t* in, uint64_t in_l
                                  float l2_bound, int rle, float* xyz, uint64_t capacity, uint64_t* n);
 
 /* Decompress a device-resident raw container into a device array owned by the context
- * (valid until the next call).  Host code reads the few header fields it needs. */
+ * (valid until the next call).  Host code reads the few header fields it needs.  The container is
+ * read where it lies, until the call returns, if that is on a 4-byte boundary of the context's
+ * device's memory; any other memory that a device copy can read (pinned host memory, another
+ * device's) is copied first. */
 xnyz_status xnyz_decompress_device(xnyz_ctx* ctx, const uint8_t* dev_container, uint64_t len, int quantizer,
                                    float l2_bound, int rle, const float** dev_xyz, uint64_t* n);
 

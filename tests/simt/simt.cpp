@@ -178,7 +178,13 @@ struct Event {
 };
 Stream null_stream;
 std::map<Stream*, int> streams{{&null_stream, 0}};
-std::map<const char*, std::pair<size_t, bool>> memory;  // bytes, pinned host memory
+struct Region {
+    size_t bytes;
+    bool pinned;          // host memory
+    int device = 0;
+    char* data = nullptr; // another device's memory: what copies read; kernels find poison at its address
+};
+std::map<const char*, Region> memory;
 size_t malloc_limit = ~size_t(0);
 std::string kernels;
 
@@ -198,17 +204,21 @@ void issue(cudaStream_t s, std::function<void()> op) {
 void run_all() {
     for (auto& s : streams) run_to(s.first, s.first->issued);
 }
-const std::pair<const char* const, std::pair<size_t, bool>>* find(const void* p) {
+const std::pair<const char* const, Region>* find(const void* p) {
     auto it = memory.upper_bound(static_cast<const char*>(p));
     if (it == memory.begin()) return nullptr;
     --it;
-    return static_cast<const char*>(p) < it->first + it->second.first ? &*it : nullptr;
+    return static_cast<const char*>(p) < it->first + it->second.bytes ? &*it : nullptr;
 }
 bool pageable(const void* p) { return !find(p); }
+const void* readable(const void* p) {
+    auto* m = find(p);
+    return m && m->second.data ? m->second.data + (static_cast<const char*>(p) - m->first) : p;
+}
 void* take(size_t n, bool pinned, unsigned char poison) {
     void* p = std::aligned_alloc(256, (n + 255) / 256 * 256 + 256);
     std::memset(p, poison, n);
-    memory[static_cast<char*>(p)] = {n, pinned};
+    memory[static_cast<char*>(p)] = Region{n, pinned};
     return p;
 }
 }  // namespace
@@ -256,7 +266,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
         issue(st, [=] { std::memcpy(d, copy->data(), n); });
     } else {
         if (k == cudaMemcpyDeviceToDevice && (pageable(d) || pageable(s))) return cudaErrorInvalidValue;
-        issue(st, [=] { std::memmove(d, s, n); });
+        issue(st, [=] { std::memmove(d, readable(s), n); });
         if (k == cudaMemcpyDeviceToHost && pageable(d)) return cudaStreamSynchronize(st);
     }
     return cudaSuccess;
@@ -340,7 +350,10 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
 cudaError_t cudaDeviceReset() { return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     *a = cudaPointerAttributes{};
-    if (auto* m = find(p)) a->type = m->second.second ? cudaMemoryTypeHost : cudaMemoryTypeDevice;
+    if (auto* m = find(p)) {
+        a->type = m->second.pinned ? cudaMemoryTypeHost : cudaMemoryTypeDevice;
+        a->device = m->second.device;
+    }
     return cudaSuccess;
 }
 
@@ -362,6 +375,13 @@ void simt_malloc_limit(uint64_t n) { malloc_limit = n; }
 void simt_drop_status(const char* kernel) { drop = kernel; }
 void* simt_device_alloc(uint64_t n) { return take(n, false, 0xA5); }
 void* simt_pinned_alloc(uint64_t n) { return take(n, true, 0x5A); }
+// Another device's memory, which only copies reach; *data is where its contents are.
+void* simt_peer_alloc(uint64_t n, void** data) {
+    char* p = static_cast<char*>(take(n, false, 0xD1));
+    memory[p].device = 1;
+    *data = memory[p].data = static_cast<char*>(std::malloc(n));
+    return p;
+}
 void simt_device_free(void* p) {  // at once, without waiting for queued work
     memory.erase(static_cast<char*>(p));
     std::memset(p, 0xEE, 64);

@@ -126,6 +126,8 @@ import xnyzip_b200 as X
 ctypes.CDLL = _real
 simt.simt_fault.restype = simt.simt_kernels.restype = ctypes.c_char_p
 simt.simt_pending.restype = ctypes.c_uint64
+simt.simt_peer_alloc.restype = ctypes.c_void_p
+simt.simt_peer_alloc.argtypes = [ctypes.c_uint64, ctypes.c_void_p]
 simt.simt_device_alloc.restype = simt.simt_pinned_alloc.restype = ctypes.c_void_p
 simt.simt_device_alloc.argtypes = simt.simt_pinned_alloc.argtypes = simt.simt_malloc_limit.argtypes = [ctypes.c_uint64]
 simt.simt_device_free.argtypes = [ctypes.c_void_p]
@@ -134,6 +136,12 @@ def device(data, pinned=False):
     data = bytes(data) if not hasattr(data, "tobytes") else data.tobytes()
     p = (simt.simt_pinned_alloc if pinned else simt.simt_device_alloc)(len(data))
     ctypes.memmove(p, data, len(data))
+    return p
+
+def peer(data):
+    at = ctypes.c_void_p()
+    p = simt.simt_peer_alloc(len(data), ctypes.byref(at))
+    ctypes.memmove(at, data, len(data))
     return p
 
 def no_fault():

@@ -112,3 +112,19 @@ assert ctx.decompress(raw, 1, 0.05, {rle}, is_zstd=False).tobytes() == want
 assert "decode_sequential_kernel" not in simt.simt_kernels().decode()
 no_fault()
 """)
+
+
+@pytest.mark.parametrize("where", ["device", "pinned", "peer"])
+@pytest.mark.parametrize("n", [200, 6000])
+def test_containers_that_only_a_copy_can_reach(oracle, where, n):
+    """decompress_device takes containers in any memory that a copy can read: another device's without
+    peer access (whose addresses hold other bytes for a kernel here), pinned host memory."""
+    simt_host.run(PARTS + f"""
+ctx = X.Context(0)
+x = np.random.default_rng({n}).uniform(0, 60, ({n}, 3)).astype(np.float32)
+raw = o.compress(x, "to", 0.05, 1, 1, 0, zstd=False)
+p = dict(device=lambda: device(raw), pinned=lambda: device(raw, pinned=True), peer=lambda: peer(raw))[{where!r}]()
+q, k = ctx.decompress_device(p, len(raw), 1, 0.05, 1)
+no_fault()
+assert ctypes.string_at(q, 12 * k) == o.decompress(raw, "to", 0.05, 1, zstd=False).tobytes()
+""")

@@ -2286,6 +2286,17 @@ xnyz_status xnyz_zstd_decompress_device(xnyz_ctx* c, uint64_t count, const uint8
     return XNYZ_OK;
 }
 
+// Whether p is memory of the context's device (0.3 us; another device's may be out of a kernel's reach, and
+// host memory is better copied than read in pieces).
+static bool on_device(const xnyz_ctx* c, const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == c->device;
+}
+
 xnyz_status xnyz_decompress_device(xnyz_ctx* c, const uint8_t* dev_container, uint64_t len, int quantizer,
                                    float l2_bound, int rle, const float** dev_xyz, uint64_t* n) {
     clear_stale_cuda_error();
@@ -2296,11 +2307,11 @@ xnyz_status xnyz_decompress_device(xnyz_ctx* c, const uint8_t* dev_container, ui
     cudaStream_t st = c->stream;
     // The kernels read the streams as aligned 4-byte words, at most 12 bytes past a stream's end
     // (the block streams in 16-byte pieces, at most 28 past it), which is where the next streams'
-    // lengths or the container's offset lie: a container on a 4-byte boundary is decoded in place,
-    // any other is copied to one.
+    // lengths or the container's offset lie: a container on a 4-byte boundary of this device's memory is
+    // decoded in place, any other is copied to one.
     const uint8_t* d_cont = dev_container;
     size_t reserved = 0;
-    if (reinterpret_cast<uintptr_t>(dev_container) & 3u) {
+    if ((reinterpret_cast<uintptr_t>(dev_container) & 3u) || !on_device(c, dev_container)) {
         reserved = align_up(len + 64);
         TRY(ensure_arena(c, reserved));
         CUDA_TRY(cudaMemcpyAsync(c->arena.base, dev_container, len, cudaMemcpyDeviceToDevice, st));
