@@ -44,10 +44,11 @@ struct Thread {
 extern Thread* self;
 extern Dim block_idx, grid_dim, block_dim;
 void barrier(int line);
-int barrier_or(int line, int p);
+int barrier_count(int line, int p);  // how many threads bring p
 void named_barrier(int id, int count);
 const uint64_t* exchange(int line, uint64_t v);  // the 32 lanes' values
 void* dynamic_shared();
+long long ticks();  // 4096 per block barrier
 bool dropped();  // the running kernel's status words get lost (simt_drop_status)
 struct Config {
     unsigned grid, block;
@@ -84,7 +85,8 @@ inline unsigned lane() { return self->tid.x & 31u; }
 #define gridDim simt::grid_dim
 #define blockDim simt::block_dim
 #define __syncthreads() simt::barrier(__LINE__)
-#define __syncthreads_or(p) simt::barrier_or(__LINE__, (p))
+#define __syncthreads_or(p) (simt::barrier_count(__LINE__, (p)) != 0)
+#define __syncthreads_count(p) simt::barrier_count(__LINE__, (p))
 #define __syncwarp() ((void)simt::exchange(__LINE__, 0))
 
 struct alignas(8) uint2 { unsigned x, y; };

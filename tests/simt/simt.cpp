@@ -37,10 +37,12 @@ std::vector<std::unique_ptr<Fiber>> pool;
 std::vector<Warp> warps;
 ucontext_t scheduler;
 std::function<void()>* body;
-int or_result;
+int barrier_sum;
 alignas(16) unsigned char shared_memory[228 << 10];
 
 std::string fault, current, drop;
+std::map<std::string, uint64_t> barriers;  // of each kernel since simt_clear
+long long barrier_clock = 0;
 int order = 0;
 
 void flag(const std::string& what) {
@@ -91,14 +93,14 @@ bool run_block(unsigned n) {
         unsigned at[5] = {0, 0, 0, 0, 0};
         int line = -1, id = -1, count = 0;
         bool mixed = false;
-        or_result = 0;
+        barrier_sum = 0;
         for (unsigned i = 0; i < n; ++i) {
             Fiber* f = pool[i].get();
             ++at[f->state];
             if (f->state == kBlock) {
                 mixed |= line >= 0 && line != f->line;
                 line = f->line;
-                or_result |= f->p;
+                barrier_sum += f->p;
             }
             if (f->state == kNamed) {
                 id = f->id;
@@ -112,6 +114,8 @@ bool run_block(unsigned n) {
             continue;
         }
         if (at[kBlock] == n && !mixed) {
+            ++barriers[current];
+            barrier_clock += 4096;
             for (unsigned i = 0; i < n; ++i) pool[i]->state = kReady;
             continue;
         }
@@ -131,13 +135,13 @@ void barrier(int line) {
     f->p = 0;
     yield();
 }
-int barrier_or(int line, int p) {
+int barrier_count(int line, int p) {
     Fiber* f = me();
     f->state = kBlock;
     f->line = line;
     f->p = p != 0;
     yield();
-    return or_result;
+    return barrier_sum;
 }
 void named_barrier(int id, int count) {
     Fiber* f = me();
@@ -163,6 +167,7 @@ const uint64_t* exchange(int line, uint64_t v) {
     }
     return w.slot[gen & 1];
 }
+long long ticks() { return barrier_clock; }
 void* dynamic_shared() { return shared_memory; }
 bool dropped() { return !drop.empty() && current.find(drop) != std::string::npos; }
 
@@ -363,8 +368,16 @@ const char* simt_fault() { return fault.c_str(); }
 void simt_clear() {
     fault.clear();
     kernels.clear();
+    barriers.clear();
 }
 const char* simt_kernels() { return kernels.c_str(); }  // launched, one per line
+// Barriers that the kernels of this name have met, over all their blocks.
+uint64_t simt_barriers(const char* name) {
+    uint64_t n = 0;
+    for (auto& b : barriers)
+        if (b.first.find(name) != std::string::npos) n += b.second;
+    return n;
+}
 // Work that has been queued and not run.
 uint64_t simt_pending() {
     uint64_t n = 0;

@@ -45,7 +45,7 @@ def translate(text, spin_limit):
         text = re.sub(pattern, lambda m: to, text, flags=re.S)
     text = re.sub(r"extern __shared__ __align__\(16\) unsigned char (\w+)\[\];",
                   r"unsigned char* \1 = static_cast<unsigned char*>(simt::dynamic_shared());", text)
-    text = text.replace("kSpinLimit = 1u << 23", f"kSpinLimit = {spin_limit}u")
+    text = text.replace("kSpinLimit = 1u << 23", f"kSpinLimit = {spin_limit}u").replace(")clock()", ")simt::ticks()")
     return LAUNCH.sub(lambda m: f'simt::launch("{m.group(1)}", simt::config({m.group(2)}), {m.group(1)}, {m.group(3)});', text)
 
 
@@ -125,7 +125,7 @@ import numpy as np
 import xnyzip_b200 as X
 ctypes.CDLL = _real
 simt.simt_fault.restype = simt.simt_kernels.restype = ctypes.c_char_p
-simt.simt_pending.restype = ctypes.c_uint64
+simt.simt_pending.restype = simt.simt_barriers.restype = ctypes.c_uint64
 simt.simt_peer_alloc.restype = ctypes.c_void_p
 simt.simt_peer_alloc.argtypes = [ctypes.c_uint64, ctypes.c_void_p]
 simt.simt_device_alloc.restype = simt.simt_pinned_alloc.restype = ctypes.c_void_p

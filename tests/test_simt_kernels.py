@@ -43,3 +43,28 @@ got = X.Context(0).decompress(raw, 0, 0.05, 0, is_zstd=False)
 no_fault()
 assert got.tobytes() == Oracle().decompress(raw, "cube", 0.05, 0, zstd=False).tobytes()
 """)
+
+
+@pytest.mark.parametrize("period", ["runs", "three bits"])
+def test_giving_a_stream_up_is_cheap(oracle, period):
+    """Streams that never fall in step (one run of the codeword 11 of the code 0, 10, 11; the codeword 110
+    of a code with lengths 2 to 4) go to the decoder with entry tables.  The blocks that find it out stop
+    after some rounds, and those that start later at once: barriers over all 24 and 36 blocks."""
+    simt_host.run(f"""
+from oracle import Oracle
+from test_gpu_stream_decode import container
+sym, lens = np.full(220_000, 3), {{1: 1, 2: 2, 3: 2}}
+sym[0] = 1
+if {period!r} == "three bits":
+    sym, lens = np.full(220_000, 8), {{1: 3, 2: 2, 3: 3, 4: 3, 5: 3, 6: 4, 7: 4, 8: 3}}
+    sym[0] = 2
+raw = container(sym, lens)
+ctx = X.Context(0)
+simt.simt_clear()
+got = ctx.decompress(raw, 0, 0.05, 0, is_zstd=False)
+no_fault()
+assert "decode_stream_kernel" in simt.simt_kernels().decode()
+runs = simt.simt_kernels().decode().count("decode_sync_kernel")
+assert simt.simt_barriers(b"decode_sync_kernel") <= 400 * runs, simt.simt_barriers(b"decode_sync_kernel")
+assert got.tobytes() == Oracle().decompress(raw, "cube", 0.05, 0, zstd=False).tobytes()
+""")

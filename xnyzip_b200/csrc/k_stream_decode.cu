@@ -891,9 +891,21 @@ __global__ void __launch_bounds__(T) decode_stream_kernel(Args a) {
 // 568 -> 113 us.
 constexpr int kSyncThreads = 128;
 constexpr int kSyncHalo = 8;
-constexpr int kMaxRounds = 64;
-constexpr u32 kMaxRedo = 256;
-constexpr int kMaxMultiBits = 10;
+// When a block gives up, looked at after every fourth round (in every round, 120K points took 2 us longer): a
+// quarter of its threads still change after eight, or the rounds took this long (again from the true entry:
+// shorter).  Of the streams of all kinds of clouds that fall in step, the slowest takes 39 rounds and 207000
+// clocks; half as long turned some of them away, which are then three times slower.  With 64 rounds, all blocks to
+// themselves and 256 second decodings, a stream of 16M bits that never falls in step took 0.48 ms more than its
+// entry tables alone (now 0.09), of 120K bits 0.5 (0.13), and 7M uniform points, whose symbols have long runs,
+// took 2.0-2.2 ms (1.4 when the entry tables came first, now 0.98).
+constexpr int kRoundsPerLook = 4;
+constexpr u32 kSettleClocks = 220000, kRedoClocks = 60000;
+// Blocks that may decode again; each makes all later ones wait, some 20 us.
+constexpr u32 kFreeRedos = 2, kBlocksPerRedo = 256;
+// Window of the several-symbols table: at least 7 bits (an entry per thread), for codes shorter than that too.
+// As narrow as the code, a round of a two-bit code took 15400 clocks; with 7 bits runs of its symbols fall in
+// step in 150 us where they took 260 (60K symbols), and 1013 points decompress in 107 us instead of 118.
+constexpr int kMinMultiBits = 7, kMaxMultiBits = 10;
 
 struct SyncArgs {
     const u32* words;
@@ -1076,7 +1088,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     constexpr int TT = kSyncThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ u32 slot;
+    __shared__ u32 slot, given_up, late;
     __shared__ u64 s_assumed, s_entry, s_first, s_wsum[TT / 32];
     u64* sx = reinterpret_cast<u64*>(smem_raw);
     u32* mlen = reinterpret_cast<u32*>(sx + TT);
@@ -1108,12 +1120,14 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     // (tile 0 stages from the stream's start)
     const u64 w0 = (u64)((long long)tile * (TT - G) - (tile == 0 ? 0 : G)) * (u32)(S / 32);
     str.org = w0 * 32 - a.base;
+    const u32 why_not = t == 0 ? ld_volatile(a.need_fallback) : 0u;
 #pragma unroll 8
     for (int i = t; i < staged; i += TT) {
         const u64 k = w0 + (u64)i;
         const u32 x = k < str.g.nwords ? __ldg(a.words + k) : 0u;
         sw[i] = KIND == kCodeGolombRice ? x : __byte_perm(x, 0, 0x0123);
     }
+    if (t == 0) given_up = why_not & ~kWideValue;
     if (KIND == kCodeHuffman) {
 #pragma unroll 8
         for (int i = t; i < (1 << a.code.rb); i += TT) root[i] = __ldg(a.code.root + i);
@@ -1137,13 +1151,15 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
         }
     }
     __syncthreads();
+    if (given_up) return;  // (whoever waits for this block looks at need_fallback too)
 
     const u64 B = valid ? (u64)sub * (u32)S : 0ull;
     const u64 Bend = valid ? min(B + (u64)S, a.total_bits) : 0ull;
     u64 entry = B;
     u32 count = 0;
     // Rounds from thread `from` on (its entry stays) until every entry is the exit before it.
-    auto settle = [&](int from, bool active) {
+    auto settle = [&](int from, bool active, u32 clocks) {
+        const u32 begin = (u32)clock();
         for (int round = 0;; ++round) {
             if (active) {
                 count = 0;
@@ -1154,10 +1170,13 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
             active = valid && t > from && e != entry;
             entry = e;
             if (!__syncthreads_or(active)) return true;
-            if (round == kMaxRounds) return false;
+            if (round % kRoundsPerLook == kRoundsPerLook - 1) {
+                if (t == 0) late = (u32)clock() - begin > clocks;
+                if ((__syncthreads_count(active) > TT / 4 && round > kRoundsPerLook) || late) return false;
+            }
         }
     };
-    bool settled = settle(first_t, valid);
+    bool settled = settle(first_t, valid, kSettleClocks);
 
     // codewords before mine within the block's own subsequences, and the block's total
     const bool own = valid && t >= G;
@@ -1256,7 +1275,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
                 __threadfence();
             }
             const bool same = E == assumed - tile_at;
-            if (!failed && !same && atomicAdd(a.redone, 1u) >= kMaxRedo) atomicOr(a.need_fallback, kNotConverged);
+            if (!failed && !same && atomicAdd(a.redone, 1u) >= kFreeRedos + gridDim.x / kBlocksPerRedo) atomicOr(a.need_fallback, kNotConverged);
             if (failed || same) st_status(&a.status[tile], tile_state(C + total, 0ull, exit_of() & 0xffffffffull), 2u);
             s_entry = failed ? assumed : tile_at + E;
             s_first = C;
@@ -1265,7 +1284,7 @@ __global__ void __launch_bounds__(kSyncThreads) decode_sync_kernel(SyncArgs a) {
     __syncthreads();
     if (s_entry != assumed) {  // block-uniform: decode again from the true entry
         if (t == G) entry = s_entry;
-        const bool ok = settle(G, t == G);
+        const bool ok = settle(G, t == G, kRedoClocks);
         sum_counts();
         if (t == 0) {
             if (!ok || (exit_of() >> 32) != 0) {
@@ -1541,7 +1560,7 @@ void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uin
     a.code.rb = kind == kCodeHuffman ? t.root_bits : 0;
     a.code.k = t.param;
     a.code.zigzag = t.zigzag;
-    a.mb = t.root_bits < kMaxMultiBits ? t.root_bits : kMaxMultiBits;
+    a.mb = t.root_bits < kMinMultiBits ? kMinMultiBits : t.root_bits < kMaxMultiBits ? t.root_bits : kMaxMultiBits;
     a.multi_out = byte_symbols && !t.symvals;
     a.nsym = nsym;
     a.out_width = out_width;
