@@ -83,7 +83,7 @@ __device__ __forceinline__ u32 digit_lookback(u64* status, u32 tile, u32 d, u32 
 __device__ __forceinline__ u64 load_now(const u64* p, bool ok) {
     u64 v;
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.b64 %0, 0; @q ld.global.b64 %0, [%1]; }"
-                 : "=l"(v)
+                 : "=&l"(v)
                  : "l"(p), "r"((u32)ok));
     return v;
 }
