@@ -945,8 +945,10 @@ xnyz_status compress_core(xnyz_ctx* c, const float* d_xyz, uint64_t n, const xny
     enc.err = SMALL_FIELD(c, err);
     const bool has_gr = P && !ext;
     if (has_gr) enc.job[enc.count++] = job(0, direct ? kEncodeGolombRice64 : kEncodeGolombRice32, uo.patches, P, grk, o_w_gr, bits_gr);
-    // (few patches: with the other coders in one launch)
-    const bool gr_early = has_gr && P >= 65536 && pe.total <= c->arena.cap;
+    // Few patches are coded with the other streams in one launch: alone they take two launches more.  Uniform
+    // clouds, whole compression, us, early and with the others: 66K patches 203 and 186, 131K 203 and 198,
+    // 524K 262 and 258, 1.05M 308 and 313, 4.2M 559 and 570.
+    const bool gr_early = has_gr && P >= (3u << 18) && pe.total <= c->arena.cap;
     if (gr_early) {
         Fills f;
         f.add(at<uint32_t>(c, o_w_gr), 4 * words_for(bits_gr), 0);
