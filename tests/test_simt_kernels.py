@@ -68,3 +68,22 @@ runs = simt.simt_kernels().decode().count("decode_sync_kernel")
 assert simt.simt_barriers(b"decode_sync_kernel") <= 400 * runs, simt.simt_barriers(b"decode_sync_kernel")
 assert got.tobytes() == Oracle().decompress(raw, "cube", 0.05, 0, zstd=False).tobytes()
 """)
+
+
+@pytest.mark.parametrize("order", ORDERS)
+def test_zstd_frames_by_a_block(order):
+    """The frame decoder as the device compiles it: 128 threads, the first warp walking the next
+    sequences' states while the other three write the output; against libzstd."""
+    simt_host.run(f"""
+import test_zstd_host as T
+simt.simt_order({order})
+ctx = X.Context(0)
+frame, data = T._zstd(), [d[:50_000] for d in T._data() if d]
+for level in (1, 19):
+    frames = [frame(d, level) for d in data]
+    out = [device(bytes(len(d))) for d in data]
+    sizes = ctx.zstd_decompress_device([device(f) for f in frames], [len(f) for f in frames], out, [len(d) for d in data])
+    no_fault()
+    for n, p, d in zip(sizes, out, data):
+        assert n == len(d) and ctypes.string_at(p, n) == d
+""")

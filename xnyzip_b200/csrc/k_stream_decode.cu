@@ -877,9 +877,9 @@ __global__ void __launch_bounds__(T) decode_stream_kernel(Args a) {
 // The first G threads of a block redo the last G subsequences of the block before, so that the
 // block's own entry has normally fallen in step as well.  A block publishes (entry it assumed,
 // exit, codewords); a later block walks back over a chain of blocks whose assumed entries match
-// the exits before them, up to one whose result is final (32 at a time), and so gets its true
+// the exits before them, up to one whose result is final (128 at a time), and so gets its true
 // entry and its output position.  A block whose assumption was wrong decodes again from the
-// true entry.  Waits are bounded.  Streams that do not fall in step (kNotConverged, or too many
+// true entry.  Waits are bounded.  Streams that do not fall in step in time (kNotConverged, or too many
 // wrong assumptions) are left to decode_stream_kernel, whose entry tables do not depend on it.
 //
 // What bounds it: the dependent chain of codewords within a subsequence (two word reads, a

@@ -12,11 +12,12 @@ struct Workspace : zd::Tables {
     zd::u8* lit;
 };
 
-// One frame per block of 128 threads (zd::BlockTeam), the tables in shared memory; registers for six
-// blocks per SM, so that 768 frames run at once.  Bound by latency: the frames with the most sequences (6170
-// in 28 KB) are last, for whom the states' chain takes 160 clocks a sequence and the copies, beside it in
-// other warps, about as much.  One warp per frame, whose lanes walked the sequences together, byte loads for
-// the bits, tables in global memory and one copy after another took 6.9 ms for 768 frames of 27 KB (81 KB of
+// One frame per block of 128 threads (zd::BlockTeam), the tables in shared memory.  Registers (80) and shared
+// memory (35 KB) for six blocks per SM, 888 frames at once; with 96 registers, so five blocks, an earlier
+// state took 2.10 ms instead of 1.98.  Bound by latency: the frames with the most sequences (6170 in 28 KB)
+// are last, for whom the states' chain takes 160 clocks a sequence and the copies, beside it in other
+// warps, about as much.  One warp per frame, whose lanes walked the sequences together, byte loads for the
+// bits, tables in global memory and one copy after another took 6.9 ms for 768 frames of 27 KB (81 KB of
 // content); this takes 1.4 ms.
 __global__ void __launch_bounds__(zd::BlockTeam::size, 6) zstd_frames_kernel(const uint8_t* const* src, const uint64_t* src_len,
                                                                           uint8_t* const* dst, const uint64_t* cap,

@@ -16,7 +16,7 @@ struct QuantParams {
     float div;      // float(double(2*l2)/sqrt(3|5))
     float s;        // l2 as float
     float rdiv;     // float(sqrt(3|5))
-    float inv;      // 1 / div correctly rounded, or 0: divide (quotients_exact)
+    float inv;      // 1 / div correctly rounded, or 0: divide (quantize_range_kernel checks the extents too)
     float rinv;     // 1 / rdiv correctly rounded, or 0: divide (a bound near the float range's ends)
     float step[3];  // adaptive: per-axis steps (decompression: from the container)
     const float* step_dev;  // adaptive compression: the steps in device memory (PointStats::step)
@@ -282,11 +282,11 @@ void launch_decode_sync(int kind, const uint32_t* words, uint64_t base_bits, uin
                         bool byte_symbols, uint64_t nsym, int out_width, void* out, void* status,
                         uint32_t* tile_counter, uint32_t* err, uint32_t* need_fallback, uint32_t* redone,
                         unsigned long long* total_codewords, cudaStream_t st);
-// One-thread decoder the host runs when a bounded wait of the parallel decoder expired.
 // A Huffman stream whose codewords all have length len (== t.root_bits <= 11): every symbol
 // from its own len bits (out_width 1: u8, 4: u32 values).
 void launch_decode_fixed(const uint32_t* words, uint64_t base_bits, uint64_t total_bits, DecodeTable t, int len,
                          uint64_t nsym, int out_width, void* out, uint32_t* err, cudaStream_t st);
+// One-thread decoder the host runs when a bounded wait of a parallel decoder expired.
 void launch_decode_sequential(int kind, const uint32_t* words, uint64_t base_bits, uint64_t total_bits,
                               DecodeTable t, uint64_t nsym, int out_width, void* out,
                               unsigned long long* total_codewords, uint32_t* err, cudaStream_t st);
